@@ -113,6 +113,12 @@ dp_status dpk_gemm_bf16w_f32(dp_ctx *ctx, const __nv_bfloat16 *W, int w_stride, 
 // f16 operands, f16 result: C [M, N] = A [M, K] W^T (f32 accumulation)
 dp_status dpk_gemm_f16_tc(dp_ctx *ctx, const __half *W, int w_stride, const __half *A, int a_stride, __half *C, int c_stride, int M, int N, int K);
 
+// ---- the tied head for several rows of a portion (head_rows.cu) ----
+bool dpk_head_rows_ok(int K);
+size_t dpk_head_rows_scratch(int K);
+dp_status dpk_head_rows(dp_ctx *ctx, const float *h, int h_stride, const int *at, int R, const GroupNorm &n, const __nv_bfloat16 *W, int w_stride, void *scratch,
+                        float *C, int N, int K);
+
 // ---- attention helpers (attn_prep.cu) ----
 // rows [q | k | v | ...] of qkv_stride floats: q and k per head optionally divided by their root mean square; q to
 // q_out [row][heads][dim] f32, k and v appended to the caches (f16 or f32) at their positions
