@@ -7,15 +7,13 @@
 // TMEM, four epilogue warps) with two accumulators in tensor memory, so the next tile's products run under this
 // tile's stores.  K tails and rows beyond M or N are zero filled by TMA.  Every wait is bounded.
 //
-// gemm_bf16w_f32_kernel (f32 activations): the 32-bit mode.  bf16 weights are exact in f32; every product and sum is
-// an f32 FMA on the CUDA cores.
-//
 // dpk_gemm_f16_tc: the same kernel with f16 operands and an f16 result.
 //
 // Optional decay: exp(-rate softplus(c + bias)) of every product is stored instead of the product.
 // Optional gated activation: weight rows in groups of sixteen (eight gate rows, then their eight up rows) and
 // g' sigmoid(slope g') (u' + shift) with g' = min(g, limit), u' = clamp(u, +-limit) stored in A's type.
 #include "layers.h"
+#include "decay.cuh"
 #include "pdl.cuh"
 #include "umma.cuh"
 
@@ -31,26 +29,13 @@ struct GluArgs {
   float limit, slope, shift;
 };
 
-__device__ __forceinline__ float glu_act(float g, float u, const GluArgs &a) {
-  if (a.limit > 0.0f) {
-    g = fminf(g, a.limit);
-    u = fminf(fmaxf(u, -a.limit), a.limit);
-  }
-  return g * (1.0f / (1.0f + expf(-a.slope * g))) * (u + a.shift);
-}
-
-// ... for a result that is stored as bf16
+// for a result that is stored as bf16
 __device__ __forceinline__ float glu_act_fast(float g, float u, const GluArgs &a) {
   if (a.limit > 0.0f) {
     g = fminf(g, a.limit);
     u = fminf(fmaxf(u, -a.limit), a.limit);
   }
   return __fdividef(g, 1.0f + __expf(-a.slope * g)) * (u + a.shift);
-}
-
-__device__ __forceinline__ float decay_of(float c, float rate, float bias) {
-  const float z = c + bias;
-  return expf(-rate * (fmaxf(z, 0.0f) + log1pf(expf(-fabsf(z)))));
 }
 
 constexpr int BT_THREADS = 256, BT_MAX_STAGES = 8;
@@ -204,59 +189,6 @@ __global__ void __launch_bounds__(BT_THREADS, 1) gemm_bf16_tc_kernel(const __gri
   if (abort_word && tid == 0) atomicExch(err, 2);
 }
 
-// ---- 32-bit mode ----
-constexpr int FM = 64, FN = 64, FK = 16;
-__global__ void __launch_bounds__(256) gemm_bf16w_f32_kernel(const __nv_bfloat16 *__restrict__ W, int w_stride, const float *__restrict__ A, int a_stride,
-                                                             float *__restrict__ C, int M, int N, int K, const GluArgs glu, const DecayOut decay) {
-  pdl_launch();
-  pdl_wait();
-  __shared__ float sa[FK][FM + 4], sw[FK][FN + 4];
-  __shared__ float sc[FM][FN + 1];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int m0 = blockIdx.y * FM, n0 = blockIdx.x * FN;
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < K; k0 += FK) {
-    for (int i = tid; i < FM * FK; i += 256) {
-      const int r = i / FK, k = i % FK;
-      sa[k][r] = (m0 + r < M && k0 + k < K) ? A[(size_t)(m0 + r) * a_stride + k0 + k] : 0.0f;
-      sw[k][r] = (n0 + r < N && k0 + k < K) ? __bfloat162float(W[(size_t)(n0 + r) * w_stride + k0 + k]) : 0.0f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < FK; k++) {
-      float av[4], wv[4];
-#pragma unroll
-      for (int i = 0; i < 4; i++) { av[i] = sa[k][ty * 4 + i]; wv[i] = sw[k][tx * 4 + i]; }
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-  if (!glu.dst) {
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-      for (int j = 0; j < 4; j++)
-        if (m0 + ty * 4 + i < M && n0 + tx * 4 + j < N) {
-          const int n = n0 + tx * 4 + j;
-          C[(size_t)(m0 + ty * 4 + i) * N + n] = decay.rate ? decay_of(acc[i][j], decay.rate[n], decay.bias[n]) : acc[i][j];
-        }
-    return;
-  }
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) sc[ty * 4 + i][tx * 4 + j] = acc[i][j];
-  __syncthreads();
-  for (int i = tid; i < FM * FN / 2; i += 256) {
-    const int r = i / (FN / 2), o = i % (FN / 2), c = (o >> 3) * 16 + (o & 7);
-    if (m0 + r < M && n0 + c < N)
-      reinterpret_cast<float *>(glu.dst)[(size_t)(m0 + r) * glu.stride + n0 / 2 + o] = glu_act(sc[r][c], sc[r][c + 8], glu);
-  }
-}
-
 GluArgs glu_args(const GluOut *g) {
   GluArgs a = {nullptr, 0, 0.0f, 0.0f, 0.0f};
   if (g) { a.dst = g->dst; a.stride = g->stride; a.limit = g->limit; a.slope = g->slope; a.shift = g->shift; }
@@ -331,13 +263,4 @@ dp_status dpk_gemm_f16_tc(dp_ctx *ctx, const __half *W, int w_stride, const __ha
   TcArgs a = {};
   a.C16 = C; a.c_stride = c_stride; a.M = M; a.N = N; a.K = K;
   return launch_tc(ctx, W, w_stride, A, a_stride, a);
-}
-
-dp_status dpk_gemm_bf16w_f32(dp_ctx *ctx, const __nv_bfloat16 *W, int w_stride, const float *A, int a_stride, float *C, int M, int N, int K,
-                             const GluOut *glu, const DecayOut *decay) {
-  DP_CHECK(ctx, M > 0 && N > 0 && K > 0, "gemm (bf16 weights, f32): bad shape");
-  DP_CHECK(ctx, !glu || N % 16 == 0, "gemm (bf16): gate and up rows come in groups of sixteen");
-  DP_LAUNCH(ctx, gemm_bf16w_f32_kernel, dim3((N + FN - 1) / FN, (M + FM - 1) / FM), 256, 0, W, w_stride, A, a_stride, C, M, N, K, glu_args(glu),
-            decay ? *decay : DecayOut());
-  return DP_OK;
 }
