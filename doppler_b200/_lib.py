@@ -176,6 +176,7 @@ SIGNATURES = {
     "dp_model_load_embed": (_i, [_vp, _vp, _i, _i]),
     "dp_model_load_lm_head": (_i, [_vp, _vp, _i, _i]),
     "dp_model_reset": (_i, [_vp]),
+    "dp_model_prefill_many": (_i, [_vp, _i, _vp, _vp, _vp, _vp]),
     "dp_model_prefill": (_i, [_vp, _i, _vp, _i, C.POINTER(C.c_int32)]),
     "dp_model_decode": (_i, [_vp, _i, _vp, _i, _vp]),
     "dp_model_extend": (_i, [_vp, _i, _vp, _i, _vp, _i, _vp]),

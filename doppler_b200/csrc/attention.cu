@@ -386,11 +386,16 @@ dp_status dpk_attention_split_only(dp_ctx *ctx, const dpk_attn_params &p, float 
 bool dpk_attention_prefill_eligible(const dpk_attn_params &p);
 dp_status dpk_attention_prefill(dp_ctx *ctx, const dpk_attn_params &p);
 
+// several causal query rows: one CTA per tile of query positions shares each K / V tile (DP_ATTN_TC=0: off)
+bool dpk_attention_uses_prefill(const dpk_attn_params &p) {
+  static const int tc_mode = [] { const char *e = getenv("DP_ATTN_TC"); return e ? atoi(e) : 1; }();
+  return tc_mode && (p.k2 || f16_square(p)) && dpk_attention_prefill_eligible(p);
+}
+
 static dp_status attention_impl(dp_ctx *ctx, const dpk_attn_params &p, float *scratch, int splits, bool combine) {
   int gt = 1;
-  // several causal query rows: one CTA per tile of query positions shares each K / V tile (DP_ATTN_TC=0: off)
-  static const int tc_mode = [] { const char *e = getenv("DP_ATTN_TC"); return e ? atoi(e) : 1; }();
-  if (tc_mode && combine && (p.k2 || f16_square(p)) && dpk_attention_prefill_eligible(p)) return dpk_attention_prefill(ctx, p);
+  if (combine && dpk_attention_uses_prefill(p)) return dpk_attention_prefill(ctx, p);
+  if (p.spans) return dp_fail(ctx, DP_ERR_UNSUPPORTED, "attention: packed portions run on the prefill kernel only");
   if (p.k2) return dp_fail(ctx, DP_ERR_UNSUPPORTED, "attention: keys in two parts run on the prefill kernel only");
   if (dpk_attention_latent_eligible(ctx, p)) {
     DP_TRY(dpk_attention_latent(ctx, p, scratch, splits));

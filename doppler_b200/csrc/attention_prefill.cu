@@ -68,25 +68,33 @@ __global__ void __launch_bounds__(APF_THREADS, 1) attn_prefill_tc_kernel(dpk_att
   const int lin = blockIdx.x + gridDim.x * blockIdx.y;
   const int kvh = lin % p.num_kv_heads, b = blockIdx.z;
   const int qtile = (int)gridDim.x - 1 - lin / p.num_kv_heads;
+  // a portion of its own per batch index: packed rows, its sequence in the cache, its position
+  int seq_len = p.seq_len, start_pos = p.start_pos, cb = b;
+  size_t row0 = (size_t)b * p.seq_len;
+  if (EXACT && p.spans) {
+    const int4 span = __ldg(p.spans + b);
+    row0 = (size_t)span.x; seq_len = span.y; cb = span.z; start_pos = span.w;
+    if (qtile * QT >= seq_len) return;
+  }
   const int hh = warp % G, rb = warp / G;         // this warp: head hh of the group, 16-row block rb of the tile
   const int h = kvh * G + hh;
   const int q0 = qtile * QT + rb * 16;       // first query row (within the call) of this warp
   const int rowA = q0 + g, rowB = q0 + g + 8;     // the two query rows this lane's accumulators belong to
-  const int posA = p.start_pos + rowA, posB = p.start_pos + rowB;  // their absolute positions
+  const int posA = start_pos + rowA, posB = start_pos + rowB;  // their absolute positions
   // keys this CTA needs: up to the position of its last query (and what the cache holds)
   int kv_len = p.kv_lens ? min(max(p.kv_lens[b], 0), p.kv_len) : p.kv_len;
-  const int last_q = min(qtile * QT + QT, p.seq_len) - 1;
-  const int cta_keys = min(kv_len, p.start_pos + last_q + 1);
-  const int warp_keys = min(kv_len, p.start_pos + min(q0 + 15, p.seq_len - 1) + 1);  // beyond this every key is masked for the warp
+  const int last_q = min(qtile * QT + QT, seq_len) - 1;
+  const int cta_keys = min(kv_len, start_pos + last_q + 1);
+  const int warp_keys = min(kv_len, start_pos + min(q0 + 15, seq_len - 1) + 1);  // beyond this every key is masked for the warp
   const int n_tiles = (cta_keys + APF_KT - 1) / APF_KT;
   // chunked attention: a row sees no key before its own chunk, a CTA (a warp) none before its first row's chunk
   const int loA = p.chunk > 0 ? posA / p.chunk * p.chunk : 0, loB = p.chunk > 0 ? posB / p.chunk * p.chunk : 0;
-  const int tile0 = p.chunk > 0 ? (p.start_pos + qtile * QT) / p.chunk * p.chunk / APF_KT : 0;
-  const int warp_lo = p.chunk > 0 ? (p.start_pos + q0) / p.chunk * p.chunk : 0;
+  const int tile0 = p.chunk > 0 ? (start_pos + qtile * QT) / p.chunk * p.chunk / APF_KT : 0;
+  const int warp_lo = p.chunk > 0 ? (start_pos + q0) / p.chunk * p.chunk : 0;
 
-  const __half *kbase = p.k + (size_t)b * p.kv_batch_stride + (size_t)kvh * k_pieces * 8;
-  const __half *vbase = p.v + (size_t)b * (p.v_batch_stride ? p.v_batch_stride : p.kv_batch_stride) + (size_t)kvh * v_pieces * 8;
-  const __half *k2base = p.k2 + (size_t)b * p.k2_batch_stride;
+  const __half *kbase = p.k + (size_t)cb * p.kv_batch_stride + (size_t)kvh * k_pieces * 8;
+  const __half *vbase = p.v + (size_t)cb * (p.v_batch_stride ? p.v_batch_stride : p.kv_batch_stride) + (size_t)kvh * v_pieces * 8;
+  const __half *k2base = p.k2 + (size_t)cb * p.k2_batch_stride;
   // elements between consecutive keys
   const size_t key_stride = !EXACT && p.k_row_stride ? (size_t)p.k_row_stride : (size_t)p.num_kv_heads * D, val_stride = !EXACT && p.v_row_stride ? (size_t)p.v_row_stride : (size_t)p.num_kv_heads * V;
   const uint32_t smem0 = (uint32_t)__cvta_generic_to_shared(apf_smem);
@@ -122,9 +130,9 @@ __global__ void __launch_bounds__(APF_THREADS, 1) attn_prefill_tc_kernel(dpk_att
   const float qmul = p.scale * LOG2E;  // scores in log2 units: softmax with exp2
   uint32_t qh[KS][4], ql[KS][4];
   {
-    const bool okA = rowA < p.seq_len, okB = rowB < p.seq_len;
-    const float *qa = p.q + (((size_t)b * p.seq_len + (okA ? rowA : 0)) * p.num_heads + h) * D;
-    const float *qb = p.q + (((size_t)b * p.seq_len + (okB ? rowB : 0)) * p.num_heads + h) * D;
+    const bool okA = rowA < seq_len, okB = rowB < seq_len;
+    const float *qa = p.q + ((row0 + (okA ? rowA : 0)) * p.num_heads + h) * D;
+    const float *qb = p.q + ((row0 + (okB ? rowB : 0)) * p.num_heads + h) * D;
     // a pair of dims where the keys have them: both parts of a key are padded to whole pieces, the query is not
     auto pair = [&](const float *q, bool ok, int d) {
       float2 v = make_float2(0.0f, 0.0f);
@@ -239,9 +247,9 @@ __global__ void __launch_bounds__(APF_THREADS, 1) attn_prefill_tc_kernel(dpk_att
 #pragma unroll
   for (int half = 0; half < 2; half++) {
     const int row = half ? rowB : rowA;
-    if (row >= p.seq_len) continue;
+    if (row >= seq_len) continue;
     const float l = half ? lB : lA;
-    const size_t z = (size_t)b * p.seq_len + row;
+    const size_t z = row0 + row;
     float inv = l > 0.0f ? 1.0f / l : 0.0f;
     if (p.gate) inv *= 1.0f / (1.0f + expf(-p.gate[z * p.gate_stride + h]));
     const bool whole = (V & 1) == 0;  // pairs do not straddle the end
@@ -281,6 +289,7 @@ bool dpk_attention_prefill_eligible(const dpk_attn_params &p) {
   if (G != 1 && G != 2 && G != 4 && G != 8) return false;
   if (p.sliding_window > 0 || p.softcap > 0.0f || p.kv_start != 0) return false;
   if (p.kv_batch_stride % 8 || (((uintptr_t)p.k | (uintptr_t)p.v) & 15) || ((uintptr_t)p.q & 7) || ((uintptr_t)p.out & 7)) return false;
+  if (p.spans && (p.k2 || p.kv_lens || p.chunk)) return false;
   if (p.out_bf16 && (p.out_stride % 2 || ((uintptr_t)p.out_bf16 & 3))) return false;
   return true;
 }

@@ -247,11 +247,15 @@ struct dpk_attn_params {
   // output gate: row r's head h times sigmoid(gate[r * gate_stride + h]); null: none (kernels that write `out` only)
   const float *gate = nullptr;
   int gate_stride = 0;
+  // prefill kernel: the batch is `batch` portions packed row after row; seq_len is the longest.  spans[b]: first row, rows,
+  // index of the sequence in k and v, position of the first row (null: batch portions of seq_len rows at start_pos)
+  const int4 *spans = nullptr;
   __nv_bfloat16 *out_bf16 = nullptr;  // rows of out_stride elements, written instead of `out`
   int out_stride = 0;
 };
 dp_status dpk_attention(dp_ctx *ctx, const dpk_attn_params &p);
 bool dpk_attention_uses_tc(dp_ctx *ctx, const dpk_attn_params &p);
+bool dpk_attention_uses_prefill(const dpk_attn_params &p);
 // variant with caller-provided scratch (no allocation); scratch_bytes must cover dpk_attention_scratch_bytes
 size_t dpk_attention_scratch_bytes(dp_ctx *ctx, const dpk_attn_params &p, int *splits_out);
 dp_status dpk_attention_with_scratch(dp_ctx *ctx, const dpk_attn_params &p, float *scratch, int splits);

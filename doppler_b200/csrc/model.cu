@@ -58,7 +58,7 @@ dp_status dp_take_dev_status(dp_ctx *ctx);
 __global__ void __launch_bounds__(256) qk_norm_rope_kv_kernel(
     const float *__restrict__ qkv, float *__restrict__ q_out, __half *__restrict__ kc, __half *__restrict__ vc,
     const float *__restrict__ q_norm, const float *__restrict__ k_norm, const float *__restrict__ cos_t,
-    const float *__restrict__ sin_t, const int *__restrict__ pos_arr, int start_pos, int seq, int tokens, int nh,
+    const float *__restrict__ sin_t, const int *__restrict__ pos_arr, const int *__restrict__ seq_arr, int start_pos, int seq, int tokens, int nh,
     int nkv, int D, float eps, size_t kv_seq_stride) {
   pdl_launch();
   pdl_wait();
@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(256) qk_norm_rope_kv_kernel(
   if (gw >= tokens * heads) return;
   const int t = gw / heads, hd = gw % heads;
   const int pos = pos_arr ? pos_arr[t] : start_pos + t;
-  const int sq = pos_arr ? t : seq;
+  const int sq = seq_arr ? seq_arr[t] : pos_arr ? t : seq;
   const float *src = qkv + (size_t)t * heads * D + (size_t)hd * D;
   const int half = D / 2, per = half / 32;  // pairs per lane
   float x0[4], x1[4];
@@ -883,6 +883,11 @@ static dp_status run_layers(dp_model *m, int tokens, bool decode, int seq, int s
       ap.batch = 1; ap.seq_len = tokens; ap.kv_len = start_pos + tokens; ap.causal = 1; ap.start_pos = start_pos;
       ap.kv_batch_stride = 0; ap.kv_lens = nullptr;
       splits = 1;
+      if (m->packed) {
+        ap.k = (const __half *)m->kc[l]->dptr; ap.v = (const __half *)m->vc[l]->dptr;
+        ap.batch = m->packed->portions; ap.seq_len = m->packed->longest < 2 ? 2 : m->packed->longest; ap.kv_len = c.max_seq; ap.start_pos = 0;
+        ap.kv_batch_stride = kv_seq_stride; ap.spans = m->packed->spans;
+      }
     }
     // ---- per-head QK norm, RoPE, KV append ----
     // Decode on the tensor-core attention kernel: that kernel does it itself (one launch less per layer).
@@ -896,8 +901,8 @@ static dp_status run_layers(dp_model *m, int tokens, bool decode, int seq, int s
     } else {
       const int warps = tokens * heads;
       DP_LAUNCH(ctx, qk_norm_rope_kv_kernel, (warps + 7) / 8, 256, 0, m->qkv, m->q, (__half *)m->kc[l]->dptr,
-                (__half *)m->vc[l]->dptr, L.q_norm, L.k_norm, m->rope_cos, m->rope_sin, decode ? m->d_pos : nullptr,
-                start_pos, seq, tokens, m->nh, m->nkv, D, c.eps, kv_seq_stride);
+                (__half *)m->vc[l]->dptr, L.q_norm, L.k_norm, m->rope_cos, m->rope_sin,
+                decode ? m->d_pos : m->packed ? m->packed->pos : nullptr, m->packed ? m->packed->seq : nullptr, start_pos, seq, tokens, m->nh, m->nkv, D, c.eps, kv_seq_stride);
     }
     float *o_dst = p == 1 ? m->h : m->partial;
     const float *o_res = p == 1 ? m->h : nullptr;
@@ -1118,6 +1123,104 @@ extern "C" dp_status dp_model_prefill(dp_model *m, int seq, const int32_t *token
   int32_t tok = 0;
   DP_TRY(run_portion(m, "prefill", seq, tokens, n, nullptr, 0, nullptr, &tok));
   if (next_token) *next_token = tok;
+  return DP_OK;
+}
+
+// out[i] = rows[at[i]]
+__global__ void __launch_bounds__(256) take_rows_kernel(const float *__restrict__ rows, const int *__restrict__ at, float *__restrict__ out, int width) {
+  pdl_launch();
+  pdl_wait();
+  const float4 *src = reinterpret_cast<const float4 *>(rows + (size_t)at[blockIdx.x] * width);
+  float4 *dst = reinterpret_cast<float4 *>(out + (size_t)blockIdx.x * width);
+  for (int i = threadIdx.x; i < width / 4; i += 256) dst[i] = src[i];
+}
+
+// Prompts of a call that fit the activation rows together, in one pass over the layers: the packed weights are read and
+// turned into tiles once instead of once per prompt.  The LAST prompt comes first, so that afterwards the hidden rows and
+// the logits start with it, as they do when prompts run one after the other.
+static dp_status run_packed(dp_model *m, const int32_t *seqs, const int32_t *const *tokens, const int32_t *lengths, int n, int32_t *next_tokens) {
+  dp_ctx *ctx = m->ctx;
+  const dp_model_cfg &c = m->cfg;
+  int rows = 0, longest = 0;
+  for (int i = 0; i < n; i++) {
+    rows += lengths[i];
+    if (lengths[i] > longest) longest = lengths[i];
+  }
+  // one upload: ids | positions | sequences of the rows | last row of every portion | spans
+  const size_t spans_at = ((size_t)3 * rows + n + 3) / 4 * 4;
+  std::vector<int> host(spans_at + (size_t)4 * n);
+  int *ids = host.data(), *pos = ids + rows, *seq = pos + rows, *last = seq + rows, *span = ids + spans_at;
+  int r = 0;
+  for (int k = 0; k < n; k++) {
+    const int i = n - 1 - k, start = m->seq_len[seqs[i]];
+    span[4 * k] = r; span[4 * k + 1] = lengths[i]; span[4 * k + 2] = seqs[i]; span[4 * k + 3] = start;
+    for (int j = 0; j < lengths[i]; j++, r++) { ids[r] = tokens[i][j]; pos[r] = start + j; seq[r] = seqs[i]; }
+    last[k] = r - 1;
+  }
+  dp_buf buf = nullptr;
+  DP_TRY(dp_buf_acquire(ctx, host.size() * 4, "packed_rows", &buf));
+  const int *dev = (const int *)buf->dptr;
+  const PackedRows packed = {dev + rows, dev + 2 * rows, (const int4 *)(dev + spans_at), n, longest};
+  auto run = [&]() -> dp_status {
+    DP_TRY(dp_buf_upload(ctx, buf, host.data(), 0, host.size() * 4));
+    DP_TRY(embed_rows(m, dev, rows, false));
+    m->packed = &packed;
+    const dp_status st = run_layers(m, rows, false, 0, 0);
+    m->packed = nullptr;
+    DP_TRY(st);
+    DP_LAUNCH(ctx, take_rows_kernel, (unsigned)n, 256, 0, (const float *)m->h, dev + 3 * rows, m->partial, c.hidden);
+    return run_head(m, m->partial, n);
+  };
+  const dp_status st = run();
+  dp_buf_release(ctx, buf);
+  DP_TRY(st);
+  for (int i = 0; i < n; i++) m->seq_len[seqs[i]] += lengths[i];
+  std::vector<int> tok(n);
+  DP_CUDA(ctx, cudaMemcpyAsync(tok.data(), m->d_tok, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream));
+  DP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  DP_TRY(dp_take_dev_status(ctx));
+  for (int k = 0; k < n; k++) next_tokens[n - 1 - k] = tok[k];
+  return DP_OK;
+}
+
+// whether prompts of this model can share a pass: the dense decoder on one GPU, on the attention kernel that takes packed rows
+static bool packs(dp_model *m) {
+  if (m->stack || m->cfg.tp_size != 1 || m->cfg.max_batch < 2) return false;
+  dpk_attn_params ap{};
+  int4 any;
+  ap.q = m->q; ap.out = m->att;
+  ap.k = (const __half *)m->kc[0]->dptr; ap.v = (const __half *)m->vc[0]->dptr;
+  ap.num_heads = m->nh; ap.num_kv_heads = m->nkv; ap.head_dim = m->cfg.head_dim;
+  ap.batch = 2; ap.seq_len = 2; ap.kv_len = m->cfg.max_seq; ap.causal = 1;
+  ap.kv_batch_stride = (size_t)m->cfg.max_seq * m->kvdim; ap.spans = &any;
+  return dpk_attention_uses_prefill(ap);
+}
+
+extern "C" dp_status dp_model_prefill_many(dp_model *m, int n, const int32_t *seqs, const int32_t *tokens, const int32_t *lengths, int32_t *next_tokens) {
+  if (!m) return DP_ERR_INVALID;
+  dp_ctx *ctx = m->ctx;
+  DP_CHECK(ctx, n > 0 && seqs && tokens && lengths && next_tokens, "prefill: no prompts or a null pointer");
+  std::vector<const int32_t *> at(n);
+  std::vector<char> used(m->cfg.max_batch, 0);
+  for (int i = 0; i < n; i++) {
+    at[i] = i ? at[i - 1] + lengths[i - 1] : tokens;
+    DP_CHECK(ctx, seqs[i] >= 0 && seqs[i] < m->cfg.max_batch && !used[seqs[i]], "prefill: sequence %d outside [0,%d) or named twice", seqs[i], m->cfg.max_batch);
+    used[seqs[i]] = 1;
+    DP_CHECK(ctx, lengths[i] > 0, "prefill: empty prompt");
+    DP_CHECK(ctx, lengths[i] <= m->cfg.max_seq - m->seq_len[seqs[i]], "prefill: %d + %d tokens exceed max_seq %d", m->seq_len[seqs[i]], lengths[i], m->cfg.max_seq);
+    for (int j = 0; j < lengths[i]; j++)
+      DP_CHECK(ctx, at[i][j] >= 0 && at[i][j] < m->cfg.vocab, "prefill: token id %d outside the vocabulary", at[i][j]);
+  }
+  // (up to 64 rows: the small-batch kernel multiplies with exact weights, the one for more rows with weights of 22 bits)
+  const bool pack = packs(m);
+  const int most = m->T < 64 ? m->T : 64;
+  for (int i = 0; i < n;) {
+    int e = i + 1, rows = lengths[i];
+    while (pack && e < n && rows + lengths[e] <= most) rows += lengths[e++];
+    if (e - i > 1) DP_TRY(run_packed(m, seqs + i, at.data() + i, lengths + i, e - i, next_tokens + i));
+    else DP_TRY(run_portion(m, "prefill", seqs[i], at[i], lengths[i], nullptr, 0, nullptr, next_tokens + i));
+    i = e;
+  }
   return DP_OK;
 }
 

@@ -11,6 +11,13 @@ struct LayerW {
   float *in_norm = nullptr, *post_norm = nullptr, *q_norm = nullptr, *k_norm = nullptr;
 };
 
+// Portions of several sequences packed row after row into one pass over the layers (device arrays)
+struct PackedRows {
+  const int *pos, *seq;  // of every row
+  const int4 *spans;     // of every portion: first row, rows, sequence, position of the first row
+  int portions, longest;
+};
+
 struct dp_model {
   dp_ctx *ctx;
   dp_model_cfg cfg;
@@ -43,6 +50,7 @@ struct dp_model {
   bool recording_decode = false;  // set while a decode step is recorded into its CUDA graph
   bool fuse_qk = true;  // decode: QK norm + RoPE + KV append inside the attention kernel
   std::vector<int> seq_len;
+  const PackedRows *packed = nullptr;  // set while run_layers runs such a pass
   dp_graph *graph[2] = {nullptr, nullptr};
   int graph_batch[2] = {0, 0};
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;

@@ -39,6 +39,15 @@ class Runner:
         self.device.check(self.device.lib.dp_model_prefill(self.h, seq, t.ctypes.data_as(C.c_void_p), t.size, C.byref(nxt)))
         return int(nxt.value)
 
+    def prefill_many(self, prompts, seqs) -> list:
+        """The greedy tokens after several prompts, one per sequence of ``seqs``; short ones share passes over the layers."""
+        parts = [np.asarray(p, np.int32) for p in prompts]
+        t = np.ascontiguousarray(np.concatenate(parts)) if parts else np.empty(0, np.int32)
+        n, s, out = np.array([p.size for p in parts], np.int32), np.ascontiguousarray(seqs, np.int32), np.empty(len(parts), np.int32)
+        self.device.check(self.device.lib.dp_model_prefill_many(self.h, len(parts), s.ctypes.data_as(C.c_void_p), t.ctypes.data_as(C.c_void_p),
+                                                                n.ctypes.data_as(C.c_void_p), out.ctypes.data_as(C.c_void_p)))
+        return out.tolist()
+
     def decode(self, first_tokens, steps: int) -> np.ndarray:
         """Greedy decode; returns int32 [steps, batch]."""
         ft = np.ascontiguousarray(np.atleast_1d(first_tokens), np.int32)

@@ -64,7 +64,10 @@ class Scheduler:
                 continue
             for i in range(len(group)):
                 m.release(i)
-            done = [[m.prefill(p, seq=i)] for i, p in enumerate(group)]
+            if len(group) > 1 and hasattr(m, "prefill_many"):
+                done = [[t] for t in m.prefill_many(group, range(len(group)))]
+            else:
+                done = [[m.prefill(p, seq=i)] for i, p in enumerate(group)]
             left = max_new_tokens - 1
             while left > 0 and not all(stop.intersection(d) for d in done):
                 room = min(m.cfg["max_seq"] - m.seq_len(i) for i in range(len(group)))

@@ -347,6 +347,10 @@ dp_status dp_model_load_lm_head(dp_model *m, const void *host_f16, int row0, int
 dp_status dp_model_reset(dp_model *m);
 /* prompt of n tokens for sequence `seq`; next_token receives the greedy token */
 dp_status dp_model_prefill(dp_model *m, int seq, const int32_t *tokens, int n, int32_t *next_token);
+/* the same for n prompts of n different sequences: tokens holds them one behind the other, lengths[i] of them for
+ * sequence seqs[i].  Short prompts share passes over the layers.  Nothing runs if one of them is invalid. */
+dp_status dp_model_prefill_many(dp_model *m, int n, const int32_t *seqs, const int32_t *tokens, const int32_t *lengths,
+                                int32_t *next_tokens);
 /* `steps` greedy decode steps for `batch` sequences; out_tokens is [steps][batch] */
 dp_status dp_model_decode(dp_model *m, int batch, const int32_t *first_tokens, int steps,
                           int32_t *out_tokens);
