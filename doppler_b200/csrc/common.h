@@ -194,11 +194,15 @@ struct dpk_tc_fuse {
   float *residual_out = nullptr;    // ... which then writes here (may be the residual itself) instead of C
   const float *norm_w = nullptr;    // RMSNorm weights: A holds the un-normalised rows and the norm is folded into their conversion to f16
   float eps = 0.0f;                 //   (the call is left unhandled, nothing launched, where that conversion cannot take it)
+  bool exact_weights = false;       // the integer-tile kernel at any size
   bool silu_done = false, residual_done = false;
 };
 dp_status dpk_gemm_q4k_tc_rowscaled(dp_ctx *ctx, const uint8_t *W, const float *A, float *C, int M, int N, int K, float alpha, int passes,
                                     bool *handled, dpk_tc_fuse *fuse = nullptr);
 
+// any N and K, integer weight tiles (gemm_q4k_int.cu)
+dp_status dpk_gemm_q4k_int(dp_ctx *ctx, const uint8_t *W, const void *A, dp_dtype a_dtype, void *C, dp_dtype c_dtype, int M, int N, int K, float alpha,
+                           bool *handled, dpk_tc_fuse *fuse = nullptr);
 dp_status dpk_gemm_q4k_tc_rows(dp_ctx *ctx, const uint8_t *W, const void *A, dp_dtype a_dtype, float *C, int M, int N, int K, float alpha,
                                bool *handled, const dpk_rows_fuse *fuse = nullptr);
 dp_status dpk_scale_cast_rows(dp_ctx *ctx, const float *A, __half *hi, __half *lo, float *row_scale, int M, int K);

@@ -386,24 +386,6 @@ __global__ void __launch_bounds__((DQ_WARPS + 2) * 32, 1) gemm_q4k_tc_kernel(con
 // read from shared memory once per pair.  Two passes (rows 0..255 and 256..511 of the tile) share each
 // B stage.  CTA 0 issues all MMAs; all "stage full" barriers live in CTA 0 (CTA 1's TMA and dequant
 // warps signal them across the cluster), "stage free" and "accumulators ready" are multicast to both.
-__device__ __forceinline__ void umma_f16_2sm(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void umma_commit_2sm(uint32_t bar) {  // arrives on this barrier offset in both CTAs
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
-               "h"((uint16_t)3)
-               : "memory");
-}
-// tensor copy into this CTA's shared memory whose completion bytes are counted on a barrier of CTA 0
-__device__ __forceinline__ void tma_load_2d_2sm(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar_cluster_addr) {
-  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-               "l"(map), "r"(x), "r"(y), "r"(bar_cluster_addr)
-               : "memory");
-}
-
 // The tile width is a run-time value (a multiple of 16 up to BNMAX): the first `wide_tiles` clusters of a
 // grid row take `bn_wide` columns, the others `bn_narrow`.  With 28 tiles of 176 and 46 of 160 columns the
 // 74 clusters of a B200 cover N = 12288 in one even wave, where uniform 256-wide tiles fill only 48.
@@ -973,25 +955,40 @@ static dp_status gemm_q4k_tc_impl(dp_ctx *ctx, const uint8_t *W, const void *A, 
   static int enabled = -1;
   if (enabled < 0) { const char *e = getenv("DP_GEMM_TC"); enabled = e ? atoi(e) : 1; }
   if (!enabled || !ctx->dev_status) return DP_OK;
-  if (K % QK_K || M < 1) return DP_OK;
-  int bn = 0;
-  if (N % 192 == 0) bn = 192;
-  else if (N % 128 == 0) bn = 128;
-  if (!bn) return DP_OK;
-  EncodeTiledFn encode = get_encode();
-  if (!encode) return DP_OK;
-  if (mode == 3 && a_dtype != DP_F16) return DP_OK;
+  if (M < 1 || (mode == 3 && a_dtype != DP_F16)) return DP_OK;
+  const bool tiled = K % QK_K == 0 && N % 128 == 0, exact = (mode == 2 && a_dtype == DP_F32) || mode == 3;
   // an RMSNorm folded into the activation conversion: row-scaled f32 rows of 1024..4096 values on the kernels below only
   if (fuse && fuse->norm_w && !(row_scaled && a_dtype == DP_F32 && c_dtype == DP_F32 && M > 64 && K % 4 == 0 && K >= 1024 && K <= 4096 &&
                                  ((uintptr_t)fuse->norm_w & 15) == 0 && ((uintptr_t)A & 15) == 0))
     return DP_OK;
-  // up to 64 rows, f32 out, exact weights (modes 2 and 3): the integer-tile kernel (gemm_q4k_tc_rows.cu)
-  if (M <= 64 && c_dtype == DP_F32 && ((mode == 2 && a_dtype == DP_F32) || mode == 3)) {
+  // up to 64 rows, f32 out, exact weights (modes 2 and 3): the small-batch kernel (gemm_q4k_tc_rows.cu)
+  if (M <= 64 && c_dtype == DP_F32 && exact && tiled) {
     DP_TRY(dpk_gemm_q4k_tc_rows(ctx, W, A, a_dtype, (float *)C, M, N, K, alpha, handled));
     if (*handled) return DP_OK;
   }
-
-  if (M < 32 && a_dtype == DP_F32) return DP_OK;  // few f32 rows on a shape that kernel does not tile: the CUDA-core kernel
+  if (M < 32 && (a_dtype == DP_F32 || !tiled)) return DP_OK;  // few rows on a shape that kernel does not tile: the CUDA-core kernel
+  // Exact weights: the integer-tile kernel (gemm_q4k_int.cu: one product less per K step, any shape) against the tiles of
+  // dequantised weights below, which lose less between K steps.  Measured, us, dequantised -> integer tiles:
+  //   f32 rows, M x N x K   65 x 24576 x 4096 87 -> 74, 512 x 6144 x 4096 84 -> 69, 1024 x 4096 x 4096 99 -> 93, 2048 x 1024 x 3072 66 -> 53, but
+  //                         512 x 24576 x 4096 207 -> 221, 1024 x 6144 x 4096 111 -> 120, 512 x 4096 x 12288 122 -> 131, 2048 x 4096 x 4096 143 -> 152
+  //   f16 rows              128 x 12288 x 4096 79 -> 43, 256 x 4096 x 4096 74 -> 43, 512 x 4096 x 4096 73 -> 53, but 512 x 12288 x 4096 75 -> 88
+  // so it takes what fills less than half a wave of the others' 512 x 256 pair tiles and has K up to 8192; very small weights
+  // stay with the one launch that needs no pass over the rows (33 x 256 x 256: 9 against 17 us).  Shapes the others do not
+  // tile ran on CUDA cores (1000 x 1000 x 1000: 103 -> 26 us); they still do where that is over within about 15 us.
+  // fuse->exact_weights (rows of several prompts, which were multiplied with exact weights one by one): always.
+  if (exact && (c_dtype == DP_F32 || c_dtype == DP_F16)) {
+    const long pair_tiles = (long)((M + 511) / 512) * ((N + 255) / 256);
+    const bool few = M <= 256 || (pair_tiles * 2 <= ctx->sm_count / 2 && K <= 8192);
+    const bool take = tiled ? (few && (long)N * K >= (1l << 19)) || (fuse && fuse->exact_weights) : (double)M * N * K >= (double)(1l << 27);
+    if (take) {
+      DP_TRY(dpk_gemm_q4k_int(ctx, W, A, a_dtype, C, c_dtype, M, N, K, alpha, handled, fuse));
+      if (*handled) return DP_OK;
+    }
+  }
+  if (!tiled) return DP_OK;
+  const int bn = N % 192 == 0 ? 192 : 128;
+  EncodeTiledFn encode = get_encode();
+  if (!encode) return DP_OK;
   const __half *a16 = (const __half *)A;
   // The f16 copies of f32 activations live in one scratch allocation of the context, reused in stream order.
   const __half *a_lo = nullptr;

@@ -668,6 +668,7 @@ static dp_status q4k_linear(dp_model *m, const uint8_t *W, const float *x, float
   // context and is never recycled while a graph is alive)
   dpk_tc_fuse f;
   f.silu_dst = silu_dst;
+  f.exact_weights = m->packed != nullptr;
   if (residual) { f.residual = residual; f.residual_out = y; }  // a K-split launch adds it in its reduction, in place
   if (norm_w) {
     if (prefill_tc) {
@@ -1211,12 +1212,10 @@ extern "C" dp_status dp_model_prefill_many(dp_model *m, int n, const int32_t *se
     for (int j = 0; j < lengths[i]; j++)
       DP_CHECK(ctx, at[i][j] >= 0 && at[i][j] < m->cfg.vocab, "prefill: token id %d outside the vocabulary", at[i][j]);
   }
-  // (up to 64 rows: the small-batch kernel multiplies with exact weights, the one for more rows with weights of 22 bits)
   const bool pack = packs(m);
-  const int most = m->T < 64 ? m->T : 64;
   for (int i = 0; i < n;) {
     int e = i + 1, rows = lengths[i];
-    while (pack && e < n && rows + lengths[e] <= most) rows += lengths[e++];
+    while (pack && e < n && rows + lengths[e] <= m->T) rows += lengths[e++];
     if (e - i > 1) DP_TRY(run_packed(m, seqs + i, at.data() + i, lengths + i, e - i, next_tokens + i));
     else DP_TRY(run_portion(m, "prefill", seqs[i], at[i], lengths[i], nullptr, 0, nullptr, next_tokens + i));
     i = e;

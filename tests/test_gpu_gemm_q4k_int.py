@@ -1,0 +1,64 @@
+"""The integer-tile Q4_K GEMM at the edges of its tiles, sum units and rows, against 64-bit products of the same blocks."""
+import numpy as np
+import pytest
+
+from doppler_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+
+def blocks(rng, n, bpr):
+    """Random packed rows: every code, scales over six orders of magnitude, some super-blocks without scale or minimum."""
+    b = rng.integers(0, 256, (n, bpr, 144), dtype=np.uint8)
+    dd = (rng.choice([-1.0, 1.0, 1.0], (n, bpr, 2)) * 10.0 ** rng.uniform(-4, 2, (n, bpr, 2))).astype(np.float16)
+    dd[rng.random((n, bpr, 2)) < 0.1] = 0.0
+    b[:, :, :4] = dd.view(np.uint8).reshape(n, bpr, 4)
+    return b
+
+
+def parts(b):
+    """d sc q and dmin m of every weight, 64 bits"""
+    n, bpr, _ = b.shape
+    dd = np.ascontiguousarray(b[:, :, :4]).view(np.float16).astype(np.float64)
+    s = b[:, :, 4:16].astype(np.int64)
+    sc = np.concatenate([s[..., :4] & 63, (s[..., 8:] & 15) | (s[..., :4] >> 6 << 4)], -1)
+    mn = np.concatenate([s[..., 4:8] & 63, (s[..., 8:] >> 4) | (s[..., 4:8] >> 6 << 4)], -1)
+    qs = b[:, :, 16:].reshape(n, bpr, 4, 32)
+    q = np.stack([qs & 15, qs >> 4], 3).reshape(n, bpr, 8, 32)
+    x = dd[..., :1, None] * (sc[..., None] * q)
+    m = np.broadcast_to((dd[..., 1:] * mn)[..., None], x.shape)
+    return x.reshape(n, -1), m.reshape(n, -1)
+
+
+def run(dev, b, n, k, a, out, **opt):
+    w, t = dev.weight_from(b.ravel(), "q4k", [n, k]), dev.tensor_from(a)
+    c = ops.run_matmul(t, w, a.shape[0], n, k, output_dtype=out, **opt)
+    got = dev.read_tensor(c).astype(np.float64).reshape(a.shape[0], n)
+    for x in (c.buffer, t.buffer, w.buffer):
+        dev.release_buffer(x)
+    return got
+
+
+@pytest.mark.parametrize("act,out", [("f32", "f32"), ("f16", "f32"), ("f16", "f16")])
+@pytest.mark.parametrize("m,n,k", [(65, 2048, 256), (65, 256, 2560), (66, 384, 2816), (127, 257, 5120), (700, 700, 300), (1024, 5, 26500), (513, 1030, 264), (33, 4095, 1000),
+                                   (300, 1000, 5376), (513, 2048, 1024), (1024, 520, 4097), (256, 1024, 8192), (32, 2049, 4104)])
+def test_edges(dev, m, n, k, act, out):
+    rng = np.random.default_rng(m * 7 + n * 3 + k)
+    b = blocks(rng, n, -(-k // 256))
+    a = rng.standard_normal((m, k)) * 10.0 ** rng.uniform(-3, 3, (m, 1))
+    if act == "f16":
+        a = a / 100.0
+    a = a.astype(np.float32 if act == "f32" else np.float16)
+    x, mn = (p[:, :k] for p in parts(b))
+    a64 = a.astype(np.float64)
+    want, size = a64 @ (x - mn).T, np.abs(a64) @ (np.abs(x) + np.abs(mn)).T
+    # rows and sub-block sums enter with 22 bits, a super-block's sums and the additions of super-blocks with f32's 24:
+    # 2^-22 + (16 + blocks) 2^-24 of the sum of magnitudes
+    tol = (2.0 ** -22 + (16 + b.shape[1] * 1.1 + 2) * 2.0 ** -24) * size
+    if out == "f16":
+        tol = tol + np.abs(want) * 2.0 ** -11 + 2.0 ** -25
+    got = run(dev, b, n, k, a, out, alpha=0.5)
+    want, tol = 0.5 * want, 0.5 * tol + (2.0 ** -25 if out == "f16" else 0.0)
+    fits = np.abs(want) < 65000.0 if out == "f16" else np.ones_like(want, bool)
+    assert (np.abs(got - want)[fits] <= tol[fits]).all(), np.max((np.abs(got - want) / tol)[fits])
+    assert np.array_equal(got, run(dev, b, n, k, a, out, alpha=0.5))  # nothing depends on timing
