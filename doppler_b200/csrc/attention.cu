@@ -182,7 +182,8 @@ __global__ void __launch_bounds__(ATT_THREADS, LPK == 16 ? 2 : 1) attn_split_ker
 }
 
 // Any query/key size and any value size up to 32 * MAXE, any GQA ratio, f16 or f32 caches: one CTA per (split, query
-// head, row), lanes over dims.  Used for shapes outside the fast kernels.
+// head, row), lanes over dims.  Used for shapes outside the fast kernels.  Bound: instructions per key; MAXE is the least
+// that holds the head sizes (a 700-token prompt in 32 bits, 16 heads of 128, with MAXE 16 for all sizes: 800 us).
 template <typename KT, int MAXE>
 __global__ void __launch_bounds__(128) attn_split_generic_kernel(dpk_attn_params p, float *__restrict__ part, int splits) {
   pdl_launch();
@@ -208,6 +209,7 @@ __global__ void __launch_bounds__(128) attn_split_generic_kernel(dpk_attn_params
   const size_t k_stride = (size_t)p.num_kv_heads * D, v_stride = p.v_row_stride ? (size_t)p.v_row_stride : (size_t)p.num_kv_heads * V;
   const KT *kb = reinterpret_cast<const KT *>(p.k) + (size_t)b * p.kv_batch_stride + (size_t)kvh * D;
   const KT *vb = reinterpret_cast<const KT *>(p.v) + (size_t)b * (p.v_batch_stride ? p.v_batch_stride : p.kv_batch_stride) + (size_t)kvh * V;
+#pragma unroll 2
   for (int key = k_begin + warp; key < k_end; key += 4) {
     float a = 0.0f;
 #pragma unroll
@@ -415,13 +417,14 @@ static dp_status attention_impl(dp_ctx *ctx, const dpk_attn_params &p, float *sc
     dim3 grid(splits, p.num_heads, p.batch * p.seq_len);
     const int most = p.head_dim > p.v_dim ? p.head_dim : p.v_dim;
     if (most > 1024) return dp_fail(ctx, DP_ERR_UNSUPPORTED, "attention: head sizes above 1024");
-    if (most > 512) {
-      if (p.kv_f32) DP_LAUNCH(ctx, (attn_split_generic_kernel<float, 32>), grid, 128, 0, p, scratch, splits);
-      else DP_LAUNCH(ctx, (attn_split_generic_kernel<__half, 32>), grid, 128, 0, p, scratch, splits);
-    } else {
-      if (p.kv_f32) DP_LAUNCH(ctx, (attn_split_generic_kernel<float, 16>), grid, 128, 0, p, scratch, splits);
-      else DP_LAUNCH(ctx, (attn_split_generic_kernel<__half, 16>), grid, 128, 0, p, scratch, splits);
-    }
+#define DP_GENERIC(E)                                                                                                  \
+  if (p.kv_f32) DP_LAUNCH(ctx, (attn_split_generic_kernel<float, E>), grid, 128, 0, p, scratch, splits);              \
+  else DP_LAUNCH(ctx, (attn_split_generic_kernel<__half, E>), grid, 128, 0, p, scratch, splits)
+    if (most <= 128) { DP_GENERIC(4); }
+    else if (most <= 256) { DP_GENERIC(8); }
+    else if (most <= 512) { DP_GENERIC(16); }
+    else { DP_GENERIC(32); }
+#undef DP_GENERIC
   }
   if (splits > 1 && combine) {
     const unsigned rows = (unsigned)((long)p.batch * p.seq_len * p.num_heads);
