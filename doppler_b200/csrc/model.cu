@@ -135,6 +135,66 @@ __global__ void advance_kernel(int *pos, int *kvlen, const int *tok, int *step, 
 }
 
 
+// The end of a decode step of one sequence in one launch: greedy token (ties to the lower index, as sample.wgsl:311-408),
+// token record, position.  Three dependent launches of a few hundred threads each (two argmax phases, advance_kernel) were
+// 8 us of every step; the block that finishes last does what the second and third did.  `arrived` is 0 before and after.
+__device__ __forceinline__ void pick_better(float &v, int &i, float cv, int ci) {
+  if (cv > v || (cv == v && ci < i)) { v = cv; i = ci; }
+}
+__global__ void __launch_bounds__(256) pick_advance_kernel(const float *__restrict__ logits, int n, float *vals, int *idxs, int *arrived, int *pos, int *kvlen, int *tok,
+                                                           int *step, int *out_tokens, unsigned *ticket) {
+  pdl_launch();
+  pdl_wait();
+  __shared__ float sv[8];
+  __shared__ int si[8], last;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  float v = -3.402823e+38f;
+  int i = 0;
+  // four loads in flight: a vocabulary of 151936 is four rounds of this grid
+  for (int k = blockIdx.x * 256 + t; k < n; k += gridDim.x * 1024) {
+    float c[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int at = k + j * (int)gridDim.x * 256;
+      c[j] = at < n ? logits[at] : -INFINITY;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) pick_better(v, i, c[j], k + j * (int)gridDim.x * 256);
+  }
+  auto reduce = [&]() {  // the block's best is thread 0's
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) pick_better(v, i, __shfl_xor_sync(0xffffffffu, v, o), __shfl_xor_sync(0xffffffffu, i, o));
+    if (lane == 0) { sv[warp] = v; si[warp] = i; }
+    __syncthreads();
+    if (t == 0)
+      for (int w = 1; w < 8; w++) pick_better(v, i, sv[w], si[w]);
+  };
+  reduce();
+  if (t == 0) {
+    vals[blockIdx.x] = v;
+    idxs[blockIdx.x] = i;
+    __threadfence();
+    last = atomicAdd(arrived, 1) == (int)gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  v = -3.402823e+38f;
+  i = 0x7fffffff;
+  for (int k = t; k < (int)gridDim.x; k += 256) pick_better(v, i, __ldcg(vals + k), __ldcg(idxs + k));
+  reduce();
+  if (t == 0) {
+    const int s = *step;
+    *tok = i;
+    out_tokens[s] = i;
+    *pos += 1;
+    *kvlen += 1;
+    *step = s + 1;
+    *ticket += 1u;
+    *arrived = 0;
+  }
+}
+
 // combine the per-rank (best value, index) pairs of a vocabulary-sharded argmax;
 // ties go to the lower global index (sample.wgsl:45-53)
 __global__ void argmax_merge_kernel(const float *pairs, int ranks, int batch, int *tok) {
@@ -927,7 +987,9 @@ static dp_status run_layers(dp_model *m, int tokens, bool decode, int seq, int s
     } else {
       DP_TRY(dpk_attention_with_scratch(ctx, ap, (float *)m->attn_scratch->dptr, splits));
       bool fused_o = false;
-      if (p == 1) {  // h += o_proj(att) in the projection's epilogue
+      if (single)  // one split (short sequences): the projection builds its digits out of the attention's rows itself
+        DP_TRY(dpk_gemv_q4k_tma_fused(ctx, (const uint8_t *)L.o->dptr, SRC_PLAIN, m->att, nullptr, 0.0f, 0, 0, o_dst, H, m->qdim, o_res, &fused_o));
+      if (!fused_o && p == 1) {  // h += o_proj(att) in the projection's epilogue
         dpk_rows_fuse f;
         f.residual = m->h;
         DP_TRY(rows_linear_fused(m, (const uint8_t *)L.o->dptr, m->att, m->h, tokens, H, m->qdim, f, &fused_o));
@@ -1241,6 +1303,13 @@ static dp_status record_decode_step(dp_model *m, int batch) {
   dp_ctx *ctx = m->ctx;
   DP_TRY(embed_rows(m, m->d_tok, batch, true));
   DP_TRY(run_layers(m, batch, true, 0, 0));
+  if (batch == 1 && m->cfg.tp_size == 1) {
+    DP_TRY(run_logits(m, m->h, 1));
+    const int blocks = m->vocab_l < 148 * 256 ? (m->vocab_l + 255) / 256 : 148;
+    DP_LAUNCH(ctx, pick_advance_kernel, blocks, 256, 0, (const float *)m->logits, m->vocab_l, m->am_vals, m->am_idx, m->d_step + 1, m->d_pos, m->d_kvlen, m->d_tok, m->d_step,
+              (int *)m->out_tokens->dptr, m->d_ticket);
+    return DP_OK;
+  }
   DP_TRY(run_head(m, m->h, batch));
   DP_LAUNCH(ctx, advance_kernel, 1, 256, 0, m->d_pos, m->d_kvlen, m->d_tok, m->d_step, (int *)m->out_tokens->dptr, batch, m->d_ticket);
   return DP_OK;
