@@ -57,8 +57,6 @@ __device__ __forceinline__ uint32_t atc_pack(__half2 h) { return *reinterpret_ca
 template <int D, bool PLO>
 __global__ void __launch_bounds__(ATC_THREADS, 2) attn_tc_kernel(dpk_attn_params p, float *__restrict__ part, int splits,
                                                                  int head_tiles, int gt) {
-  pdl_launch();
-  pdl_wait();
   constexpr int CH = D / 8;        // 16-byte chunks per key row
   constexpr int ROWB = D * 2;      // bytes per key row
   constexpr int TILE = 16 * ROWB;  // one 16-key K (or V) tile
@@ -74,6 +72,11 @@ __global__ void __launch_bounds__(ATC_THREADS, 2) attn_tc_kernel(dpk_attn_params
   const int G = p.num_heads / p.num_kv_heads;
   const int h0 = kvh * G + ht * gt;
 
+  // Where the kernel appends the new key and value itself, what it reads of the cache, and lengths and positions, come from
+  // earlier steps (which ended before this one's first kernel began): the first tiles are asked for before the previous
+  // kernel, which brings the new token's projections, has ended.
+  const bool fused = p.fuse.qkv != nullptr;
+  if (!fused) pdl_wait();
   int kv_len = p.kv_lens ? min(max(p.kv_lens[b], 0), p.kv_len) : p.kv_len;  // the host checked the cache for p.kv_len keys
   const AttnRange range = attn_range(p, kv_len, qi);
   const int lo = range.lo, hi = range.hi;
@@ -83,14 +86,47 @@ __global__ void __launch_bounds__(ATC_THREADS, 2) attn_tc_kernel(dpk_attn_params
   int k_end = k_begin + per_split;
   if (k_end > hi) k_end = hi;
 
+  const int new_pos = fused ? p.fuse.pos[b] : -1;  // the key that is not in the cache yet
+  const size_t fuse_stride = p.fuse.row_stride ? p.fuse.row_stride : (size_t)(p.fuse.nh + 2 * p.fuse.nkv) * D;
+
+  const size_t row_stride = (size_t)p.num_kv_heads * D;
+  const __half *kbase = p.k + (size_t)b * p.kv_batch_stride + (size_t)kvh * D;
+  const __half *vbase = p.v + (size_t)b * p.kv_batch_stride + (size_t)kvh * D;
+
+  unsigned char *ring = atc_smem + (size_t)warp * ATC_STAGES * STAGE;
+  const uint32_t ring_u32 = atc_smem_u32(ring);
+  const int n_blocks = (k_end > k_begin) ? (k_end - k_begin + 15) / 16 : 0;
+  const int my_n = n_blocks > warp ? (n_blocks - warp + ATC_WARPS - 1) / ATC_WARPS : 0;
+
+  auto issue = [&](int i, int stage) {
+    const int key0 = k_begin + (warp + i * ATC_WARPS) * 16;
+    const uint32_t sK = ring_u32 + stage * STAGE;
+#pragma unroll
+    for (int c = 0; c < (16 * CH) / 32; c++) {
+      const int piece = c * 32 + lane;
+      const int key = piece / CH, ch = piece % CH;
+      const int kk = key0 + key;
+      const bool ok = kk < k_end && kk != new_pos;  // the new token's row is built in place below
+      const size_t off = (size_t)(ok ? kk : k_begin) * row_stride + ch * 8;
+      const uint32_t dst = sK + key * ROWB + ((ch ^ (key & 7)) << 4);
+      atc_cp_async16(dst, kbase + off, ok ? 16 : 0);          // rows past the range are zero filled
+      atc_cp_async16(dst + TILE, vbase + off, ok ? 16 : 0);
+    }
+  };
+
+#pragma unroll
+  for (int s = 0; s < ATC_STAGES - 1; s++) {
+    if (s < my_n) issue(s, s);
+    atc_commit();
+  }
+  if (fused) pdl_wait();
+  pdl_launch();
+
   const float LOG2E = 1.4426950408889634f;
   const bool capped = p.softcap > 0.0f;
   const float qmul = capped ? p.scale : p.scale * LOG2E;
 
   // A fragments of Q for every k-step: rows g (hi) and g+8 (lo).  This lane owns dims 16ks + 2t + {0,1,8,9}.
-  const bool fused = p.fuse.qkv != nullptr;
-  const int new_pos = fused ? p.fuse.pos[b] : -1;  // the key that is not in the cache yet
-  const size_t fuse_stride = p.fuse.row_stride ? p.fuse.row_stride : (size_t)(p.fuse.nh + 2 * p.fuse.nkv) * D;
   uint32_t qa[KS][4];
   {
     float x[KS][4];
@@ -155,37 +191,6 @@ __global__ void __launch_bounds__(ATC_THREADS, 2) attn_tc_kernel(dpk_attn_params
 #pragma unroll
   for (int j = 0; j < KS; j++) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.0f;
   float m_run = -INFINITY, l_run = 0.0f;  // head g; l is this lane's share (keys 2t, 2t+1 of every block)
-
-  const size_t row_stride = (size_t)p.num_kv_heads * D;
-  const __half *kbase = p.k + (size_t)b * p.kv_batch_stride + (size_t)kvh * D;
-  const __half *vbase = p.v + (size_t)b * p.kv_batch_stride + (size_t)kvh * D;
-
-  unsigned char *ring = atc_smem + (size_t)warp * ATC_STAGES * STAGE;
-  const uint32_t ring_u32 = atc_smem_u32(ring);
-  const int n_blocks = (k_end > k_begin) ? (k_end - k_begin + 15) / 16 : 0;
-  const int my_n = n_blocks > warp ? (n_blocks - warp + ATC_WARPS - 1) / ATC_WARPS : 0;
-
-  auto issue = [&](int i, int stage) {
-    const int key0 = k_begin + (warp + i * ATC_WARPS) * 16;
-    const uint32_t sK = ring_u32 + stage * STAGE;
-#pragma unroll
-    for (int c = 0; c < (16 * CH) / 32; c++) {
-      const int piece = c * 32 + lane;
-      const int key = piece / CH, ch = piece % CH;
-      const int kk = key0 + key;
-      const bool ok = kk < k_end && kk != new_pos;  // the new token's row is built in place below
-      const size_t off = (size_t)(ok ? kk : k_begin) * row_stride + ch * 8;
-      const uint32_t dst = sK + key * ROWB + ((ch ^ (key & 7)) << 4);
-      atc_cp_async16(dst, kbase + off, ok ? 16 : 0);          // rows past the range are zero filled
-      atc_cp_async16(dst + TILE, vbase + off, ok ? 16 : 0);
-    }
-  };
-
-#pragma unroll
-  for (int s = 0; s < ATC_STAGES - 1; s++) {
-    if (s < my_n) issue(s, s);
-    atc_commit();
-  }
 
   for (int i = 0; i < my_n; i++) {
     __syncwarp();  // every lane has finished reading the stage that is refilled next
