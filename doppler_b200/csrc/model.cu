@@ -1263,6 +1263,7 @@ extern "C" dp_status dp_model_prefill_many(dp_model *m, int n, const int32_t *se
   if (!m) return DP_ERR_INVALID;
   dp_ctx *ctx = m->ctx;
   DP_CHECK(ctx, n > 0 && seqs && tokens && lengths && next_tokens, "prefill: no prompts or a null pointer");
+  DP_CHECK(ctx, n <= m->cfg.max_batch, "prefill: %d prompts for %d sequences", n, m->cfg.max_batch);
   std::vector<const int32_t *> at(n);
   std::vector<char> used(m->cfg.max_batch, 0);
   for (int i = 0; i < n; i++) {

@@ -55,7 +55,7 @@ def test_same_as_one_by_one(dev, lengths):
 
 def test_nothing_runs_where_a_prompt_is_invalid(dev):
     m = DecoderModel(dev, CFG, max_seq=64, max_batch=3)
-    for prompts, seqs in (([[1], []], [0, 1]), ([[1], [CFG["vocab"]]], [0, 1]), ([[1], [2] * 65], [0, 1]), ([[1], [2]], [0, 0]), ([[1], [2]], [0, 3])):
+    for prompts, seqs in (([[1], []], [0, 1]), ([[1], [CFG["vocab"]]], [0, 1]), ([[1], [2] * 65], [0, 1]), ([[1], [2]], [0, 0]), ([[1], [2]], [0, 3]), ([[1]] * 4, [0, 1, 2, 0])):
         with pytest.raises(RuntimeError):
             m.prefill_many(prompts, seqs)
     assert [m.seq_len(s) for s in range(3)] == [0, 0, 0]
