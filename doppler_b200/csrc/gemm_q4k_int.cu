@@ -95,8 +95,8 @@ __device__ __forceinline__ int qi_exponent(float most) {
 __device__ __forceinline__ float qi_pow2(int e) { return __uint_as_float((uint32_t)(127 + e) << 23); }
 
 // arrive on a barrier of the pair's other CTA.  (With a release at cluster scope the arrive costs a thousand cycles, in the
-// drains' path to the next super-block.  Nothing that generic loads read is handed over: tensor memory is ordered by
-// tcgen05.wait and the tcgen05 fences.)
+// drains' path to the next super-block.  Nothing that generic loads read goes this way: tensor memory is ordered by
+// tcgen05.wait and the tcgen05 fences, and the row scales have barriers of their own inside each CTA.)
 __device__ __forceinline__ void qi_arrive_remote(uint32_t cluster_bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(QI_THREADS, 1) gemm_q4k_int_kernel(const __gri
                                                                      int *__restrict__ err) {
   extern __shared__ uint8_t qi_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(qi_raw) + 1023) & ~(uintptr_t)1023);
-  __shared__ __align__(8) uint64_t bar_words[4 * QI_RING + 2];
+  __shared__ __align__(8) uint64_t bar_words[5 * QI_RING + 2];
   __shared__ float row_scales[QI_SCALES][QI_ROWS];  // what a unit's product is multiplied by on read-back: d, or the sum unit's power of two
   __shared__ uint32_t tmem_word;
   __shared__ int abort_word;
@@ -152,7 +152,11 @@ __global__ void __launch_bounds__(QI_THREADS, 1) gemm_q4k_int_kernel(const __gri
   auto parity = [&](uint32_t g) { return (g / QI_RING) & 1u; };
   auto full_p = [&](uint32_t s) { return bars + 8u * (2 * QI_RING + s); };
   auto free_p = [&](uint32_t s) { return bars + 8u * (3 * QI_RING + s); };
-  auto empty = [&](uint32_t b) { return bars + 8u * (4 * QI_RING + b); };
+  // The row scales of unit n are written: builders to drains of the same CTA (by way of "full", the MMAs and "multiplied" they
+  // would leave the CTA and come back through arrives that order nothing there).  The ring is long enough: a builder reaches
+  // unit n + 4 only after unit n + 2 has been started, and that after every drain has handed back unit n.
+  auto scaled = [&](uint32_t n) { return bars + 8u * (4 * QI_RING + (n & (QI_RING - 1))); };
+  auto empty = [&](uint32_t b) { return bars + 8u * (5 * QI_RING + b); };
   // item -> tile and part: neighbouring clusters share the weight rows
   auto tile_n_of = [&](int item) { return item / (p.tiles_m * p.parts); };
   auto tile_m_of = [&](int item) { return item % p.tiles_m; };
@@ -169,6 +173,7 @@ __global__ void __launch_bounds__(QI_THREADS, 1) gemm_q4k_int_kernel(const __gri
       mbar_init(done(s), 1);
       mbar_init(full_p(s), 1);
       mbar_init(free_p(s), QI_BUILDERS);
+      mbar_init(scaled(s), QI_BUILDERS / 2);
     }
     for (uint32_t b = 0; b < 2; b++) mbar_init(empty(b), 2 * QI_DRAINERS);  // CTA 0's: the drains of both CTAs
     *abort_flag = 0;
@@ -353,7 +358,11 @@ __global__ void __launch_bounds__(QI_THREADS, 1) gemm_q4k_int_kernel(const __gri
           put(3 * nsb, zero);
         }
         written();
-        if (lane == 0) { mbar_arrive(full(g)); mbar_arrive(full(g + 1)); }
+        if (lane == 0) {
+          if (step == 0) mbar_arrive(scaled(g >> 1));
+          mbar_arrive(full(g));
+          mbar_arrive(full(g + 1));
+        }
         g += 2;
       }
       // ---- super-blocks ----
@@ -391,6 +400,7 @@ __global__ void __launch_bounds__(QI_THREADS, 1) gemm_q4k_int_kernel(const __gri
           qi_tmem_st16(at + 16u, v);
           written();
           if (lane == 0) {
+            if (h == 0 && step == 0) mbar_arrive(scaled(g >> 1));
             mbar_arrive(full(g));
             if (h == 1) mbar_arrive(free_p(rp.i));
           }
@@ -413,7 +423,7 @@ __global__ void __launch_bounds__(QI_THREADS, 1) gemm_q4k_int_kernel(const __gri
       for (int i = 0; i < QI_BN / 2; i++) acc[i] = 0.0f;
       for (int u = 0; u < units; u++, n++) {
         const uint32_t g = 2u * n + 1u, b = n & 1u;
-        const bool ready = mbar_wait_bounded(done(g), parity(g), abort_flag);
+        const bool ready = mbar_wait_bounded(scaled(n), parity(n), abort_flag) && mbar_wait_bounded(done(g), parity(g), abort_flag);
         if (!__all_sync(0xffffffffu, ready)) { ok = false; break; }  // tcgen05.ld is warp-wide: together or not at all
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const float scale = row_scales[n % QI_SCALES][quad * 32 + lane];
