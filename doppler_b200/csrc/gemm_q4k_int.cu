@@ -651,6 +651,9 @@ __global__ void __launch_bounds__(256) int_reduce_kernel(const float *__restrict
   }
 }
 
+// shared memory a plan's rings may take: what a launch may ask for, less alignment, barriers and row scales
+size_t qi_ring_budget(const dp_ctx *ctx) { return ctx->smem_optin - 1024 - 8192; }
+
 // Tile width and parts of K with the least estimated time, in cycles: an MMA of sixteen K takes half a cycle per activation
 // row, a super-block no less than what builders and drains need; an item has a fixed cost (fill, store); a K split is paid
 // for with the traffic of its parts.
@@ -658,7 +661,7 @@ IntPlan qi_plan(dp_ctx *ctx, int M, int N, int K, bool lo, bool may_split) {
   IntPlan best = {};
   double best_cost = -1.0;
   const int clusters = ctx->sm_count / 2, bpr = (K + QK_K - 1) / QK_K, tiles_n = (N + 255) / 256;
-  const size_t budget = ctx->smem_optin - 1024 - 8192;  // alignment; barriers and row scales
+  const size_t budget = qi_ring_budget(ctx);
   for (int parts = 1; parts <= (may_split ? 8 : 1); parts++) {
     if (bpr % parts || (parts > 1 && bpr / parts < 2)) continue;
     for (int bn = 32; bn <= QI_BN; bn += 32) {
@@ -690,7 +693,13 @@ template <bool LO, typename OutT>
 dp_status launch_int(dp_ctx *ctx, const CUtensorMap *tm, const uint8_t *W, OutT *C, int M, int N, const IntPlan &p, const IntOut &o) {
   const size_t smem = qi_rings(p, LO) + 1024;
   auto kernel = gemm_q4k_int_kernel<LO, OutT>;
-  DP_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // once, to the most any plan takes: set to each launch's own size, a small one lowered it under a large one that another
+  // thread was about to launch
+  static dp_per_device_once limit;
+  if (limit.pending(ctx->device)) {
+    DP_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(qi_ring_budget(ctx) + 1024)));
+    limit.done(ctx->device);
+  }
   const int clusters = ctx->sm_count / 2;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * (unsigned)(p.items < clusters ? p.items : clusters));

@@ -1,4 +1,6 @@
 """The integer-tile Q4_K GEMM at the edges of its tiles, sum units and rows, against 64-bit products of the same blocks."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -62,3 +64,31 @@ def test_edges(dev, m, n, k, act, out):
     fits = np.abs(want) < 65000.0 if out == "f16" else np.ones_like(want, bool)
     assert (np.abs(got - want)[fits] <= tol[fits]).all(), np.max((np.abs(got - want) / tol)[fits])
     assert np.array_equal(got, run(dev, b, n, k, a, out, alpha=0.5))  # nothing depends on timing
+
+
+def test_two_threads_with_plans_of_different_sizes():
+    """Two contexts of one process, a thread each: launches with large and small rings of the same kernel do not disturb each other."""
+    failed, start = [], threading.Barrier(2)
+
+    def work(m, n, k, seed):
+        d = ops.Device(0)
+        try:
+            rng = np.random.default_rng(seed)
+            t = d.tensor_from(rng.standard_normal((m, k)).astype(np.float32))
+            w = d.weight_from(blocks(rng, n, k // 256).ravel(), "q4k", [n, k])
+            out = d.acquire_buffer(m * n * 4, "out")
+            start.wait()
+            for _ in range(3000):
+                ops.run_matmul(t, w, m, n, k, output_buffer=out, output_dtype="f32")
+            d.sync()
+        except Exception as e:  # noqa: BLE001
+            failed.append(e)
+        finally:
+            d.close()
+
+    threads = [threading.Thread(target=work, args=a) for a in ((512, 2048, 1024, 1), (70, 2048, 512, 2))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
