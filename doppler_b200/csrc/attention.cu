@@ -182,8 +182,15 @@ __global__ void __launch_bounds__(ATT_THREADS, LPK == 16 ? 2 : 1) attn_split_ker
 }
 
 // Any query/key size and any value size up to 32 * MAXE, any GQA ratio, f16 or f32 caches: one CTA per (split, query
-// head, row), lanes over dims.  Used for shapes outside the fast kernels.  Bound: instructions per key; MAXE is the least
-// that holds the head sizes (a 700-token prompt in 32 bits, 16 heads of 128, with MAXE 16 for all sizes: 800 us).
+// head, row), lanes over dims.  Used for shapes outside the fast kernels.  Bound: instructions and loads in flight per key,
+// one key per warp at a time: a value that is not there costs its predicated load.  MAXE is chosen from 4, 5, 8, 16 and 32 by
+// the head's size; against 16 for all sizes up to 512 the kernel takes, in us (f16 unless it says f32):
+//   32 sequences of 2048 keys, 16 heads of 128 / 160 / 192 / 256: 586 -> 268, 695 -> 290, 768 -> 384, 1006 -> 430
+//   4 sequences of 8192 keys, 32 heads: 468 -> 410, 573 -> 451, 629 -> 605, 812 -> 676
+//   700-token portion, 16 heads, f32: 774 -> 414, 1045 -> 428, 1049 -> 686, 1059 -> 698
+// (5 because heads of 129 to 160 would be up to 6 % slower with 8 than with 16).  Two keys at a time pay up to 128 values
+// only, where the registers of both fit beside enough warps; beyond, the loop is left alone (256 values, 4 x 8192 keys, two at
+// a time: 1275 us; 512 values: 2962 against 1182).
 template <typename KT, int MAXE>
 __global__ void __launch_bounds__(128) attn_split_generic_kernel(dpk_attn_params p, float *__restrict__ part, int splits) {
   pdl_launch();
@@ -209,7 +216,7 @@ __global__ void __launch_bounds__(128) attn_split_generic_kernel(dpk_attn_params
   const size_t k_stride = (size_t)p.num_kv_heads * D, v_stride = p.v_row_stride ? (size_t)p.v_row_stride : (size_t)p.num_kv_heads * V;
   const KT *kb = reinterpret_cast<const KT *>(p.k) + (size_t)b * p.kv_batch_stride + (size_t)kvh * D;
   const KT *vb = reinterpret_cast<const KT *>(p.v) + (size_t)b * (p.v_batch_stride ? p.v_batch_stride : p.kv_batch_stride) + (size_t)kvh * V;
-#pragma unroll 2
+#pragma unroll(MAXE <= 4 ? 2 : 1)
   for (int key = k_begin + warp; key < k_end; key += 4) {
     float a = 0.0f;
 #pragma unroll
@@ -421,6 +428,7 @@ static dp_status attention_impl(dp_ctx *ctx, const dpk_attn_params &p, float *sc
   if (p.kv_f32) DP_LAUNCH(ctx, (attn_split_generic_kernel<float, E>), grid, 128, 0, p, scratch, splits);              \
   else DP_LAUNCH(ctx, (attn_split_generic_kernel<__half, E>), grid, 128, 0, p, scratch, splits)
     if (most <= 128) { DP_GENERIC(4); }
+    else if (most <= 160) { DP_GENERIC(5); }
     else if (most <= 256) { DP_GENERIC(8); }
     else if (most <= 512) { DP_GENERIC(16); }
     else { DP_GENERIC(32); }

@@ -189,6 +189,23 @@ def test_prefill_query_tiled(dev, H, Hkv, T, start):
             assert_close(got[r], np.asarray(exp).ravel(), f"query-tiled prefill row {r} of {T}")
 
 
+@pytest.mark.parametrize("G", [1, 2, 4, 8])
+@pytest.mark.parametrize("D", [96, 129, 132, 160, 161, 256, 257, 512])
+def test_heads_of_every_size(dev, D, G):
+    """Sizes at the edges of the generic kernel's instantiations: decode (one sequence, split; several) and a causal portion."""
+    Hkv = 2
+    H = Hkv * G
+    for B, T, kv in ((1, 1, 704), (3, 1, 72), (1, 37, 88)):
+        s = synthetic.key(59, D * 100 + G * 10 + T)
+        q = synthetic.normal_f32(s, B * T * H * D)
+        k16, v16 = (synthetic.normal_f16(s + i, B * kv * Hkv * D) for i in (1, 2))
+        got = _attn(dev, q, k16, v16, H, D, seq_len=T, kv_len=kv, num_kv_heads=Hkv, causal=T > 1, start_pos=kv - T, batch=B,
+                    kv_batch_stride=kv * Hkv * D).reshape(B, -1)
+        for b, (qb, kb, vb) in enumerate(zip(*(x.reshape(B, -1) for x in (q, k16, v16)))):
+            exp = O.attention_f16kv(qb, kb, vb, T, kv, H, Hkv, D, causal=True, start_pos=kv - T)
+            assert_close(got[b], exp, f"D{D} G{G} B{B} T{T} sequence {b}")
+
+
 def test_attention_argument_errors(dev):
     q = dev.tensor_from(np.zeros(8 * 128, np.float32))
     kv = dev.tensor_from(np.zeros(16 * 2 * 128, np.float16))
