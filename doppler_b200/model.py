@@ -41,9 +41,11 @@ class Runner:
 
     def prefill_many(self, prompts, seqs) -> list:
         """The greedy tokens after several prompts, one per sequence of ``seqs``; short ones share passes over the layers."""
-        parts = [np.asarray(p, np.int32) for p in prompts]
+        parts = [np.asarray(p, np.int32).ravel() for p in prompts]
         t = np.ascontiguousarray(np.concatenate(parts)) if parts else np.empty(0, np.int32)
-        n, s, out = np.array([p.size for p in parts], np.int32), np.ascontiguousarray(seqs, np.int32), np.empty(len(parts), np.int32)
+        n, s, out = np.array([p.size for p in parts], np.int32), np.ascontiguousarray(seqs, np.int32).ravel(), np.empty(len(parts), np.int32)
+        if s.size != len(parts):
+            raise ValueError(f"{len(parts)} prompts for {s.size} sequences")
         self.device.check(self.device.lib.dp_model_prefill_many(self.h, len(parts), s.ctypes.data_as(C.c_void_p), t.ctypes.data_as(C.c_void_p),
                                                                 n.ctypes.data_as(C.c_void_p), out.ctypes.data_as(C.c_void_p)))
         return out.tolist()

@@ -58,5 +58,8 @@ def test_nothing_runs_where_a_prompt_is_invalid(dev):
     for prompts, seqs in (([[1], []], [0, 1]), ([[1], [CFG["vocab"]]], [0, 1]), ([[1], [2] * 65], [0, 1]), ([[1], [2]], [0, 0]), ([[1], [2]], [0, 3]), ([[1]] * 4, [0, 1, 2, 0])):
         with pytest.raises(RuntimeError):
             m.prefill_many(prompts, seqs)
+    for prompts, seqs in (([[1], [2], [3]], [0, 1]), ([[1]], [0, 1]), ([[1]], [])):
+        with pytest.raises(ValueError):
+            m.prefill_many(prompts, seqs)
     assert [m.seq_len(s) for s in range(3)] == [0, 0, 0]
     m.destroy()
