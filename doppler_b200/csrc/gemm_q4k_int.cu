@@ -17,6 +17,17 @@
 // of two per weight row, the sums by one per activation row, both undone on read-back).  hi + lo holds all 17 bits of
 // dmin * m; 22 bits of the sums.
 //
+// The tensor core cuts off what falls below its accumulator's last bit, so that products added while the accumulator is
+// small cost no accuracy.  f32 rows have two orders of their products: lo and hi in turn for every K slice, or (lo_first) the lo
+// products of the whole super-block before its hi products, which waits for both of its groups first.  Error against 64 bits,
+// random normal rows, K 1024 to 12288: 9.3e-7 in turn, 4.6e-7 to 5.1e-7 lo first (f32 FMAs: 5.7e-7 at K = 1024, 1.9e-6 at
+// 11111; gemm_q4k_tc_rows.cu: 5.2e-7 to 5.4e-7; dequantised tiles: 3.7e-6 to 2.2e-5).  us in turn -> lo first: 128 x 6144 x 4096
+// 44.1 -> 45.7, 256 x 24576 x 4096 137 -> 144, 512 x 6144 x 4096 (192-wide tiles, a ring of two weight groups) 69 -> 79.  Lo
+// first therefore where calls would otherwise lose accuracy: shapes no tile divides, which f32 FMAs multiplied, and rows of
+// several prompts, which one by one go through gemm_q4k_tc_rows.cu.  The small products of a sum unit come first from seven
+// super-blocks on (K = 12288: 6.3e-7 -> 5.3e-7); up to six, what is cut off there and in the super-blocks cancels in part
+// (four: 4.6e-7, with the small ones first 5.1e-7), and so it does at any number where lo and hi take turns (9.2e-7, 1.08e-6).
+//
 // A cluster of two CTAs owns 256 weight rows x bn activation rows (cta_group::2, M = 256: CTA r holds 128 weight rows and
 // their 128 lanes of the result, and half of the activation tile).  Sharing the activation tile halves its L2 and
 // shared-memory traffic.  The weight tiles are the A operand in TENSOR MEMORY: out of shared memory every MMA would read
@@ -46,6 +57,7 @@ using namespace umma;
 constexpr int QI_ROWS = 128;       // weight rows per CTA
 constexpr int QI_BN = 192;         // most activation rows of a tile
 constexpr int QI_SUMS = 10;        // super-blocks of a sum unit: 3 * 8 * 10 = 240 of its 256 columns
+constexpr int QI_SUMS_LO_FIRST = 8, QI_SUMS_LONG = 6;  // ... lo first; and where a part is longer than 24 (more f32 additions)
 constexpr int QI_BUILDERS = 8, QI_DRAINERS = 8;
 constexpr int QI_THREADS = (4 + QI_BUILDERS + QI_DRAINERS) * 32;
 constexpr int QI_RING = 4;         // most stages of a ring; also the rings of barriers that go by group
@@ -58,6 +70,12 @@ struct IntPlan {
 };
 
 __host__ __device__ __forceinline__ int qi_sum_begin(const IntPlan &p, int u) { return u * p.pb / p.npu; }
+// places (eighths of columns) of the products of a sum unit of nsb super-blocks: [hi hi], [lo hi], [hi lo] of weights and sums
+struct QiSumOrder {
+  int hh, lh, hl;
+};
+constexpr QiSumOrder qi_sums_in_turn(int nsb) { return QiSumOrder{0, nsb, 2 * nsb}; }
+constexpr QiSumOrder qi_sums_lo_first(int nsb) { return nsb < 7 ? qi_sums_in_turn(nsb) : QiSumOrder{2 * nsb, 0, nsb}; }
 
 constexpr uint32_t QI_P_STAGE = QI_ROWS * Q4K_BLOCK_BYTES;  // packed super-blocks of the CTA's weight rows
 constexpr uint32_t QI_W_COLS = 64;                          // tensor-memory columns of a weight group: 128 K, two f16 each
@@ -125,11 +143,13 @@ struct IntOut {
   int silu;                // f32 output: weight rows are gate|up pairs (groups of sixteen); store silu(gate) * up, N / 2 columns
 };
 
-template <bool LO, typename OutT>
+// F32: f16 activations (0), f32 activations with lo and hi products in turn (1) or the lo products first (2)
+template <int F32, typename OutT>
 __global__ void __launch_bounds__(QI_THREADS, 1) gemm_q4k_int_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_lo,
                                                                      const __grid_constant__ CUtensorMap tmap_s, const __grid_constant__ CUtensorMap tmap_w,
                                                                      const uint8_t *__restrict__ W, OutT *C, int M, int N, IntPlan p, IntOut o,
                                                                      int *__restrict__ err) {
+  constexpr bool LO = F32 > 0;
   extern __shared__ uint8_t qi_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(qi_raw) + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) uint64_t bar_words[5 * QI_RING + 2];
@@ -190,9 +210,9 @@ __global__ void __launch_bounds__(QI_THREADS, 1) gemm_q4k_int_kernel(const __gri
   // columns: two accumulators, then the weight groups
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(&tmem_word), tmem_w = tmem + 2u * (uint32_t)p.bn;
 
-  // 4 warps x 40 + 8 x 72 + 8 x 144 registers, of what the launch holds (20 warps x 96)
+  // 4 warps x 40 (lo first: 48) + 8 x 72 + 8 x 144 registers, of what the launch holds (20 warps x 96)
   if (warp < 4) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(F32 == 2 ? 48 : 40));
     if (warp == 0 && lane == 0) {
       // ---------------- activation tiles: this CTA's half of the rows ----------------
       uint32_t g = 0;
@@ -261,6 +281,29 @@ __global__ void __launch_bounds__(QI_THREADS, 1) gemm_q4k_int_kernel(const __gri
         const bool sums = u < p.npu;
         // K slices of sixteen: a sum unit's columns are three for every sub-block
         const int slices = sums ? (3 * (qi_sum_begin(p, u + 1) - qi_sum_begin(p, u)) + 1) / 2 : 16;
+        if (F32 == 2 && !sums) {
+          uint32_t w0[2];
+          uint64_t x0[2];
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            const uint32_t g = 2u * (uint32_t)n + (uint32_t)h;
+            if (!mbar_wait_bounded(full(g), parity(g), abort_flag)) { ok = false; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            w0[h] = tmem_w + rw.i * QI_W_COLS;
+            x0[h] = umma_desc_sw128(smem_u32(smem) + rx.i * x_stage);
+#pragma unroll
+            for (int k = 0; k < 8; k++) qi_umma(acc, w0[h] + 8u * k, x0[h] + to_lo + (k >> 2) * to_step + 2 * (k & 3), idesc, h == 0 && k == 0 ? 0u : 1u);
+            rx.next(p.sa);
+            rw.next(p.sb);
+          }
+          if (!ok) break;
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+#pragma unroll
+            for (int k = 0; k < 8; k++) qi_umma(acc, w0[h] + 8u * k, x0[h] + (k >> 2) * to_step + 2 * (k & 3), idesc, 1u);
+            umma_commit_2sm(done(2u * (uint32_t)n + (uint32_t)h));
+          }
+        } else {
 #pragma unroll
         for (int h = 0; h < 2; h++) {
           const uint32_t g = 2u * (uint32_t)n + (uint32_t)h;
@@ -281,6 +324,7 @@ __global__ void __launch_bounds__(QI_THREADS, 1) gemm_q4k_int_kernel(const __gri
           umma_commit_2sm(done(g));
           rx.next(p.sa);
           rw.next(p.sb);
+        }
         }
         for (int i = 0; i < 2; i++) { rx.next(p.sa); rw.next(p.sb); }  // the other lane's unit
         u += 2;
@@ -332,6 +376,7 @@ __global__ void __launch_bounds__(QI_THREADS, 1) gemm_q4k_int_kernel(const __gri
         const uint32_t s1 = rw.i;
         rw.next(p.sb);
         if (step == 0) row_scales[(g >> 1) % QI_SCALES][row] = -64.0f * qi_pow2(qi_exponent(most) - 8);  // (the sums are stored divided by 64)
+        const QiSumOrder at = F32 == 2 ? qi_sums_lo_first(nsb) : qi_sums_in_turn(nsb);
         // eight values of a super-block, four columns: place c of the unit's 32
         auto put = [&](int c, const uint32_t (&v)[4]) { qi_tmem_st4(lanes + (c < 16 ? s0 : s1) * QI_W_COLS + (uint32_t)(c & 15) * 4u, v); };
 #pragma unroll
@@ -348,9 +393,9 @@ __global__ void __launch_bounds__(QI_THREADS, 1) gemm_q4k_int_kernel(const __gri
               hi[j] = qi_hmul2(dm, m);
               lo[j] = qi_hfma2(dm, m, hi[j] ^ 0x80008000u);  // exactly what the rounding dropped
             }
-            put(k, hi);
-            put(nsb + k, lo);
-            put(2 * nsb + k, hi);
+            put(at.hh + k, hi);
+            put(at.lh + k, lo);
+            put(at.hl + k, hi);
           }
         }
         if ((nsb & 1) && step == 0) {  // the other half of the last K slice
@@ -508,15 +553,17 @@ __global__ void __launch_bounds__(QI_THREADS, 1) gemm_q4k_int_kernel(const __gri
 }
 
 // ---- activation rows: f16 halves, scales and sub-block sums ----
-// Where a sub-block's sum goes: its unit's columns [hi | hi | lo], eight per super-block
+// Where a sub-block's sum goes: its unit's three places, eight columns per super-block
+template <bool LO_FIRST>
 __device__ __forceinline__ void qi_put_sum(__half *sums_row, const IntPlan &p, int s, float v) {
   const int sb = s >> 3, part = sb / p.pb, k = sb - part * p.pb;
   const int u = ((k + 1) * p.npu - 1) / p.pb, b0 = qi_sum_begin(p, u), nsb = qi_sum_begin(p, u + 1) - b0;
+  const QiSumOrder to = LO_FIRST ? qi_sums_lo_first(nsb) : qi_sums_in_turn(nsb);
   __half *at = sums_row + (size_t)(part * p.npu + u) * 256 + (s & 7);
   const __half hi = __float2half_rn(v), lo = __float2half_rn(v - __half2float(hi));
-  at[(k - b0) * 8] = hi;
-  at[(nsb + k - b0) * 8] = hi;
-  at[(2 * nsb + k - b0) * 8] = lo;
+  at[(to.hh + k - b0) * 8] = hi;
+  at[(to.lh + k - b0) * 8] = hi;
+  at[(to.hl + k - b0) * 8] = lo;
   if ((nsb & 1) && k == b0) at[3 * nsb * 8] = __float2half_rn(0.0f);  // pairs with the weights' zero place
 }
 
@@ -540,7 +587,7 @@ __device__ __forceinline__ float qi_block_max(float v, float *sh) {  // eight wa
 // One block per row, any K and alignment.  f32 rows: scaled by a power of two and split, x * 2^-e = hi + lo (rows of kp
 // halves, zeros beyond K), row_scale = 2^e.  f16 rows: left as they are (copied to hi where hi is given), the sums alone
 // are scaled, sum_scale = 2^e.  The sums are divided by 64 on top.
-template <typename AT>
+template <typename AT, bool LO_FIRST>
 __global__ void __launch_bounds__(256) int_rows_kernel(const AT *__restrict__ in, __half *__restrict__ hi, __half *__restrict__ lo, float *__restrict__ scale,
                                                        __half *__restrict__ sums, int K, int kp, const IntPlan p) {
   pdl_launch();
@@ -550,7 +597,8 @@ __global__ void __launch_bounds__(256) int_rows_kernel(const AT *__restrict__ in
   const AT *x = in + (size_t)row * K;
   float mx = 0.0f;
   for (int i = threadIdx.x; i < K; i += 256) mx = fmaxf(mx, fabsf((float)x[i]));
-  const int e = qi_row_exponent(qi_block_max(mx, sh));
+  mx = qi_block_max(mx, sh);
+  const int e = qi_row_exponent(mx);
   const float down = qi_pow2(-e);
   if (threadIdx.x == 0) scale[row] = qi_pow2(e);
   for (int s = warp; s < p.bpr * 8; s += 8) {
@@ -568,14 +616,14 @@ __global__ void __launch_bounds__(256) int_rows_kernel(const AT *__restrict__ in
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) t += __shfl_xor_sync(0xffffffffu, t, d);
-    if (lane == 0) qi_put_sum(sums + (size_t)row * ((size_t)p.parts * p.npu * 256), p, s, t * 0.015625f);
+    if (lane == 0) qi_put_sum<LO_FIRST>(sums + (size_t)row * ((size_t)p.parts * p.npu * 256), p, s, t * 0.015625f);
   }
 }
 
 // The same for f32 rows with the row in registers (K % 32 == 0, K <= 1024 * NV, 16-byte aligned): one pass, 16-byte loads.
 // With norm_w the row is RMS-normalised first (rmsnorm.wgsl:119-187), element for element and reduction step for
 // reduction step as rmsnorm_vec_kernel (small_ops.cu) does it for rows of 1024..4096 values.
-template <int NV>
+template <int NV, bool LO_FIRST>
 __global__ void __launch_bounds__(256) int_rows_vec_kernel(const float *__restrict__ in, __half *__restrict__ hi, __half *__restrict__ lo, float *__restrict__ scale,
                                                            __half *__restrict__ sums, int K, const IntPlan p, const float *__restrict__ norm_w, float eps) {
   pdl_launch();
@@ -613,7 +661,8 @@ __global__ void __launch_bounds__(256) int_rows_vec_kernel(const float *__restri
   float mx = 0.0f;
 #pragma unroll
   for (int i = 0; i < NV; i++) mx = fmaxf(fmaxf(mx, fmaxf(fabsf(v[i].x), fabsf(v[i].y))), fmaxf(fabsf(v[i].z), fabsf(v[i].w)));
-  const int e = qi_row_exponent(qi_block_max(mx, sh));
+  mx = qi_block_max(mx, sh);
+  const int e = qi_row_exponent(mx);
   const float down = qi_pow2(-e);
   if (threadIdx.x == 0) scale[row] = qi_pow2(e);
   __half *sums_row = sums + (size_t)row * ((size_t)p.parts * p.npu * 256);
@@ -631,10 +680,10 @@ __global__ void __launch_bounds__(256) int_rows_vec_kernel(const float *__restri
     const __half2 l01 = __floats2half2_rn(s0 - f01.x, s1 - f01.y), l23 = __floats2half2_rn(s2 - f23.x, s3 - f23.y);
     *reinterpret_cast<uint2 *>(hi + base + 4 * idx) = make_uint2(*reinterpret_cast<const uint32_t *>(&h01), *reinterpret_cast<const uint32_t *>(&h23));
     *reinterpret_cast<uint2 *>(lo + base + 4 * idx) = make_uint2(*reinterpret_cast<const uint32_t *>(&l01), *reinterpret_cast<const uint32_t *>(&l23));
-    if ((threadIdx.x & 7) == 0) qi_put_sum(sums_row, p, idx >> 3, t * 0.015625f);
+    if ((threadIdx.x & 7) == 0) qi_put_sum<LO_FIRST>(sums_row, p, idx >> 3, t * 0.015625f);
   }
   // (sub-blocks beyond a K that is no multiple of 256)
-  for (int s = (K >> 5) + (int)threadIdx.x; s < p.bpr * 8; s += 256) qi_put_sum(sums_row, p, s, 0.0f);
+  for (int s = (K >> 5) + (int)threadIdx.x; s < p.bpr * 8; s += 256) qi_put_sum<LO_FIRST>(sums_row, p, s, 0.0f);
 }
 
 // C = sum of the parts of a K-split launch, in a fixed order (+ residual, which may be C itself)
@@ -657,7 +706,7 @@ size_t qi_ring_budget(const dp_ctx *ctx) { return ctx->smem_optin - 1024 - 8192;
 // Tile width and parts of K with the least estimated time, in cycles: an MMA of sixteen K takes half a cycle per activation
 // row, a super-block no less than what builders and drains need; an item has a fixed cost (fill, store); a K split is paid
 // for with the traffic of its parts.
-IntPlan qi_plan(dp_ctx *ctx, int M, int N, int K, bool lo, bool may_split) {
+IntPlan qi_plan(dp_ctx *ctx, int M, int N, int K, bool lo, bool lo_first, bool may_split) {
   IntPlan best = {};
   double best_cost = -1.0;
   const int clusters = ctx->sm_count / 2, bpr = (K + QK_K - 1) / QK_K, tiles_n = (N + 255) / 256;
@@ -666,7 +715,8 @@ IntPlan qi_plan(dp_ctx *ctx, int M, int N, int K, bool lo, bool may_split) {
     if (bpr % parts || (parts > 1 && bpr / parts < 2)) continue;
     for (int bn = 32; bn <= QI_BN; bn += 32) {
       IntPlan p;
-      p.bpr = bpr; p.parts = parts; p.pb = bpr / parts; p.npu = (p.pb + QI_SUMS - 1) / QI_SUMS;
+      p.bpr = bpr; p.parts = parts; p.pb = bpr / parts;       const int most = !lo_first ? QI_SUMS : p.pb > 24 ? QI_SUMS_LONG : QI_SUMS_LO_FIRST;
+      p.npu = (p.pb + most - 1) / most;
       p.bn = bn; p.tiles_n = tiles_n; p.tiles_m = (M + bn - 1) / bn;
       p.items = p.tiles_n * p.tiles_m * parts;
       // tensor memory beside the accumulators; shared memory: activation groups first, then packed blocks
@@ -689,10 +739,10 @@ IntPlan qi_plan(dp_ctx *ctx, int M, int N, int K, bool lo, bool may_split) {
   return best;
 }
 
-template <bool LO, typename OutT>
+template <int F32, typename OutT>
 dp_status launch_int(dp_ctx *ctx, const CUtensorMap *tm, const uint8_t *W, OutT *C, int M, int N, const IntPlan &p, const IntOut &o) {
-  const size_t smem = qi_rings(p, LO) + 1024;
-  auto kernel = gemm_q4k_int_kernel<LO, OutT>;
+  const size_t smem = qi_rings(p, F32 > 0) + 1024;
+  auto kernel = gemm_q4k_int_kernel<F32, OutT>;
   // once, to the most any plan takes: set to each launch's own size, a small one lowered it under a large one that another
   // thread was about to launch
   static dp_per_device_once limit;
@@ -735,27 +785,32 @@ dp_status dpk_gemm_q4k_int(dp_ctx *ctx, const uint8_t *W, const void *A, dp_dtyp
   const bool vec = f32a && K % 32 == 0 && K <= 16384 && ((uintptr_t)A & 15) == 0;
   if (norm_w && !(vec && K >= 1024 && K <= 4096 && ((uintptr_t)norm_w & 15) == 0)) return DP_OK;
   const bool silu = fuse && fuse->silu_dst && c_dtype == DP_F32 && N % 16 == 0;
-  const IntPlan p = qi_plan(ctx, M, N, K, f32a, !silu);
+  const bool lo_first = f32a && (K % QK_K != 0 || N % 128 != 0 || (fuse && fuse->exact_weights));
+  const IntPlan p = qi_plan(ctx, M, N, K, f32a, lo_first, !silu);
 
   const int kp = (K + 7) / 8 * 8;
   const bool copy = f32a || K % 8 || ((uintptr_t)A & 15);  // f16 rows that TMA can read stay where they are
   const size_t a_bytes = copy ? ((size_t)M * kp * 2 + 255) / 256 * 256 : 0;
   const size_t sum_cols = (size_t)p.parts * p.npu * 256, s_bytes = ((size_t)M * sum_cols * 2 + 255) / 256 * 256;
-  DP_TRY(dp_scratch(ctx, &ctx->gemm_scratch, a_bytes * (f32a ? 2 : 1) + s_bytes + (size_t)M * 4, "matmul_a_f16"));
+  dp_status st = dp_scratch(ctx, &ctx->gemm_scratch, a_bytes * (f32a ? 2 : 1) + s_bytes + (size_t)M * 4, "matmul_a_f16");
+  if (st == DP_OK && p.parts > 1) st = dp_scratch(ctx, &ctx->gemm_split_scratch, (size_t)p.parts * M * N * 4, "matmul_k_split_parts");
+  DP_TRY(st);
   char *base = (char *)ctx->gemm_scratch->dptr;
   __half *hi = (__half *)base, *lo = (__half *)(base + a_bytes), *sums = (__half *)(base + a_bytes * (f32a ? 2 : 1));
   float *scale = (float *)((char *)sums + s_bytes);
   const float eps = fuse ? fuse->eps : 0.0f;
   if (vec) {
     const float *a = (const float *)A;
-    if (K <= 1024) DP_LAUNCH(ctx, int_rows_vec_kernel<1>, (unsigned)M, 256, 0, a, hi, lo, scale, sums, K, p, norm_w, eps);
-    else if (K <= 4096) DP_LAUNCH(ctx, int_rows_vec_kernel<4>, (unsigned)M, 256, 0, a, hi, lo, scale, sums, K, p, norm_w, eps);
-    else if (K <= 12288) DP_LAUNCH(ctx, int_rows_vec_kernel<12>, (unsigned)M, 256, 0, a, hi, lo, scale, sums, K, p, norm_w, eps);
-    else DP_LAUNCH(ctx, int_rows_vec_kernel<16>, (unsigned)M, 256, 0, a, hi, lo, scale, sums, K, p, norm_w, eps);
+    auto rows = K <= 1024    ? (lo_first ? int_rows_vec_kernel<1, true> : int_rows_vec_kernel<1, false>)
+                : K <= 4096  ? (lo_first ? int_rows_vec_kernel<4, true> : int_rows_vec_kernel<4, false>)
+                : K <= 12288 ? (lo_first ? int_rows_vec_kernel<12, true> : int_rows_vec_kernel<12, false>)
+                             : (lo_first ? int_rows_vec_kernel<16, true> : int_rows_vec_kernel<16, false>);
+    DP_LAUNCH(ctx, rows, (unsigned)M, 256, 0, a, hi, lo, scale, sums, K, p, norm_w, eps);
   } else if (f32a) {
-    DP_LAUNCH(ctx, int_rows_kernel<float>, (unsigned)M, 256, 0, (const float *)A, hi, lo, scale, sums, K, kp, p);
+    auto rows = lo_first ? int_rows_kernel<float, true> : int_rows_kernel<float, false>;
+    DP_LAUNCH(ctx, rows, (unsigned)M, 256, 0, (const float *)A, hi, lo, scale, sums, K, kp, p);
   } else {
-    DP_LAUNCH(ctx, int_rows_kernel<__half>, (unsigned)M, 256, 0, (const __half *)A, copy ? hi : (__half *)nullptr, (__half *)nullptr, scale, sums, K, kp, p);
+    DP_LAUNCH(ctx, (int_rows_kernel<__half, false>), (unsigned)M, 256, 0, (const __half *)A, copy ? hi : (__half *)nullptr, (__half *)nullptr, scale, sums, K, kp, p);
     if (!copy) hi = (__half *)A;
   }
 
@@ -787,15 +842,14 @@ dp_status dpk_gemm_q4k_int(dp_ctx *ctx, const uint8_t *W, const void *A, dp_dtyp
   }
   if (silu) fuse->silu_done = true;
   if (p.parts > 1) {
-    DP_TRY(dp_scratch(ctx, &ctx->gemm_split_scratch, (size_t)p.parts * M * N * 4, "matmul_k_split_parts"));
     dst = ctx->gemm_split_scratch->dptr;
   } else {
     o.residual = residual;
   }
-  dp_status st;
-  if (f32a) st = launch_int<true, float>(ctx, tm, W, (float *)dst, M, N, p, o);
-  else if (c_dtype == DP_F32 || p.parts > 1) st = launch_int<false, float>(ctx, tm, W, (float *)dst, M, N, p, o);
-  else st = launch_int<false, __half>(ctx, tm, W, (__half *)dst, M, N, p, o);
+  if (f32a && lo_first) st = launch_int<2, float>(ctx, tm, W, (float *)dst, M, N, p, o);
+  else if (f32a) st = launch_int<1, float>(ctx, tm, W, (float *)dst, M, N, p, o);
+  else if (c_dtype == DP_F32 || p.parts > 1) st = launch_int<0, float>(ctx, tm, W, (float *)dst, M, N, p, o);
+  else st = launch_int<0, __half>(ctx, tm, W, (__half *)dst, M, N, p, o);
   DP_TRY(st);
   if (p.parts > 1) {
     const size_t n = (size_t)M * N;

@@ -972,14 +972,20 @@ static dp_status gemm_q4k_tc_impl(dp_ctx *ctx, const uint8_t *W, const void *A, 
   //   f32 rows, M x N x K   65 x 24576 x 4096 87 -> 74, 512 x 6144 x 4096 84 -> 69, 1024 x 4096 x 4096 99 -> 93, 2048 x 1024 x 3072 66 -> 53, but
   //                         512 x 24576 x 4096 207 -> 221, 1024 x 6144 x 4096 111 -> 120, 512 x 4096 x 12288 122 -> 131, 2048 x 4096 x 4096 143 -> 152
   //   f16 rows              128 x 12288 x 4096 79 -> 43, 256 x 4096 x 4096 74 -> 43, 512 x 4096 x 4096 73 -> 53, but 512 x 12288 x 4096 75 -> 88
-  // so it takes what fills less than half a wave of the others' 512 x 256 pair tiles and has K up to 8192; very small weights
+  // so it takes what fills less than half a wave of the others' 512 x 256 pair tiles and has K up to 8192, and up to 256 rows at
+  // any N and K: there 40 to 390 % of its speed is gained with most shapes of f16 rows and up to 50 % with most of f32 rows (16 %
+  // lost at worst: 128 x 6144 x 4096 f32 37 -> 44, 100 x 24576 x 4096 f32 87 -> 102; f16 with K of 1024 and less 12 -> 15, 18 -> 21,
+  // 256 x 24576 x 4096 f16 93 -> 103), and everywhere the accuracy (3.7e-6 to 2.2e-5 -> 9e-7 for f32 rows, 4e-7 for f16 rows) and
+  // the range: a weight beyond f16's is an infinity in the others' tiles.  Very small weights
   // stay with the one launch that needs no pass over the rows (33 x 256 x 256: 9 against 17 us).  Shapes the others do not
-  // tile ran on CUDA cores (1000 x 1000 x 1000: 103 -> 26 us); they still do where that is over within about 15 us.
+  // tile ran on CUDA cores (1000 x 1000 x 1000: f32 rows 105 -> 30, f16 rows 102 -> 27 us); they still do where that is over within about 15 us, where the result
+  // is f32 and K below 640 (error of the f32 FMAs 4.1e-7 at K = 512, of the integer tiles 4.8e-7; 5.7e-7 and 4.6e-7 at 1024).
   // fuse->exact_weights (rows of several prompts, which were multiplied with exact weights one by one): always.
   if (exact && (c_dtype == DP_F32 || c_dtype == DP_F16)) {
     const long pair_tiles = (long)((M + 511) / 512) * ((N + 255) / 256);
     const bool few = M <= 256 || (pair_tiles * 2 <= ctx->sm_count / 2 && K <= 8192);
-    const bool take = tiled ? (few && (long)N * K >= (1l << 19)) || (fuse && fuse->exact_weights) : (double)M * N * K >= (double)(1l << 27);
+    const bool whole = (double)M * N * K >= (double)(1l << 27) && (K >= 640 || c_dtype == DP_F16);
+    const bool take = tiled ? (few && (long)N * K >= (1l << 19)) || (fuse && fuse->exact_weights) : whole;
     if (take) {
       DP_TRY(dpk_gemm_q4k_int(ctx, W, A, a_dtype, C, c_dtype, M, N, K, alpha, handled, fuse));
       if (*handled) return DP_OK;

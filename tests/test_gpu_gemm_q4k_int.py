@@ -66,6 +66,20 @@ def test_edges(dev, m, n, k, act, out):
     assert np.array_equal(got, run(dev, b, n, k, a, out, alpha=0.5))  # nothing depends on timing
 
 
+@pytest.mark.parametrize("m,n,k", [(1024, 600, 256), (300, 2049, 512), (1024, 600, 640), (300, 2049, 1024), (130, 4095, 2560), (70, 1023, 3100), (768, 513, 12288)])
+def test_untiled_f32_rows_keep_the_accuracy_of_f32_sums(dev, m, n, k):
+    """Shapes no tile divides: no further from 64 bits than f32 FMAs in order of K, the general path, are (mean over the outputs)."""
+    rng = np.random.default_rng(k)
+    b = blocks(rng, n, -(-k // 256))
+    d = (0.75 + 0.5 * rng.random(b.shape[:2])) / (190.0 * np.sqrt(k))
+    b[:, :, :4] = np.stack([d, 7.5 * d], -1).astype(np.float16).view(np.uint8).reshape(*b.shape[:2], 4)
+    a = rng.standard_normal((m, k)).astype(np.float32)
+    x, mn = (p[:, :k] for p in parts(b))
+    want = a.astype(np.float64) @ (x - mn).T
+    off = [np.linalg.norm(run(dev, b, n, k, a, "f32", exact_weights=e) - want) / np.linalg.norm(want) for e in (False, True)]
+    assert off[0] <= 1.02 * off[1], off  # (equal where the call is on that path; else by 7 % at K = 640, by more from there on)
+
+
 def test_two_threads_with_plans_of_different_sizes():
     """Two contexts of one process, a thread each: launches with large and small rings of the same kernel do not disturb each other."""
     failed, start = [], threading.Barrier(2)
