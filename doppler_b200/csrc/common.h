@@ -177,8 +177,9 @@ dp_status dpk_dequant_q4k(dp_ctx *ctx, const uint8_t *packed, size_t rows, size_
                           void *out, dp_dtype out_dtype);
 dp_status dpk_gemv_q4k(dp_ctx *ctx, const uint8_t *W, const float *x, void *y, dp_dtype y_dtype,
                        int N, int K, float alpha, const float *residual);
+// only (optional, [M]): the rows whose entry is NaN
 dp_status dpk_gemm_q4k_simt(dp_ctx *ctx, const uint8_t *W, const void *A, dp_dtype a_dtype, void *C,
-                            dp_dtype c_dtype, int M, int N, int K, float alpha);
+                            dp_dtype c_dtype, int M, int N, int K, float alpha, const float *only = nullptr);
 enum { DPK_ROWS_PRE_NONE = 0, DPK_ROWS_PRE_RMSNORM = 1, DPK_ROWS_PRE_SILU = 2 };
 struct dpk_rows_fuse {
   int pre = 0;                      // operation on the input rows folded into the pre-pass

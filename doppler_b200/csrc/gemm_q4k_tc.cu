@@ -29,6 +29,7 @@
 
 #include <cuda.h>
 
+#include <cmath>
 #include <cstdlib>
 #include <map>
 
@@ -979,12 +980,14 @@ static dp_status gemm_q4k_tc_impl(dp_ctx *ctx, const uint8_t *W, const void *A, 
   // the range: a weight beyond f16's is an infinity in the others' tiles.  Very small weights
   // stay with the one launch that needs no pass over the rows (33 x 256 x 256: 9 against 17 us).  Shapes the others do not
   // tile ran on CUDA cores (1000 x 1000 x 1000: f32 rows 105 -> 30, f16 rows 102 -> 27 us); they still do where that is over within about 15 us, where the result
-  // is f32 and K below 640 (error of the f32 FMAs 4.1e-7 at K = 512, of the integer tiles 4.8e-7; 5.7e-7 and 4.6e-7 at 1024).
+  // is f32 and K below 640 (error of the f32 FMAs 4.1e-7 at K = 512, of the integer tiles 4.8e-7; 5.7e-7 and 4.6e-7 at 1024), and
+  // with an alpha that a row's scale might carry out of f32's range.
   // fuse->exact_weights (rows of several prompts, which were multiplied with exact weights one by one): always.
   if (exact && (c_dtype == DP_F32 || c_dtype == DP_F16)) {
     const long pair_tiles = (long)((M + 511) / 512) * ((N + 255) / 256);
     const bool few = M <= 256 || (pair_tiles * 2 <= ctx->sm_count / 2 && K <= 8192);
-    const bool whole = (double)M * N * K >= (double)(1l << 27) && (K >= 640 || c_dtype == DP_F16);
+    const float size = fabsf(alpha);
+    const bool whole = (double)M * N * K >= (double)(1l << 27) && (K >= 640 || c_dtype == DP_F16) && (size == 0.0f || (size >= 0x1p-60f && size <= 0x1p60f));
     const bool take = tiled ? (few && (long)N * K >= (1l << 19)) || (fuse && fuse->exact_weights) : whole;
     if (take) {
       DP_TRY(dpk_gemm_q4k_int(ctx, W, A, a_dtype, C, c_dtype, M, N, K, alpha, handled, fuse));

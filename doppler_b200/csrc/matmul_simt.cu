@@ -120,17 +120,19 @@ dp_status dpk_gemv_q4k(dp_ctx *ctx, const uint8_t *W, const float *x, void *y, d
 // Q4_K GEMM with f32-exact weights on the CUDA cores (any M, N, K).  64x64
 // output tile, one 32-wide sub-block of K per step, 4x4 outputs per thread.
 // This is the exact-weight path; the tensor-core path lives in gemm_q4k_tc.cu.
+// only (optional, [M]): compute the rows whose entry is NaN and leave the others alone (a block without such a row ends at once).
 // ---------------------------------------------------------------------------
 template <typename AT, typename OutT>
 __global__ void __launch_bounds__(256) gemm_q4k_simt_kernel(const uint8_t *__restrict__ W, const AT *__restrict__ A,
                                                             OutT *__restrict__ C, int M, int N, int K, int bpr,
-                                                            float alpha) {
+                                                            float alpha, const float *__restrict__ only) {
   pdl_launch();
   pdl_wait();
   __shared__ float As[32][64 + 4];  // [k][m]
   __shared__ float Ws[32][64 + 4];  // [k][n]
   const int tid = threadIdx.x;
   const int n0 = blockIdx.x * 64, m0 = blockIdx.y * 64;
+  if (only && !__syncthreads_or(tid < 64 && m0 + tid < M && isnan(only[m0 + tid]))) return;
   const int tn = tid & 15, tm = tid >> 4;  // outputs (m0+tm*4.., n0+tn*4..)
   float acc[4][4];
 #pragma unroll
@@ -196,7 +198,7 @@ __global__ void __launch_bounds__(256) gemm_q4k_simt_kernel(const uint8_t *__res
 #pragma unroll
   for (int i = 0; i < 4; i++) {
     const int m = m0 + tm * 4 + i;
-    if (m >= M) continue;
+    if (m >= M || (only && !isnan(only[m]))) continue;
 #pragma unroll
     for (int jx = 0; jx < 4; jx++) {
       const int n = n0 + tn * 4 + jx;
@@ -208,17 +210,17 @@ __global__ void __launch_bounds__(256) gemm_q4k_simt_kernel(const uint8_t *__res
 }
 
 dp_status dpk_gemm_q4k_simt(dp_ctx *ctx, const uint8_t *W, const void *A, dp_dtype a_dtype, void *C, dp_dtype c_dtype,
-                            int M, int N, int K, float alpha) {
+                            int M, int N, int K, float alpha, const float *only) {
   const int bpr = (K + QK_K - 1) / QK_K;
   dim3 grid((N + 63) / 64, (M + 63) / 64);
   if (a_dtype == DP_F32 && c_dtype == DP_F32) {
-    DP_LAUNCH(ctx, (gemm_q4k_simt_kernel<float, float>), grid, 256, 0, W, (const float *)A, (float *)C, M, N, K, bpr, alpha);
+    DP_LAUNCH(ctx, (gemm_q4k_simt_kernel<float, float>), grid, 256, 0, W, (const float *)A, (float *)C, M, N, K, bpr, alpha, only);
   } else if (a_dtype == DP_F32 && c_dtype == DP_F16) {
-    DP_LAUNCH(ctx, (gemm_q4k_simt_kernel<float, __half>), grid, 256, 0, W, (const float *)A, (__half *)C, M, N, K, bpr, alpha);
+    DP_LAUNCH(ctx, (gemm_q4k_simt_kernel<float, __half>), grid, 256, 0, W, (const float *)A, (__half *)C, M, N, K, bpr, alpha, only);
   } else if (a_dtype == DP_F16 && c_dtype == DP_F32) {
-    DP_LAUNCH(ctx, (gemm_q4k_simt_kernel<__half, float>), grid, 256, 0, W, (const __half *)A, (float *)C, M, N, K, bpr, alpha);
+    DP_LAUNCH(ctx, (gemm_q4k_simt_kernel<__half, float>), grid, 256, 0, W, (const __half *)A, (float *)C, M, N, K, bpr, alpha, only);
   } else if (a_dtype == DP_F16 && c_dtype == DP_F16) {
-    DP_LAUNCH(ctx, (gemm_q4k_simt_kernel<__half, __half>), grid, 256, 0, W, (const __half *)A, (__half *)C, M, N, K, bpr, alpha);
+    DP_LAUNCH(ctx, (gemm_q4k_simt_kernel<__half, __half>), grid, 256, 0, W, (const __half *)A, (__half *)C, M, N, K, bpr, alpha, only);
   } else {
     return dp_fail(ctx, DP_ERR_INVALID, "matmul q4k: unsupported dtypes A=%s C=%s", dp_dtype_name(a_dtype), dp_dtype_name(c_dtype));
   }

@@ -80,6 +80,48 @@ def test_untiled_f32_rows_keep_the_accuracy_of_f32_sums(dev, m, n, k):
     assert off[0] <= 1.02 * off[1], off  # (equal where the call is on that path; else by 7 % at K = 640, by more from there on)
 
 
+@pytest.mark.parametrize("act,out", [("f32", "f32"), ("f16", "f32"), ("f16", "f16")])
+@pytest.mark.parametrize("m,n,k", [(130, 1030, 1024), (70, 2000, 1000), (600, 300, 4100)])
+def test_rows_beyond_f16_halves(dev, m, n, k, act, out):
+    """Shapes no tile divides: rows with infinities, NaN and values at the ends of the type's range are what f32 FMAs make of them."""
+    rng = np.random.default_rng(m)
+    b = blocks(rng, n, -(-k // 256))
+    b[:, :, :4] = (10.0 ** rng.uniform(-4, -2, (n, b.shape[1], 2))).astype(np.float16).view(np.uint8).reshape(n, -1, 4)
+    a = rng.standard_normal((m, k)).astype(np.float32)
+    a[3, 5] = np.inf
+    a[4, [7, k - 1]] = -np.inf
+    a[5, 9], a[5, 11] = np.inf, -np.inf
+    a[64, k // 2] = np.nan
+    a[66] = 0.0
+    if act == "f32":
+        a[10] *= 2.0 ** 120
+        a[11] *= 2.0 ** -110
+        a[12] = np.where(np.arange(k) % 64 == 0, 1e35, 1.0) * np.sign(a[12])
+        a[13] *= 2.0 ** 71  # the last exponents that f16 halves take
+        a[14] *= 2.0 ** -46
+        a[65] *= 2.0 ** -140
+    else:
+        a[10], a[11] = np.float16(65504) * np.sign(a[10]), np.float16(6e-8) * np.sign(a[11])
+    a = a.astype(np.float32 if act == "f32" else np.float16)
+    x, mn = (p[:, :k] for p in parts(b))
+    a64 = a.astype(np.float64)
+    with np.errstate(all="ignore"):
+        want = a64 @ (x - mn).T
+        size = np.abs(a64) @ (np.abs(x) + np.abs(mn)).T
+        whole = np.isfinite(a64).all(1)
+        # FMAs in order of K: K 2^-24 of the sum of magnitudes at most
+        tol = k * 2.0 ** -24 * size + (np.abs(want) * 2.0 ** -11 + 2.0 ** -24 if out == "f16" else 2.0 ** -140)
+        got = run(dev, b, n, k, a, out)
+        fits = np.abs(want) < (65000.0 if out == "f16" else 3e38)
+        rows = whole[:, None] & fits
+        assert (np.abs(got - want)[rows] <= tol[rows]).all()
+        for r in np.flatnonzero(~whole):  # infinite or NaN, as the sum of the products is
+            w32 = (x - mn)  # (a weight of exactly zero makes NaN of an infinity on both sides)
+            sure = np.isfinite(w32).all(1)
+            assert np.array_equal(np.isnan(got[r])[sure], np.isnan(want[r])[sure]) and np.array_equal(np.sign(got[r])[sure], np.sign(want[r])[sure], equal_nan=True)
+            assert not np.isfinite(got[r]).any()
+
+
 def test_two_threads_with_plans_of_different_sizes():
     """Two contexts of one process, a thread each: launches with large and small rings of the same kernel do not disturb each other."""
     failed, start = [], threading.Barrier(2)
