@@ -805,6 +805,7 @@ dp_status dpk_gemm_q4k_int(dp_ctx *ctx, const uint8_t *W, const void *A, dp_dtyp
   const size_t sum_cols = (size_t)p.parts * p.npu * 256, s_bytes = ((size_t)M * sum_cols * 2 + 255) / 256 * 256;
   dp_status st = dp_scratch(ctx, &ctx->gemm_scratch, a_bytes * (f32a ? 2 : 1) + s_bytes + (size_t)M * 4, "matmul_a_f16");
   if (st == DP_OK && p.parts > 1) st = dp_scratch(ctx, &ctx->gemm_split_scratch, (size_t)p.parts * M * N * 4, "matmul_k_split_parts");
+  if (st == DP_ERR_OOM && guard) return DP_OK;  // no memory for the pass over the rows: the CUDA cores need none
   DP_TRY(st);
   char *base = (char *)ctx->gemm_scratch->dptr;
   __half *hi = (__half *)base, *lo = (__half *)(base + a_bytes), *sums = (__half *)(base + a_bytes * (f32a ? 2 : 1));
