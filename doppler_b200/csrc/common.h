@@ -212,6 +212,8 @@ dp_status dpk_gemm_f16w_rows(dp_ctx *ctx, const __half *W, const void *A, dp_dty
                              float alpha, bool *handled);
 dp_status dpk_gemv_f16w(dp_ctx *ctx, const __half *W, const void *A, dp_dtype a_dtype, void *C,
                         dp_dtype c_dtype, int M, int N, int K, float alpha);
+// f32 rows and results, every row bit for bit as M = 1 computes it
+dp_status dpk_gemv_f16w_each(dp_ctx *ctx, const __half *W, const float *A, float *C, int M, int N, int K);
 dp_status dpk_gemv_f32w(dp_ctx *ctx, const float *W, const float *A, float *C, int M, int N, int K,
                         float alpha);
 // Optional fusion of the decode step's per-head QK RMSNorm + RoPE + KV append into the attention

@@ -283,51 +283,69 @@ __global__ void __launch_bounds__(256) gemv_f16w_kernel(const __half *__restrict
   }
 }
 
-// M == 1, f32 activations: x is staged once per CTA in shared memory; a warp streams FOUR weight rows at a time
-// (four 16-byte loads in flight per lane and pass, two passes unrolled), so the shared-memory reads of x are
-// shared by four rows and the shuffle reduction is paid once per 32 KB of weights instead of once per 8 KB.
-template <typename OutT>
+// f32 activations, one row at a time as far as the numbers go: x is staged once per CTA in shared memory; a warp streams FOUR
+// weight rows at a time (four 16-byte loads in flight per lane and pass, two passes unrolled), so the shared-memory reads of x
+// are shared by four rows and the shuffle reduction is paid once per 32 KB of weights instead of once per 8 KB (WR = 4).
+// R activation rows (those beyond M repeat the last one and are not stored) share the weights that are read; every row's sums
+// are those of R = 1, bit for bit.
+template <typename OutT, int R, int WR>
 __global__ void __launch_bounds__(256) gemv_f16w_m1_kernel(const __half *__restrict__ W, const float *__restrict__ x,
-                                                           OutT *__restrict__ y, int N, int K, float alpha) {
+                                                           OutT *__restrict__ y, int M, int N, int K, float alpha) {
   pdl_launch();
   pdl_wait();
   extern __shared__ float xs[];
-  for (int i = threadIdx.x; i < K / 4; i += blockDim.x)
-    reinterpret_cast<float4 *>(xs)[i] = __ldg(reinterpret_cast<const float4 *>(x) + i);
+#pragma unroll
+  for (int m = 0; m < R; m++)
+    for (int i = threadIdx.x; i < K / 4; i += blockDim.x)
+      reinterpret_cast<float4 *>(xs + (size_t)m * K)[i] = __ldg(reinterpret_cast<const float4 *>(x + (size_t)min(m, M - 1) * K) + i);
   __syncthreads();
   const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   const int n16 = K / 8;
-  for (int row0 = (blockIdx.x * warps + (threadIdx.x >> 5)) * 4; row0 < N; row0 += gridDim.x * warps * 4) {
-    const uint4 *wr[4];
+  for (int row0 = (blockIdx.x * warps + (threadIdx.x >> 5)) * WR; row0 < N; row0 += gridDim.x * warps * WR) {
+    const uint4 *wr[WR];
 #pragma unroll
-    for (int r = 0; r < 4; r++) wr[r] = reinterpret_cast<const uint4 *>(W + (size_t)min(row0 + r, N - 1) * K);
-    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll 2
+    for (int r = 0; r < WR; r++) wr[r] = reinterpret_cast<const uint4 *>(W + (size_t)min(row0 + r, N - 1) * K);
+    float acc[R][WR];
+#pragma unroll
+    for (int m = 0; m < R; m++)
+#pragma unroll
+      for (int r = 0; r < WR; r++) acc[m][r] = 0.0f;
+#pragma unroll(R == 1 ? 2 : 1)
     for (int c = lane; c < n16; c += 32) {
-      uint4 wv[4];
+      uint4 wv[WR];
 #pragma unroll
-      for (int r = 0; r < 4; r++) wv[r] = __ldg(wr[r] + c);
-      const float4 x0 = *reinterpret_cast<const float4 *>(xs + 8 * c), x1 = *reinterpret_cast<const float4 *>(xs + 8 * c + 4);
+      for (int r = 0; r < WR; r++) wv[r] = __ldg(wr[r] + c);
+      float4 x0[R], x1[R];
 #pragma unroll
-      for (int r = 0; r < 4; r++) {
+      for (int m = 0; m < R; m++) {
+        x0[m] = *reinterpret_cast<const float4 *>(xs + (size_t)m * K + 8 * c);
+        x1[m] = *reinterpret_cast<const float4 *>(xs + (size_t)m * K + 8 * c + 4);
+      }
+#pragma unroll
+      for (int r = 0; r < WR; r++) {
         const __half2 *h = reinterpret_cast<const __half2 *>(&wv[r]);
         const float2 f0 = __half22float2(h[0]), f1 = __half22float2(h[1]), f2 = __half22float2(h[2]), f3 = __half22float2(h[3]);
-        float a = acc[r];
-        a = fmaf(f0.x, x0.x, a); a = fmaf(f0.y, x0.y, a); a = fmaf(f1.x, x0.z, a); a = fmaf(f1.y, x0.w, a);
-        a = fmaf(f2.x, x1.x, a); a = fmaf(f2.y, x1.y, a); a = fmaf(f3.x, x1.z, a); a = fmaf(f3.y, x1.w, a);
-        acc[r] = a;
+#pragma unroll
+        for (int m = 0; m < R; m++) {
+          float a = acc[m][r];
+          a = fmaf(f0.x, x0[m].x, a); a = fmaf(f0.y, x0[m].y, a); a = fmaf(f1.x, x0[m].z, a); a = fmaf(f1.y, x0[m].w, a);
+          a = fmaf(f2.x, x1[m].x, a); a = fmaf(f2.y, x1[m].y, a); a = fmaf(f3.x, x1[m].z, a); a = fmaf(f3.y, x1[m].w, a);
+          acc[m][r] = a;
+        }
       }
     }
 #pragma unroll
-    for (int r = 0; r < 4; r++) {
-      float a = acc[r];
+    for (int m = 0; m < R; m++)
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-      if (lane == 0 && row0 + r < N) {
-        const float v = a * alpha;
-        if constexpr (sizeof(OutT) == 4) y[row0 + r] = v; else y[row0 + r] = __float2half_rn(v);
+      for (int r = 0; r < WR; r++) {
+        float a = acc[m][r];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        if (lane == 0 && row0 + r < N && m < M) {
+          const float v = a * alpha;
+          if constexpr (sizeof(OutT) == 4) y[(size_t)m * N + row0 + r] = v; else y[(size_t)m * N + row0 + r] = __float2half_rn(v);
+        }
       }
-    }
   }
 }
 
@@ -347,15 +365,38 @@ static dp_status launch_f16w(dp_ctx *ctx, const __half *W, const AT *A, OutT *C,
   return DP_OK;
 }
 
+// f32 rows and results, every row as M = 1 computes it.  Four rows share a pass over the weights, and eight weight rows a warp
+// share the reads of them, where their values fit shared memory beside those of a second CTA.  64 rows of a 32000 x 4096 head:
+// 0.95 ms, 3.1 ms row by row; the tensor-core kernel for several rows is off by 9.7e-6 there, this one by 2.1e-7.
+dp_status dpk_gemv_f16w_each(dp_ctx *ctx, const __half *W, const float *A, float *C, int M, int N, int K) {
+  const bool four = K % 8 == 0 && K <= 6144;
+  if (four && M > 1) {
+    static dp_per_device_once limit;
+    if (limit.pending(ctx->device)) {
+      DP_CUDA(ctx, cudaFuncSetAttribute(gemv_f16w_m1_kernel<float, 4, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 6144 * 4));
+      limit.done(ctx->device);
+    }
+  }
+  int grid = (N + 63) / 64;
+  if (grid > ctx->sm_count * 8) grid = ctx->sm_count * 8;
+  for (int m = 0; m < M; m += four ? 4 : 1) {
+    const float *x = A + (size_t)m * K;
+    float *y = C + (size_t)m * N;
+    if (four && M - m > 1) DP_LAUNCH(ctx, (gemv_f16w_m1_kernel<float, 4, 8>), grid, 256, (size_t)K * 16, W, x, y, M - m < 4 ? M - m : 4, N, K, 1.0f);
+    else DP_TRY(dpk_gemv_f16w(ctx, W, x, DP_F32, y, DP_F32, 1, N, K, 1.0f));
+  }
+  return DP_OK;
+}
+
 dp_status dpk_gemv_f16w(dp_ctx *ctx, const __half *W, const void *A, dp_dtype a_dtype, void *C, dp_dtype c_dtype, int M,
                         int N, int K, float alpha) {
   if (M == 1 && a_dtype == DP_F32 && K % 8 == 0 && (size_t)K * 4 <= 48 * 1024) {
     int grid = (N + 31) / 32;  // eight warps of four rows
     if (grid > ctx->sm_count * 8) grid = ctx->sm_count * 8;
     if (c_dtype == DP_F32) {
-      DP_LAUNCH(ctx, gemv_f16w_m1_kernel<float>, grid, 256, (size_t)K * 4, W, (const float *)A, (float *)C, N, K, alpha);
+      DP_LAUNCH(ctx, (gemv_f16w_m1_kernel<float, 1, 4>), grid, 256, (size_t)K * 4, W, (const float *)A, (float *)C, 1, N, K, alpha);
     } else {
-      DP_LAUNCH(ctx, gemv_f16w_m1_kernel<__half>, grid, 256, (size_t)K * 4, W, (const float *)A, (__half *)C, N, K, alpha);
+      DP_LAUNCH(ctx, (gemv_f16w_m1_kernel<__half, 1, 4>), grid, 256, (size_t)K * 4, W, (const float *)A, (__half *)C, 1, N, K, alpha);
     }
     return DP_OK;
   }

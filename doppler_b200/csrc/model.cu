@@ -1070,7 +1070,7 @@ static dp_status run_layers(dp_model *m, int tokens, bool decode, int seq, int s
   return DP_OK;
 }
 
-// final norm + LM head for `rows` rows of hidden state starting at hrow -> m->logits
+// final norm + LM head for `rows` rows of hidden state starting at hrow -> m->logits (m->packed: every row as it would be by itself)
 static dp_status run_logits(dp_model *m, const float *hrow, int rows) {
   if (m->stack) return dp_stack_logits(m, hrow, rows);
   dp_ctx *ctx = m->ctx;
@@ -1078,6 +1078,7 @@ static dp_status run_logits(dp_model *m, const float *hrow, int rows) {
   if (!(m->final_norm_done && rows == 1))
     DP_TRY(dpk_rmsnorm(ctx, hrow, m->final_norm, false, nullptr, false, nullptr, m->n, rows, c.hidden, c.eps, false, 1.0f));
   m->final_norm_done = false;
+  if (m->packed) return dpk_gemv_f16w_each(ctx, (const __half *)m->lm_head->dptr, m->n, m->logits, rows, m->vocab_l, c.hidden);
   return dpk_gemv_f16w(ctx, (const __half *)m->lm_head->dptr, m->n, DP_F32, m->logits, DP_F32, rows, m->vocab_l, c.hidden, 1.0f);
 }
 
@@ -1228,13 +1229,12 @@ static dp_status run_packed(dp_model *m, const int32_t *seqs, const int32_t *con
     DP_TRY(dp_buf_upload(ctx, buf, host.data(), 0, host.size() * 4));
     DP_TRY(embed_rows(m, dev, rows, false));
     m->packed = &packed;
-    const dp_status st = run_layers(m, rows, false, 0, 0);
-    m->packed = nullptr;
-    DP_TRY(st);
+    DP_TRY(run_layers(m, rows, false, 0, 0));
     DP_LAUNCH(ctx, take_rows_kernel, (unsigned)n, 256, 0, (const float *)m->h, dev + 3 * rows, m->partial, c.hidden);
     return run_head(m, m->partial, n);
   };
   const dp_status st = run();
+  m->packed = nullptr;
   dp_buf_release(ctx, buf);
   DP_TRY(st);
   for (int i = 0; i < n; i++) m->seq_len[seqs[i]] += lengths[i];
@@ -1275,13 +1275,22 @@ extern "C" dp_status dp_model_prefill_many(dp_model *m, int n, const int32_t *se
     for (int j = 0; j < lengths[i]; j++)
       DP_CHECK(ctx, at[i][j] >= 0 && at[i][j] < m->cfg.vocab, "prefill: token id %d outside the vocabulary", at[i][j]);
   }
+  // A prompt of one token runs by itself: its products are those of a decode step, which keep 24 bits of the activations (error
+  // 3.1e-7 against 5.0e-7 in a pass of several rows).  Such prompts go first; the last prompt still runs last.
+  std::vector<int> order;
+  for (int single : {1, 0})
+    for (int i = 0; i < n; i++)
+      if ((lengths[i] == 1 && i < n - 1) == (single == 1)) order.push_back(i);
   const bool pack = packs(m);
+  std::vector<int32_t> next(n), seq(n), len(n);
+  std::vector<const int32_t *> prompt(n);
+  for (int i = 0; i < n; i++) { seq[i] = seqs[order[i]]; len[i] = lengths[order[i]]; prompt[i] = at[order[i]]; }
   for (int i = 0; i < n;) {
-    int e = i + 1, rows = lengths[i];
-    while (pack && e < n && rows + lengths[e] <= m->T) rows += lengths[e++];
-    if (e - i > 1) DP_TRY(run_packed(m, seqs + i, at.data() + i, lengths + i, e - i, next_tokens + i));
-    else DP_TRY(run_portion(m, "prefill", seqs[i], at[i], lengths[i], nullptr, 0, nullptr, next_tokens + i));
-    i = e;
+    int e = i + 1, rows = len[i];
+    while (pack && len[i] > 1 && e < n && len[e] > 1 && rows + len[e] <= m->T) rows += len[e++];
+    if (e - i > 1) DP_TRY(run_packed(m, &seq[i], &prompt[i], &len[i], e - i, &next[i]));
+    else DP_TRY(run_portion(m, "prefill", seq[i], prompt[i], len[i], nullptr, 0, nullptr, &next[i]));
+    for (; i < e; i++) next_tokens[order[i]] = next[i];
   }
   return DP_OK;
 }

@@ -63,3 +63,43 @@ def test_nothing_runs_where_a_prompt_is_invalid(dev):
             m.prefill_many(prompts, seqs)
     assert [m.seq_len(s) for s in range(3)] == [0, 0, 0]
     m.destroy()
+
+
+def test_logits_behind_a_shared_pass(dev):
+    """The head after a shared pass is the one-row head: f32 products and sums, not f16 halves."""
+    m = DecoderModel(dev, CFG, max_seq=64, max_batch=5)
+    m.load_all(weights())
+    H, V, last = CFG["hidden"], CFG["vocab"], 30
+    m.prefill_many([np.arange(k) * 7 % V for k in (5, 9, 2, 33, last)], range(5))
+    x = m.read_hidden(last)[-1].astype(np.float64)  # (the last prompt's rows come first)
+    w = weights()
+    want = (x / np.sqrt(np.mean(x * x) + CFG["eps"]) * w["final_norm"]) @ w["lm_head"].astype(np.float64).T
+    got = m.read_logits(V)
+    # 1024 products in f32: 1.2e-7 with lanes that add 32 of them each, and the rounding of the normalised row
+    assert np.linalg.norm(got - want) < 4e-7 * np.linalg.norm(want)
+    m.destroy()
+
+
+@pytest.mark.parametrize("lengths", [[3, 2, 1], [1, 1], [1, 4, 1, 5, 1], [64, 1, 300, 1]])
+def test_prompts_of_one_token(dev, lengths):
+    """A prompt of one token is computed as by itself, bit for bit."""
+    m = DecoderModel(dev, CFG, max_seq=320, max_batch=len(lengths))
+    m.load_all(weights())
+    prompts = [(np.arange(k) * 11 + 3 * i) % CFG["vocab"] for i, k in enumerate(lengths)]
+    n = len(lengths) - 1
+    one = [m.prefill(p, seq=i) for i, p in enumerate(prompts)]
+    logits, hidden = m.read_logits(CFG["vocab"]), m.read_hidden()
+    m.reset()
+    assert m.prefill_many(prompts, range(n + 1)) == one
+    assert [m.seq_len(i) for i in range(n + 1)] == lengths
+    if lengths[-1] == 1:
+        assert np.array_equal(m.read_logits(CFG["vocab"]), logits) and np.array_equal(m.read_hidden(), hidden)
+    # every sequence goes on from its own state
+    follow = [m.extend([5], [0], i) for i in range(n + 1)]
+    m.reset()
+    for i, p in enumerate(prompts):
+        m.prefill(p, seq=i)
+    for i, k in enumerate(lengths):
+        want = m.extend([5], [0], i)
+        assert np.array_equal(follow[i], want) if k == 1 else np.sqrt(np.mean((follow[i] - want) ** 2)) < 1e-4 * want.std()
+    m.destroy()
