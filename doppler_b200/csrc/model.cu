@@ -1118,9 +1118,9 @@ static dp_status embed_rows(dp_model *m, const int *ids, int rows, bool decode) 
 // stays with the one-row kernel, which is faster for it.
 static dp_status wanted_rows(dp_model *m, const char *op, const int32_t *want, int n, int off, float *logits) {
   dp_ctx *ctx = m->ctx;
-  const int V = m->vocab_l;
-  for (int i = 0; i < n; i += DP_WANTED_ROWS) {
-    const int cnt = n - i < DP_WANTED_ROWS ? n - i : DP_WANTED_ROWS;
+  const int V = m->vocab_l, most = dp_stack_wanted_rows(m);
+  for (int i = 0; i < n; i += most) {
+    const int cnt = n - i < most ? n - i : most;
     int at[DP_WANTED_ROWS];
     for (int j = 0; j < cnt; j++) at[j] = want[i + j] - off;
     const float *rows = nullptr;
@@ -1160,7 +1160,7 @@ static dp_status run_portion(dp_model *m, const char *op, int seq, const int32_t
       m->seq_len[seq] += cnt;
       int last = w;
       while (last < n_want && want[last] < off + cnt) last++;
-      if (m->stack && last - w > 1 && dp_stack_logits_many_ok(m)) {
+      if (m->stack && last - w > 1 && dp_stack_wanted_rows(m) > 0) {
         st = wanted_rows(m, op, want + w, last - w, off, logits + (size_t)w * m->vocab_l);
         w = last;
       }

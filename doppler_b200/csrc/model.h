@@ -70,7 +70,7 @@ dp_status dp_stack_ready(dp_model *m);  // every tensor loaded
 dp_status dp_stack_embed(dp_model *m, const int *ids, int rows, bool decode);
 dp_status dp_stack_run_layers(dp_model *m, int rows, bool decode, int seq, int start_pos);
 dp_status dp_stack_logits(dp_model *m, const float *hrow, int rows);
-// logits of rows at[0..n) of m->h, 2 to DP_WANTED_ROWS of them, in a buffer of the model; where dp_stack_logits_many_ok
+// logits of rows at[0..n) of m->h, 2 to dp_stack_wanted_rows of them (0: none), in the activations of the portion that has run
 constexpr int DP_WANTED_ROWS = 32;
-bool dp_stack_logits_many_ok(dp_model *m);
+int dp_stack_wanted_rows(dp_model *m);
 dp_status dp_stack_logits_many(dp_model *m, const int *at, int n, const float **out);

@@ -92,7 +92,6 @@ struct dp_stack {
   __nv_bfloat16 *final_norm = nullptr;
   uint64_t missing = 0;
   dp_buf vectors = nullptr, state = nullptr, acts = nullptr, entries = nullptr;
-  dp_buf wanted = nullptr;     // logits of several places of a portion, and their normed rows before them (null: one by one)
   int n_entries = 0, max_channels = 0;
   size_t state_bytes = 0;
   float *x[2], *y, *proj, *q, *xbc, *dt, *mix, *act_f32;
@@ -814,8 +813,6 @@ extern "C" dp_status dp_model_create_stack(dp_ctx *ctx, const dp_stack_cfg *cfg,
     s->state_bytes += s->state->bytes;
     DP_TRY(carve(&s->acts, "activations", [&](Carver &k) { carve_acts(m, k); }));
     DP_TRY(dp_buf_acquire(ctx, scratch, "attention_split_partials", &m->attn_scratch));
-    if (dpk_head_rows_ok(c.width))
-      DP_TRY(dp_buf_acquire(ctx, up(dpk_head_rows_scratch(c.width), 256) + (size_t)DP_WANTED_ROWS * c.vocab * 4, "wanted_logits", &s->wanted));
     // one stream: in = out = 1, mix = 1, the plain residual sum, unless vectors are loaded
     if (c.streams == 1) {
       const float v = 1.0f, mult = c.residual_mult == 0.0f ? 1.0f : c.residual_mult;
@@ -871,7 +868,7 @@ void dp_stack_destroy(dp_model *m) {
       for (const Mat *t : {&L.proj, &L.o, &L.gateup, &L.down, &L.a2, &L.g2, &L.uq, &L.uk, &L.uv, &L.ukv}) rel(t->buf);
   rel(s->expanded);
   for (RopeTable &t : s->ropes) rel(t.buf);
-  rel(s->embed.buf); rel(s->vectors); rel(s->state); rel(s->acts); rel(s->entries); rel(s->wanted);
+  rel(s->embed.buf); rel(s->vectors); rel(s->state); rel(s->acts); rel(s->entries);
   delete s;
   m->stack = nullptr;
 }
@@ -1066,13 +1063,22 @@ dp_status dp_stack_logits(dp_model *m, const float *hrow, int rows) {
   return product(m, s->embed, s->a, st, m->logits, rows);
 }
 
-bool dp_stack_logits_many_ok(dp_model *m) { return m->stack->wanted != nullptr; }
+// Logits of several places of a portion, and their normed rows before them, go where the portion's activations were: behind
+// m->h nothing of them is read again.  (A buffer of their own was 19 MB for every model at a vocabulary of 151936, or, acquired by
+// the first call that needs it, 6 to 13 ms of that call.)
+int dp_stack_wanted_rows(dp_model *m) {
+  dp_stack *s = m->stack;
+  if (!dpk_head_rows_ok(s->cfg.width)) return 0;
+  const size_t room = s->acts->bytes - (size_t)((char *)s->proj - (char *)s->acts->dptr), scratch = up(dpk_head_rows_scratch(s->cfg.width), 256);
+  const size_t rows = room > scratch ? (room - scratch) / ((size_t)s->cfg.vocab * 4) : 0;
+  return rows < 2 ? 0 : rows < DP_WANTED_ROWS ? (int)rows : DP_WANTED_ROWS;
+}
 
 dp_status dp_stack_logits_many(dp_model *m, const int *at, int n, const float **out) {
   dp_stack *s = m->stack;
   GroupNorm g;
   g.w = s->final_norm; g.groups = s->cfg.norm_groups; g.eps = s->cfg.eps;
-  float *rows = (float *)((char *)s->wanted->dptr + up(dpk_head_rows_scratch(s->cfg.width), 256));
+  float *rows = (float *)((char *)s->proj + up(dpk_head_rows_scratch(s->cfg.width), 256));
   *out = rows;
-  return dpk_head_rows(m->ctx, m->h, s->cfg.width, at, n, g, s->embed.w(), s->embed.stride, s->wanted->dptr, rows, s->embed.N, s->cfg.width);
+  return dpk_head_rows(m->ctx, m->h, s->cfg.width, at, n, g, s->embed.w(), s->embed.stride, s->proj, rows, s->embed.N, s->cfg.width);
 }
