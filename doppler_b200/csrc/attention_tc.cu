@@ -73,8 +73,8 @@ __global__ void __launch_bounds__(ATC_THREADS, 2) attn_tc_kernel(dpk_attn_params
   const int h0 = kvh * G + ht * gt;
 
   // Where the kernel appends the new key and value itself, what it reads of the cache, and lengths and positions, come from
-  // earlier steps (which ended before this one's first kernel began): the first tiles are asked for before the previous
-  // kernel, which brings the new token's projections, has ended.
+  // earlier steps, which are complete when a kernel of this one starts (pdl.cuh): the first tiles are asked for before the
+  // previous kernel, which brings the new token's projections, has ended.
   const bool fused = p.fuse.qkv != nullptr;
   if (!fused) pdl_wait();
   int kv_len = p.kv_lens ? min(max(p.kv_lens[b], 0), p.kv_len) : p.kv_len;  // the host checked the cache for p.kv_len keys

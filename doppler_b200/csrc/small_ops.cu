@@ -233,8 +233,8 @@ dp_status dpk_residual_add(dp_ctx *ctx, const float *a, const float *b, float *o
 // src/gpu/kernels/gather_f16.wgsl:35-66: embedding rows f16 -> f32
 __global__ void gather_f16_kernel(const int *__restrict__ ids, const __half *__restrict__ table, float *__restrict__ out,
                                   int hidden) {
-  pdl_launch();
   pdl_wait();
+  pdl_launch();  // the first kernel of a decode step: no other starts before the previous step is complete (pdl.cuh)
   // 16-byte pieces where the rows allow it: one value at a time the single row of a decode step of 4096 values took 9 us
   const int t = blockIdx.x;
   const __half *row = table + (size_t)ids[t] * hidden;

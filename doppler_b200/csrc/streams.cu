@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(256) stream_sum_kernel(const float *__restrict
 __global__ void __launch_bounds__(256) stream_embed_kernel(const int *__restrict__ ids, const __nv_bfloat16 *__restrict__ table, int table_stride, float scale,
                                                            int S, int H, float *__restrict__ x, const float *__restrict__ in, float *__restrict__ u, int rows) {
   pdl_wait();
-  pdl_launch();
+  pdl_launch();  // the first kernel of a decode step (pdl.cuh)
   float w = 0.0f;
   if (u) for (int s = 0; s < S; s++) w += in[s];
   const size_t total = (size_t)rows * H;
