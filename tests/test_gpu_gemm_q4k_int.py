@@ -148,3 +148,57 @@ def test_two_threads_with_plans_of_different_sizes():
     for t in threads:
         t.join()
     assert not failed, failed
+
+
+EPILOGUES = {
+    # norm folded into q|k|v and gate|up, silu(gate) * up stored, residual added where the parts of K are summed
+    "parts": dict(hidden=1024, n_heads=16, n_kv_heads=8, head_dim=128, inter=3072),
+    # the same, residual added by the products themselves (K too short to be cut)
+    "whole": dict(hidden=4096, n_heads=4, n_kv_heads=2, head_dim=128, inter=512),
+}
+
+
+@pytest.mark.parametrize("rows", [65, 131, 256, 300])
+@pytest.mark.parametrize("name", EPILOGUES)
+def test_epilogues_through_one_layer(dev, name, rows):
+    """The norm, silu and residual fusions, through the hidden rows of one decoder layer in 64 bits."""
+    from doppler_b200.model import DecoderModel
+    from model_util import gaussian_model_weights
+
+    cfg = dict(EPILOGUES[name], n_layers=1, vocab=300, eps=1e-6, rope_theta=1e6)
+    w = gaussian_model_weights(cfg, 3)
+    m = DecoderModel(dev, cfg, max_seq=rows, max_batch=1)
+    m.load_all(w)
+    t = np.random.default_rng(rows).integers(0, cfg["vocab"], rows)
+    m.prefill(t)
+    got = m.read_hidden(rows).astype(np.float64)
+    m.destroy()
+
+    H, D, Q, G = cfg["hidden"], cfg["head_dim"], cfg["n_heads"], cfg["n_kv_heads"]
+    lw, size = w["layers"][0], {"wq": (Q * D, H), "wk": (G * D, H), "wv": (G * D, H), "wo": (H, Q * D), "wgate": (cfg["inter"], H), "wup": (cfg["inter"], H),
+                                "wdown": (H, cfg["inter"])}
+    mat = {k: np.subtract(*parts(np.asarray(lw[k], np.uint8).reshape(n, -1, 144))) for k, (n, _) in size.items()}
+    rms = lambda x, g: x / np.sqrt((x * x).mean(-1, keepdims=True) + cfg["eps"]) * g  # noqa: E731
+    angle = np.arange(rows)[:, None, None] * (cfg["rope_theta"] ** (-np.arange(0, D, 2) / D)).astype(np.float32).astype(np.float64)
+
+    def turn(x):
+        a, b = x[..., :D // 2], x[..., D // 2:]
+        return np.concatenate([a * np.cos(angle) - b * np.sin(angle), a * np.sin(angle) + b * np.cos(angle)], -1)
+
+    x = w["embed"][t].astype(np.float64)
+    h = rms(x, lw["in_norm"])
+    q, k, v = ((h @ mat[n].T).reshape(rows, -1, D) for n in ("wq", "wk", "wv"))
+    q, k = turn(rms(q, lw["q_norm"])), turn(rms(k, lw["k_norm"])).astype(np.float16).astype(np.float64)
+    v = v.astype(np.float16).astype(np.float64)
+    s = np.einsum("thd,shd->hts", q, k.repeat(Q // G, 1)) / np.sqrt(D)
+    s[:, np.triu(np.ones((rows, rows), bool), 1)] = -np.inf
+    p = np.exp(s - s.max(-1, keepdims=True))
+    o = np.einsum("hts,shd->thd", p / p.sum(-1, keepdims=True), v.repeat(Q // G, 1)).reshape(rows, -1)
+    x = x + o @ mat["wo"].T
+    h = rms(x, lw["post_norm"])
+    g = h @ mat["wgate"].T
+    x = x + (g / (1.0 + np.exp(-g)) * (h @ mat["wup"].T)) @ mat["wdown"].T
+    # f32 sums alone: about 1e-6.  An f16 cache entry on the other side of a rounding boundary is off by 2^-11 of itself, and a
+    # key or value off by 1e-6 is there for one entry in 500: 2^-11 / sqrt(500) = 2e-5 of the attention's share of a row
+    err = np.sqrt(((got - x) ** 2).mean()) / x.std()
+    assert err < 4e-5, err
