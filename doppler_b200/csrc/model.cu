@@ -1315,7 +1315,8 @@ static dp_status record_decode_step(dp_model *m, int batch) {
   DP_TRY(run_layers(m, batch, true, 0, 0));
   if (batch == 1 && m->cfg.tp_size == 1) {
     DP_TRY(run_logits(m, m->h, 1));
-    const int blocks = m->vocab_l < 148 * 256 ? (m->vocab_l + 255) / 256 : 148;
+    const int most = ctx->sm_count < 256 ? ctx->sm_count : 256;  // (one block per SM; am_vals holds 256 entries a sequence)
+    const int blocks = m->vocab_l < most * 256 ? (m->vocab_l + 255) / 256 : most;
     DP_LAUNCH(ctx, pick_advance_kernel, blocks, 256, 0, (const float *)m->logits, m->vocab_l, m->am_vals, m->am_idx, m->d_step + 1, m->d_pos, m->d_kvlen, m->d_tok, m->d_step,
               (int *)m->out_tokens->dptr, m->d_ticket);
     return DP_OK;
