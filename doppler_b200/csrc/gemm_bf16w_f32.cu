@@ -11,7 +11,7 @@
 // are the MMA's M side (128 rows), the activation rows its N side (32..128, chosen so that the tiles fill whole waves); a
 // stage of the ring holds the weight tile once and the three terms of the activations.  Persistent, one CTA per SM.  The
 // products of a 700-token prompt (width 1024, 4 layers) average 41 us and 4 us for the terms; the prompt and four tokens
-// behind it take 3.29 ms, 5.97 ms with CUDA-core FMAs.
+// behind it took 5.97 ms with CUDA-core FMAs, 3.29 with these products, and take 2.94 ms now.
 // Every wait is bounded.
 //
 // Optional decay and gated activation as in gemm_bf16.cu, the activation stored as f32.

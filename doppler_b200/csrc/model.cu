@@ -712,15 +712,15 @@ static dp_status q4k_linear(dp_model *m, const uint8_t *W, const float *x, float
   }
   // the GEMM may not alias its output with the residual: go through the partial buffer
   float *dst = (residual && residual == y) ? m->partial : y;
-  // Prefill chunks of 32 rows or more run on the tensor-core kernel: each activation row is scaled into f16
-  // range by a power of two (FFN intermediates of a random-init model reach 1e7, far outside f16) and
-  // scaled back in the epilogue.  Default: three passes, A_hi.W_hi + A_lo.W_hi + A_hi.W_lo with the f16
-  // rounding residues of activations and weights, which reproduces the f32-exact product (the reference's
-  // rule for f32 activations, matmul.rules.json:15-22) to f32 accuracy at about a tenth of the CUDA-core
-  // kernel's time.  DP_PREFILL_TC=1: one pass, activations and weights rounded to f16 as in the reference's
-  // tiled f16 prefill kernel (fused_matmul_q4_prefill_tiled_f16.wgsl), about 1e-3 of the output's rms away
-  // from the exact product; DP_PREFILL_TC=0, small chunks and shapes the tensor-core kernel does not tile:
-  // the f32-exact CUDA-core kernel.
+  // Several rows run on the tensor-core kernels: each activation row is scaled into f16 range by a power of two (FFN
+  // intermediates of a random-init model reach 1e7, far outside f16) and scaled back in the epilogue.  Default: the f32
+  // product (the reference's rule for f32 activations, matmul.rules.json:15-22), with integer weight tiles and the rows
+  // as two f16 halves (gemm_q4k_int.cu, gemm_q4k_tc_rows.cu) or, on full waves, in three passes A_hi.W_hi + A_lo.W_hi +
+  // A_hi.W_lo with the f16 rounding residues of activations and weights; rows of several prompts (exact_weights) always with
+  // integer tiles, to the accuracy that the prompts have one by one.  DP_PREFILL_TC=1: one pass, activations and weights
+  // rounded to f16 as in the reference's tiled f16 prefill kernel (fused_matmul_q4_prefill_tiled_f16.wgsl), about 1e-3 of
+  // the output's rms away from the exact product; DP_PREFILL_TC=0 and few rows of shapes those kernels do not take: the
+  // f32-exact CUDA-core kernel.
   static int prefill_tc = -1;
   if (prefill_tc < 0) { const char *e = getenv("DP_PREFILL_TC"); prefill_tc = e ? atoi(e) : 3; }
   bool handled = false;

@@ -148,10 +148,15 @@ uint32_t dp_recorder_op_count(dp_recorder *rec);
  * M>1 with Q4_K weights follows the reference's rule (matmul.rules.json:15-22):
  * the dequantised weights enter the product with f32 accuracy and the sum is
  * kept in f32 (f16 outputs are rounded once, at the store:
- * fused_matmul_q4_batched_f16a.wgsl:107,151).  On the tensor cores that is the
- * f16 halves AND the f16 rounding residues of the weights (and, for f32
- * activations from 32 rows on, of the activations) multiplied into one f32
- * accumulator; smaller or untiled f32 problems run on CUDA cores.
+ * fused_matmul_q4_batched_f16a.wgsl:107,151).  On the tensor cores that is,
+ * up to 256 rows and wherever the launch is short of a wave, integer weight
+ * tiles (sc * q, exact in f16) times the activations (f32 ones as two f16
+ * halves), d applied per super-block and the min term a product of its own;
+ * on full waves the f16 halves AND the f16 rounding residues of the weights
+ * (and of f32 activations) multiplied into one f32 accumulator.  Shapes that
+ * no tile divides (N % 128, K % 256) take the integer tiles from M*N*K = 2^27
+ * on; smaller ones, f32 results of K < 640, and rows that f16 halves do not
+ * hold (infinities, largest values beyond 2^+-60) run on CUDA cores.
  * opts.f16_weights = 1 selects the numerics of the reference's opt-in tiled
  * prefill kernel instead (fused_matmul_q4_prefill_tiled_f16.wgsl:201: every
  * dequantised weight rounded to f16 first), one tensor-core product. */
@@ -348,7 +353,9 @@ dp_status dp_model_reset(dp_model *m);
 /* prompt of n tokens for sequence `seq`; next_token receives the greedy token */
 dp_status dp_model_prefill(dp_model *m, int seq, const int32_t *tokens, int n, int32_t *next_token);
 /* the same for n prompts of n different sequences: tokens holds them one behind the other, lengths[i] of them for
- * sequence seqs[i].  Short prompts share passes over the layers.  Nothing runs if one of them is invalid. */
+ * sequence seqs[i].  Prompts of two tokens and more share passes over the layers on one GPU where heads of 128 values come in
+ * groups of 1, 2, 4 or 8 per key/value head; else, and for decoders described layer by layer, one pass per prompt.
+ * Nothing runs if one of them is invalid. */
 dp_status dp_model_prefill_many(dp_model *m, int n, const int32_t *seqs, const int32_t *tokens, const int32_t *lengths,
                                 int32_t *next_tokens);
 /* `steps` greedy decode steps for `batch` sequences; out_tokens is [steps][batch] */
