@@ -122,6 +122,33 @@ def test_rows_beyond_f16_halves(dev, m, n, k, act, out):
             assert not np.isfinite(got[r]).any()
 
 
+@pytest.mark.parametrize("m,n,k", [(130, 1030, 1024), (600, 300, 4100)])
+def test_rows_beyond_f16_halves_in_a_graph(dev, m, n, k):
+    """A recorded product meets such rows first when it is replayed."""
+    rng = np.random.default_rng(m)
+    b = blocks(rng, n, -(-k // 256))
+    w, t = dev.weight_from(b.ravel(), "q4k", [n, k]), dev.tensor_from(rng.standard_normal((m, k)).astype(np.float32))
+    out = dev.acquire_buffer(m * n * 4, "out")
+    rec = ops.CommandRecorder(dev, "graph", capture_graph=True)
+    c = ops.record_matmul(rec, t, w, m, n, k, output_buffer=out, output_dtype="f32")
+    graph = rec.finish_graph()
+    for scale in (1.0, 2.0 ** 118, 2.0 ** -105):
+        a = rng.standard_normal((m, k)).astype(np.float32)
+        a[::3] *= np.float32(scale)
+        a[1, 5] = np.inf
+        dev.upload_data(t.buffer, a)
+        graph.launch()
+        got = dev.read_tensor(c).reshape(m, n)
+        assert np.array_equal(got, run(dev, b, n, k, a, "f32").astype(np.float32), equal_nan=True)
+        if scale != 1.0:
+            exact = run(dev, b, n, k, a, "f32", exact_weights=True).astype(np.float32)
+            rows = [r for r in range(m) if r % 3 == 0 or r == 1]
+            assert np.array_equal(got[rows], exact[rows], equal_nan=True)
+    graph.destroy()
+    for x in (out, t.buffer, w.buffer):
+        dev.release_buffer(x)
+
+
 def test_two_threads_with_plans_of_different_sizes():
     """Two contexts of one process, a thread each: launches with large and small rings of the same kernel do not disturb each other."""
     failed, start = [], threading.Barrier(2)
