@@ -92,6 +92,7 @@ struct dp_stack {
   __nv_bfloat16 *final_norm = nullptr;
   uint64_t missing = 0;
   dp_buf vectors = nullptr, state = nullptr, acts = nullptr, entries = nullptr;
+  dp_buf wanted = nullptr;     // logits of several places of a portion, where its activations are too small for them
   int n_entries = 0, max_channels = 0;
   size_t state_bytes = 0;
   float *x[2], *y, *proj, *q, *xbc, *dt, *mix, *act_f32;
@@ -251,6 +252,16 @@ void carve_acts(dp_model *m, Carver &c) {
   char *a = nullptr, *act = nullptr;
   c.take(&a, T * k * e); c.take(&act, T * ff * e); c.take(&s->act_f32, ff);
   s->a = a; s->act = act;
+}
+
+// Logits of several places of a portion, and their normed rows before them, go where the portion's f32 activations were: from
+// proj to the delta rule's records nothing is read again.  (Not further: 16-bit rows have padding that products may read against
+// zero weights, and halves of an f32 number can be infinities.)  Portions of few rows have a buffer of their own for them; with
+// one for every model, 19 MB at a vocabulary of 151936 lay idle in most, and acquired by the first call that needs it, it cost that
+// call 6 to 13 ms.
+size_t wanted_room(const dp_stack *s) { return (size_t)((char *)s->dl.records - (char *)s->proj); }
+size_t wanted_bytes(const dp_model *m, int rows) {
+  return up(dpk_head_rows_scratch(m->stack->cfg.width), 256) + (size_t)rows * m->stack->cfg.vocab * 4;
 }
 
 SublayerIn sub_in(const dp_stack *s, const StackLayer &L, int q) {
@@ -813,6 +824,9 @@ extern "C" dp_status dp_model_create_stack(dp_ctx *ctx, const dp_stack_cfg *cfg,
     s->state_bytes += s->state->bytes;
     DP_TRY(carve(&s->acts, "activations", [&](Carver &k) { carve_acts(m, k); }));
     DP_TRY(dp_buf_acquire(ctx, scratch, "attention_split_partials", &m->attn_scratch));
+    const size_t places = wanted_bytes(m, m->T < DP_WANTED_ROWS ? m->T : DP_WANTED_ROWS);  // of one block of a portion
+    if (dpk_head_rows_ok(c.width) && wanted_room(s) < places && dp_buf_acquire(ctx, places, "wanted_logits", &s->wanted) != DP_OK)
+      s->wanted = nullptr;  // fewer at a time, or one by one
     // one stream: in = out = 1, mix = 1, the plain residual sum, unless vectors are loaded
     if (c.streams == 1) {
       const float v = 1.0f, mult = c.residual_mult == 0.0f ? 1.0f : c.residual_mult;
@@ -868,7 +882,7 @@ void dp_stack_destroy(dp_model *m) {
       for (const Mat *t : {&L.proj, &L.o, &L.gateup, &L.down, &L.a2, &L.g2, &L.uq, &L.uk, &L.uv, &L.ukv}) rel(t->buf);
   rel(s->expanded);
   for (RopeTable &t : s->ropes) rel(t.buf);
-  rel(s->embed.buf); rel(s->vectors); rel(s->state); rel(s->acts); rel(s->entries);
+  rel(s->embed.buf); rel(s->vectors); rel(s->state); rel(s->acts); rel(s->entries); rel(s->wanted);
   delete s;
   m->stack = nullptr;
 }
@@ -1063,22 +1077,21 @@ dp_status dp_stack_logits(dp_model *m, const float *hrow, int rows) {
   return product(m, s->embed, s->a, st, m->logits, rows);
 }
 
-// Logits of several places of a portion, and their normed rows before them, go where the portion's activations were: behind
-// m->h nothing of them is read again.  (A buffer of their own was 19 MB for every model at a vocabulary of 151936, or, acquired by
-// the first call that needs it, 6 to 13 ms of that call.)
 int dp_stack_wanted_rows(dp_model *m) {
   dp_stack *s = m->stack;
   if (!dpk_head_rows_ok(s->cfg.width)) return 0;
-  const size_t room = s->acts->bytes - (size_t)((char *)s->proj - (char *)s->acts->dptr), scratch = up(dpk_head_rows_scratch(s->cfg.width), 256);
-  const size_t rows = room > scratch ? (room - scratch) / ((size_t)s->cfg.vocab * 4) : 0;
-  return rows < 2 ? 0 : rows < DP_WANTED_ROWS ? (int)rows : DP_WANTED_ROWS;
+  int n = m->T < DP_WANTED_ROWS ? m->T : DP_WANTED_ROWS;
+  const size_t room = s->wanted ? s->wanted->bytes : wanted_room(s);
+  while (n > 1 && wanted_bytes(m, n) > room) n--;
+  return n < 2 ? 0 : n;
 }
 
 dp_status dp_stack_logits_many(dp_model *m, const int *at, int n, const float **out) {
   dp_stack *s = m->stack;
   GroupNorm g;
   g.w = s->final_norm; g.groups = s->cfg.norm_groups; g.eps = s->cfg.eps;
-  float *rows = (float *)((char *)s->proj + up(dpk_head_rows_scratch(s->cfg.width), 256));
+  char *base = s->wanted ? (char *)s->wanted->dptr : (char *)s->proj;
+  float *rows = (float *)(base + wanted_bytes(m, 0));
   *out = rows;
-  return dpk_head_rows(m->ctx, m->h, s->cfg.width, at, n, g, s->embed.w(), s->embed.stride, s->proj, rows, s->embed.N, s->cfg.width);
+  return dpk_head_rows(m->ctx, m->h, s->cfg.width, at, n, g, s->embed.w(), s->embed.stride, base, rows, s->embed.N, s->cfg.width);
 }
