@@ -184,7 +184,9 @@ __global__ void __launch_bounds__(QI_THREADS, 1) gemm_q4k_int_kernel(const __gri
   // unit -> super-block: every item starts at its own place, so that clusters do not ask L2 for the same lines at once
   auto block_of = [&](int item, int u) { return part_of(item) * p.pb + (u - p.npu + item) % p.pb; };
 
-  pdl_launch();
+  // No early launch of dependents here: in decode steps of 65 to 256 sequences the next kernel was seen to read rows that this one
+  // (a launch of clusters without the programmatic attribute) had not stored yet, its own wait notwithstanding.  It now
+  // starts when this kernel is complete.
   pdl_wait();
   if (tid == 0) {
     for (uint32_t s = 0; s < QI_RING; s++) {
@@ -871,7 +873,7 @@ dp_status dpk_gemm_q4k_int(dp_ctx *ctx, const uint8_t *W, const void *A, dp_dtyp
     if (c_dtype == DP_F32) DP_LAUNCH(ctx, int_reduce_kernel<float>, (unsigned)grid, 256, 0, parts, (float *)final_dst, n, p.parts, residual);
     else DP_LAUNCH(ctx, int_reduce_kernel<__half>, (unsigned)grid, 256, 0, parts, (__half *)final_dst, n, p.parts, residual);
   }
-  if (guard) {  // launched while the kernel before it runs: it has nothing to do as a rule (1000 x 1000 x 1000: 26.9 us of f16 rows, 29.1 launched behind it)
+  if (guard) {  // its launch prepared while the kernel before it runs: it has nothing to do as a rule
     const bool pdl = ctx->pdl;
     ctx->pdl = true;
     st = dpk_gemm_q4k_simt(ctx, W, A, a_dtype, C, c_dtype, M, N, K, alpha, scale);

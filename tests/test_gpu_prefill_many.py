@@ -103,3 +103,26 @@ def test_prompts_of_one_token(dev, lengths):
         want = m.extend([5], [0], i)
         assert np.array_equal(follow[i], want) if k == 1 else np.sqrt(np.mean((follow[i] - want) ** 2)) < 1e-4 * want.std()
     m.destroy()
+
+
+@pytest.mark.parametrize("batch", [65, 71, 96])
+def test_steps_of_more_sequences_than_the_small_batch_kernel_takes(dev, batch):
+    """Decode steps beyond 64 sequences (another GEMM inside the step's graph): the same step after step, and the logits of the
+    same sequences in smaller groups."""
+    rng = np.random.default_rng(batch)
+    prompts = [rng.integers(0, CFG["vocab"], 2 + i % 3).tolist() for i in range(batch)]
+    V, rows = CFG["vocab"], []
+    for most in (batch, batch, 32):
+        out = []
+        m = DecoderModel(dev, CFG, max_seq=16, max_batch=most)
+        m.load_all(weights())
+        for i in range(0, batch, most):
+            part = prompts[i:i + most]
+            m.reset()
+            m.decode(m.prefill_many(part, range(len(part))), 5)
+            out.append(m.read_logits(len(part) * V).reshape(len(part), V))
+        m.destroy()
+        rows.append(np.concatenate(out))
+    assert np.array_equal(rows[0], rows[1])
+    # f32-exact products in another kernel, and cache entries on the other side of a rounding boundary
+    assert (np.linalg.norm(rows[0] - rows[2], axis=1) < 2e-3 * np.linalg.norm(rows[2], axis=1)).all()
