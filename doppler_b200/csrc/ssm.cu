@@ -204,48 +204,120 @@ __global__ void __launch_bounds__(128) ssm_conv_kernel(const float *__restrict__
 }
 
 // ---- several tokens of one sequence, token by token: grid (heads, column tiles) ----
-constexpr int SCAN_TB = 16;  // tokens staged at a time
+// Bound by instructions (two FMAs per state value and token, and one for the read-out) and the chain from token to token.
+// A warp owns all of the state of four columns: B and C of a token are read from shared memory once for them, with every
+// lane at another address; products of two columns go together (fma.rn.f32x2); and the sums over the state are left open for
+// four tokens, whose sixteen sums then cross the lanes in sixteen shuffles.  700 tokens of 32 heads x 64 values x 128 states: 345 us
+// with eight lanes per column, where all columns read the same B and C again and every token had a reduction of its own, 186 us
+// with eight columns a warp, 132 us with four.
+constexpr int SCAN_TB = 16;    // tokens staged at a time
+constexpr int SCAN_COLS = 4;   // of a warp
+constexpr int SCAN_WARPS = 4;  // 16 columns a block: 32 heads x 64 values are a block for nearly every SM
+constexpr int SCAN_THREADS = SCAN_WARPS * 32;
+
 __device__ __forceinline__ void scan_cp4(float *dst, const float *src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
+__device__ __forceinline__ void scan_cp16(float *dst, const float *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+typedef unsigned long long scan_f2;  // two floats
+__device__ __forceinline__ scan_f2 scan_pack(float a, float b) {
+  scan_f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void scan_unpack(scan_f2 v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ scan_f2 scan_fma(scan_f2 a, scan_f2 b, scan_f2 c) {
+  scan_f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ scan_f2 scan_mul(scan_f2 a, scan_f2 b) {
+  scan_f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// this lane's NV state values of a row in memory or shared memory: pieces of up to four, lanes side by side
 template <int NV>
-__global__ void __launch_bounds__(SSM_THREADS) ssm_scan_kernel(const float *__restrict__ proj, int proj_stride, const float *__restrict__ xbc,
-                                                               const float *__restrict__ dt, const SsmShape sh, const SsmWeights w, const SsmState st,
-                                                               float *__restrict__ out, int rows, int start_pos, int seq) {
+__device__ __forceinline__ void scan_load(const float *row, int lane, float (&r)[NV]) {
+  if constexpr (NV == 1) r[0] = row[lane];
+  else if constexpr (NV == 2) {
+    const float2 q = *reinterpret_cast<const float2 *>(row + 2 * lane);
+    r[0] = q.x; r[1] = q.y;
+  } else {
+#pragma unroll
+    for (int i = 0; i < NV; i += 4) {
+      const float4 q = *reinterpret_cast<const float4 *>(row + 32 * i + 4 * lane);
+      r[i] = q.x; r[i + 1] = q.y; r[i + 2] = q.z; r[i + 3] = q.w;
+    }
+  }
+}
+template <int NV>
+__device__ __forceinline__ void scan_store(float *row, int lane, const float (&r)[NV]) {
+  if constexpr (NV == 1) row[lane] = r[0];
+  else if constexpr (NV == 2) *reinterpret_cast<float2 *>(row + 2 * lane) = make_float2(r[0], r[1]);
+  else
+#pragma unroll
+    for (int i = 0; i < NV; i += 4) *reinterpret_cast<float4 *>(row + 32 * i + 4 * lane) = make_float4(r[i], r[i + 1], r[i + 2], r[i + 3]);
+}
+
+template <int NV>
+__global__ void __launch_bounds__(SCAN_THREADS) ssm_scan_kernel(const float *__restrict__ proj, int proj_stride, const float *__restrict__ xbc,
+                                                                const float *__restrict__ dt, const SsmShape sh, const SsmWeights w, const SsmState st,
+                                                                float *__restrict__ out, int rows, int start_pos, int seq, int wide) {
   pdl_launch();
   pdl_wait();
-  constexpr int NP = NV * 32, TOK = 2 * NP + SSM_COLS + 4;  // floats staged per token: B, C, x, dt
-  extern __shared__ __align__(16) float scan_smem[];         // [2][SCAN_TB][TOK], then y [SCAN_TB][SSM_COLS]
+  constexpr int NP = NV * 32, COLS = SCAN_COLS, CT = COLS * SCAN_WARPS, TOK = 2 * NP + CT + 4;  // floats staged per token: B, C, x, step, decay
+  constexpr int SUMS = 4 * COLS, PER = SCAN_TB * CT / SCAN_THREADS;
+  extern __shared__ __align__(16) float scan_smem[];  // [2][SCAN_TB][TOK], then y [SCAN_TB][CT]
   float *sy = scan_smem + 2 * SCAN_TB * TOK;
-  const int tid = threadIdx.x, h = blockIdx.x, p0 = blockIdx.y * SSM_COLS;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h = blockIdx.x, p0 = blockIdx.y * CT;
   const int P = sh.vdim, N = sh.state, G = sh.groups, inner = sh.heads * P, CH = inner + 2 * G * N;
-  const int g = h / (sh.heads / G), cols = min(SSM_COLS, P - p0);
-  const int col = tid / SSM_LANES, sub = tid % SSM_LANES;
-  for (int i = tid; i < 2 * SCAN_TB * TOK; i += SSM_THREADS) scan_smem[i] = 0.0f;  // padded state columns stay zero
+  const int g = h / (sh.heads / G), cols = min(CT, P - p0);
+  for (int i = tid; i < 2 * SCAN_TB * TOK; i += SCAN_THREADS) scan_smem[i] = 0.0f;  // padded state columns stay zero
   __syncthreads();
   auto stage = [&](int blk) {
     float *dst = scan_smem + (blk & 1) * SCAN_TB * TOK;
     const int r0 = blk * SCAN_TB, n = min(SCAN_TB, rows - r0);
-    const int per = 2 * N + cols + (w.decay ? 0 : 1);
-    for (int i = tid; i < n * per; i += SSM_THREADS) {
-      const int t = i / per, e = i - t * per;
+    for (int t = warp; t < n; t += SCAN_WARPS) {
       const float *src = xbc + (size_t)(r0 + t) * CH;
+      const float *sb = src + inner + g * N, *sc = src + inner + (G + g) * N;
       float *d = dst + t * TOK;
-      if (e < N) scan_cp4(d + e, src + inner + g * N + e);
-      else if (e < 2 * N) scan_cp4(d + NP + e - N, src + inner + (G + g) * N + e - N);
-      else if (e < 2 * N + cols) scan_cp4(d + 2 * NP + e - 2 * N, src + h * P + p0 + e - 2 * N);
-      else scan_cp4(d + 2 * NP + SSM_COLS, dt + (size_t)(r0 + t) * sh.heads + h);
+      if (wide) {  // (rows and their parts begin on 16-byte boundaries)
+        for (int e = lane * 4; e < N; e += 128) { scan_cp16(d + e, sb + e); scan_cp16(d + NP + e, sc + e); }
+      } else {
+        for (int e = lane; e < N; e += 32) { scan_cp4(d + e, sb + e); scan_cp4(d + NP + e, sc + e); }
+      }
+      if (lane < cols) scan_cp4(d + 2 * NP + lane, src + h * P + p0 + lane);
+      if (lane == 16 && !w.decay) scan_cp4(d + 2 * NP + CT, dt + (size_t)(r0 + t) * sh.heads + h);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  float4 v[NV];
-  float4 *S = reinterpret_cast<float4 *>(st.s + (size_t)seq * st.s_seq + ((size_t)h * P + p0 + col) * NP) + sub;
+  scan_f2 v[COLS / 2][NV];
+  float *S = st.s + (size_t)seq * st.s_seq + ((size_t)h * P + p0 + warp * COLS) * NP;
 #pragma unroll
-  for (int i = 0; i < NV; i++) v[i] = (col < cols && start_pos > 0) ? S[8 * i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  for (int j = 0; j < COLS; j += 2) {
+    float a[NV], b[NV];
+#pragma unroll
+    for (int i = 0; i < NV; i++) a[i] = b[i] = 0.0f;
+    if (start_pos > 0 && warp * COLS + j < cols) scan_load<NV>(S + (size_t)j * NP, lane, a);
+    if (start_pos > 0 && warp * COLS + j + 1 < cols) scan_load<NV>(S + (size_t)(j + 1) * NP, lane, b);
+#pragma unroll
+    for (int i = 0; i < NV; i++) v[j / 2][i] = scan_pack(a[i], b[i]);
+  }
   const float a = w.a[h], dh = w.d ? w.d[h] : 0.0f, fixed = w.decay ? w.decay[h] : 0.0f;
   const int blocks = (rows + SCAN_TB - 1) / SCAN_TB;
   stage(0);
   for (int blk = 0; blk < blocks; blk++) {
+    const int r0 = blk * SCAN_TB, n = min(SCAN_TB, rows - r0);
+    float z[PER];  // the output gate's values of this block, on their way while its tokens are computed
+    if (sh.gated)
+#pragma unroll
+      for (int k = 0; k < PER; k++) {
+        const int i = tid + k * SCAN_THREADS, t = i / CT, c = i % CT;
+        z[k] = t < n && c < cols ? __ldg(proj + (size_t)(r0 + t) * proj_stride + h * P + p0 + c) : 0.0f;
+      }
     if (blk + 1 < blocks) {
       stage(blk + 1);
       asm volatile("cp.async.wait_group 1;" ::: "memory");
@@ -253,36 +325,83 @@ __global__ void __launch_bounds__(SSM_THREADS) ssm_scan_kernel(const float *__re
       asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
     __syncthreads();
-    const float *src = scan_smem + (blk & 1) * SCAN_TB * TOK;
-    const int r0 = blk * SCAN_TB, n = min(SCAN_TB, rows - r0);
-#pragma unroll 2
-    for (int t = 0; t < n; t++) {
-      const float *d = src + t * TOK;
-      const float step = w.decay ? 1.0f : d[2 * NP + SSM_COLS], decay = w.decay ? fixed : expf(a * step), x = d[2 * NP + col], xdt = step * x;
-      float y = 0.0f;
-#pragma unroll
-      for (int i = 0; i < NV; i++) {
-        const float4 b = *reinterpret_cast<const float4 *>(d + sub * 4 + 32 * i), c = *reinterpret_cast<const float4 *>(d + NP + sub * 4 + 32 * i);
-        v[i].x = fmaf(decay, v[i].x, xdt * b.x); v[i].y = fmaf(decay, v[i].y, xdt * b.y);
-        v[i].z = fmaf(decay, v[i].z, xdt * b.z); v[i].w = fmaf(decay, v[i].w, xdt * b.w);
-        y = fmaf(v[i].x, c.x, fmaf(v[i].y, c.y, fmaf(v[i].z, c.z, fmaf(v[i].w, c.w, y))));
-      }
-#pragma unroll
-      for (int o = 4; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
-      if (sub == 0) sy[t * SSM_COLS + col] = fmaf(dh, x, y);
+    float *src = scan_smem + (blk & 1) * SCAN_TB * TOK;
+    if (tid < n) {
+      float *d = src + tid * TOK + 2 * NP + CT;
+      const float step = w.decay ? 1.0f : d[0];
+      d[0] = step;
+      d[1] = w.decay ? fixed : expf(a * step);
     }
     __syncthreads();
-    for (int i = tid; i < n * SSM_COLS; i += SSM_THREADS) {
-      const int t = i / SSM_COLS, c = i - t * SSM_COLS;
-      if (c < cols) {
-        const int e = h * P + p0 + c;
-        out[(size_t)(r0 + t) * inner + e] = sh.gated ? sy[i] * ssm_silu(proj[(size_t)(r0 + t) * proj_stride + e]) : sy[i];
+#pragma unroll 1
+    for (int t0 = 0; t0 < n; t0 += 4) {
+      float val[SUMS];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        scan_f2 y[COLS / 2];
+#pragma unroll
+        for (int j = 0; j < COLS / 2; j++) y[j] = 0;
+        if (t0 + k < n) {  // (uniform)
+          const float *d = src + (t0 + k) * TOK;
+          float bb[NV], cc[NV];
+          scan_load<NV>(d, lane, bb);
+          scan_load<NV>(d + NP, lane, cc);
+          const float2 sd = *reinterpret_cast<const float2 *>(d + 2 * NP + CT);
+          const scan_f2 step = scan_pack(sd.x, sd.x), decay = scan_pack(sd.y, sd.y);
+          const float4 *xv = reinterpret_cast<const float4 *>(d + 2 * NP + warp * COLS);
+          scan_f2 x[COLS / 2];
+#pragma unroll
+          for (int j = 0; j < COLS / 4; j++) {
+            const float4 q = xv[j];
+            x[2 * j] = scan_mul(step, scan_pack(q.x, q.y));
+            x[2 * j + 1] = scan_mul(step, scan_pack(q.z, q.w));
+          }
+#pragma unroll
+          for (int i = 0; i < NV; i++) {
+            const scan_f2 b2 = scan_pack(bb[i], bb[i]), c2 = scan_pack(cc[i], cc[i]);
+#pragma unroll
+            for (int j = 0; j < COLS / 2; j++) {
+              v[j][i] = scan_fma(decay, v[j][i], scan_mul(x[j], b2));
+              y[j] = scan_fma(v[j][i], c2, y[j]);
+            }
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < COLS / 2; j++) scan_unpack(y[j], val[k * COLS + 2 * j], val[k * COLS + 2 * j + 1]);
       }
+      // sums across the lanes: every round halves the values a lane holds; in the end lane l holds sum l (SUMS = 16: l / 2)
+#pragma unroll
+      for (int o = 16, m = SUMS / 2; o > 0; o >>= 1, m >>= 1) {
+        if (m > 0) {
+          const bool up = lane & o;
+#pragma unroll
+          for (int i = 0; i < SUMS / 2; i++)
+            if (i < m) {
+              const float keep = up ? val[i + m] : val[i], give = up ? val[i] : val[i + m];
+              val[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+            }
+        } else {
+          val[0] += __shfl_xor_sync(0xffffffffu, val[0], o);
+        }
+      }
+      const int l = lane / (32 / SUMS), t = t0 + l / COLS, c = warp * COLS + l % COLS;
+      if (lane % (32 / SUMS) == 0 && t < n) sy[t * CT + c] = fmaf(dh, src[t * TOK + 2 * NP + c], val[0]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+      const int i = tid + k * SCAN_THREADS, t = i / CT, c = i % CT;
+      if (t < n && c < cols) out[(size_t)(r0 + t) * inner + h * P + p0 + c] = sh.gated ? sy[i] * ssm_silu(z[k]) : sy[i];
     }
   }
-  if (col < cols)
 #pragma unroll
-    for (int i = 0; i < NV; i++) S[8 * i] = v[i];
+  for (int j = 0; j < COLS; j += 2) {
+    float a2[NV], b2[NV];
+#pragma unroll
+    for (int i = 0; i < NV; i++) scan_unpack(v[j / 2][i], a2[i], b2[i]);
+    if (warp * COLS + j < cols) scan_store<NV>(S + (size_t)j * NP, lane, a2);
+    if (warp * COLS + j + 1 < cols) scan_store<NV>(S + (size_t)(j + 1) * NP, lane, b2);
+  }
 }
 
 template <typename KB, typename KF>
@@ -296,14 +415,16 @@ dp_status launch_conv(dp_ctx *ctx, bool bf16, KB kb, KF kf, dim3 grid, const flo
 template <int NV>
 dp_status launch_scan(dp_ctx *ctx, const float *proj, int proj_stride, const float *xbc, const float *dt, const SsmShape &sh, const SsmWeights &w,
                       const SsmState &st, float *out, int rows, const RowMap &map) {
-  const size_t smem = (size_t)(2 * SCAN_TB * (2 * NV * 32 + SSM_COLS + 4) + SCAN_TB * SSM_COLS) * 4;
+  constexpr int CT = SCAN_COLS * SCAN_WARPS;
+  const size_t smem = (size_t)(2 * SCAN_TB * (2 * NV * 32 + CT + 4) + SCAN_TB * CT) * 4;
   static dp_per_device_once attr;
   if (attr.pending(ctx->device)) {
     DP_CUDA(ctx, cudaFuncSetAttribute(ssm_scan_kernel<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     attr.done(ctx->device);
   }
-  DP_LAUNCH(ctx, ssm_scan_kernel<NV>, dim3(sh.heads, (sh.vdim + SSM_COLS - 1) / SSM_COLS), SSM_THREADS, smem, proj, proj_stride, xbc, dt, sh, w, st, out, rows,
-            map.start_pos, map.seq);
+  const int wide = sh.state % 4 == 0 && (sh.heads * sh.vdim) % 4 == 0 && ((uintptr_t)xbc & 15) == 0;
+  DP_LAUNCH(ctx, ssm_scan_kernel<NV>, dim3(sh.heads, (sh.vdim + CT - 1) / CT), SCAN_THREADS, smem, proj, proj_stride, xbc, dt, sh, w, st, out, rows,
+            map.start_pos, map.seq, wide);
   return DP_OK;
 }
 

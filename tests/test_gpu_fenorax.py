@@ -299,6 +299,23 @@ def test_split_keys_bf16(dev, heads, kv_heads, dim):
     m.destroy()
 
 
+@pytest.mark.parametrize("vdim,state", [(15, 3), (16, 64), (17, 36), (40, 128), (9, 130), (33, 300)])
+def test_scan_of_tokens_f32(dev, vdim, state):
+    """The recurrence token by token: columns that fill no block, states of every register count and with a padded end, portions
+    that end inside a group of four tokens and inside a stage of sixteen."""
+    cfg, cuts = config([mamba(heads=2, vdim=vdim, state=state, groups=1, norm_groups=2)]), [2, 16, 15, 4, 33]
+    w = weights(cfg)
+    t = tokens(cfg, sum(cuts), 3)
+    logits, res = ho.forward(cfg, values(w), t)
+    m = build(dev, cfg, w, len(t))
+    at = 0
+    for n in cuts:
+        check(m.extend(t[at:at + n], range(n)), logits[at:at + n], F32_TOL)
+        at += n
+    check(m.read_hidden(cuts[-1]), res[-1][-cuts[-1]:], F32_TOL)
+    m.destroy()
+
+
 def test_recurrence_in_chunks_is_32_bit(dev):
     """Inputs that bf16 holds exactly (one-hot projections of small integers, a convolution that passes its input through a
     saturated silu) leave only the recurrence's own arithmetic: chunks, token by token and the f32 mode agree closely."""
