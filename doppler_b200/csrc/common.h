@@ -180,13 +180,6 @@ dp_status dpk_gemv_q4k(dp_ctx *ctx, const uint8_t *W, const float *x, void *y, d
 // only (optional, [M]): the rows whose entry is NaN
 dp_status dpk_gemm_q4k_simt(dp_ctx *ctx, const uint8_t *W, const void *A, dp_dtype a_dtype, void *C,
                             dp_dtype c_dtype, int M, int N, int K, float alpha, const float *only = nullptr);
-enum { DPK_ROWS_PRE_NONE = 0, DPK_ROWS_PRE_RMSNORM = 1, DPK_ROWS_PRE_SILU = 2 };
-struct dpk_rows_fuse {
-  int pre = 0;                      // operation on the input rows folded into the pre-pass
-  const float *norm_w = nullptr;    // DPK_ROWS_PRE_RMSNORM
-  float eps = 0.0f;
-  const float *residual = nullptr;  // added to the output [M, N] (may be the output buffer itself)
-};
 // Optional fusions of the row-scaled tensor-core GEMM (f32 in, f32 out).  The caller asks by filling the pointers;
 // the *_done flags say what the launch took over, the rest stays with the caller.
 struct dpk_tc_fuse {
@@ -195,7 +188,7 @@ struct dpk_tc_fuse {
   float *residual_out = nullptr;    // ... which then writes here (may be the residual itself) instead of C
   const float *norm_w = nullptr;    // RMSNorm weights: A holds the un-normalised rows and the norm is folded into their conversion to f16
   float eps = 0.0f;                 //   (the call is left unhandled, nothing launched, where that conversion cannot take it)
-  bool exact_weights = false;       // the integer-tile kernel at any size
+  bool exact_weights = false;       // rows of several prompts: the order of products that costs the least accuracy, whatever their number
   bool silu_done = false, residual_done = false;
 };
 dp_status dpk_gemm_q4k_tc_rowscaled(dp_ctx *ctx, const uint8_t *W, const float *A, float *C, int M, int N, int K, float alpha, int passes,
@@ -204,8 +197,6 @@ dp_status dpk_gemm_q4k_tc_rowscaled(dp_ctx *ctx, const uint8_t *W, const float *
 // any N and K, integer weight tiles (gemm_q4k_int.cu)
 dp_status dpk_gemm_q4k_int(dp_ctx *ctx, const uint8_t *W, const void *A, dp_dtype a_dtype, void *C, dp_dtype c_dtype, int M, int N, int K, float alpha,
                            bool *handled, dpk_tc_fuse *fuse = nullptr);
-dp_status dpk_gemm_q4k_tc_rows(dp_ctx *ctx, const uint8_t *W, const void *A, dp_dtype a_dtype, float *C, int M, int N, int K, float alpha,
-                               bool *handled, const dpk_rows_fuse *fuse = nullptr);
 dp_status dpk_scale_cast_rows(dp_ctx *ctx, const float *A, __half *hi, __half *lo, float *row_scale, int M, int K);
 // f16 weights times 2..64+ activation rows, the weights streamed once (gemm_f16w_rows.cu)
 dp_status dpk_gemm_f16w_rows(dp_ctx *ctx, const __half *W, const void *A, dp_dtype a_dtype, void *C, dp_dtype c_dtype, int M, int N, int K,

@@ -50,12 +50,11 @@ struct TcSmem {
 // NPROD = products per K step that go into the one f32 accumulator:
 //   1  A . f16(W)                                   (weights rounded to f16: the opt-in tiled kernel's numerics)
 //   2  A . f16(W) + A . (W - f16(W))                (f16 activations, weights to f32 accuracy)
-//   3  A_hi . f16(W) + A_hi . (W - f16(W)) + A_lo . f16(W)   (f32 activations as two f16 halves: the f32-exact product)
-// A weight stage then holds the f16 tile and the residue tile, an activation stage the hi and the lo tiles.
+// A weight stage then holds the f16 tile and the residue tile.  (f32 activations: gemm_q4k_int.cu.)
 __host__ __device__ constexpr inline TcSmem tc_layout(int BN, int SA, int SB, int MT = 2, int NPROD = 1) {
   TcSmem l{};
-  l.stage_a = (uint32_t)MT * 128u * 128u * (NPROD == 3 ? 2u : 1u);  // MT 128-row tiles of 64 f16 (x2: hi and lo halves)
-  l.stage_b = (uint32_t)BN * 128u * (NPROD >= 2 ? 2u : 1u);
+  l.stage_a = (uint32_t)MT * 128u * 128u ;  // MT 128-row tiles of 64 f16
+  l.stage_b = (uint32_t)BN * 128u * (uint32_t)NPROD;
   l.a = 0;
   l.b = (uint32_t)SA * l.stage_a;
   l.bars = l.b + (uint32_t)SB * l.stage_b;  // full_a[SA], full_b[SB], done[max(SA, SB)], accum
@@ -68,14 +67,12 @@ __host__ __device__ constexpr inline TcSmem tc_layout(int BN, int SA, int SB, in
 // MT = number of 128-row accumulators per CTA (output tile 128*MT x BN).
 template <int BN, int DQ_WARPS, typename OutT, int SA, int SB, int MT = 2, int NPROD = 1>
 __global__ void __launch_bounds__((DQ_WARPS + 2) * 32, 1) gemm_q4k_tc_kernel(const __grid_constant__ CUtensorMap tmap_a,
-                                                                    const __grid_constant__ CUtensorMap tmap_a_lo,
                                                                     const uint8_t *__restrict__ W, OutT *__restrict__ C, int M,
                                                                     int N, int K, TcAlpha alpha, int *__restrict__ err) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const TcSmem L = tc_layout(BN, SA, SB, MT, NPROD);
   static_assert(MT * BN <= 512, "accumulators exceed tensor memory");
-  constexpr uint32_t A_TILES = (uint32_t)MT * 128u * 128u;  // bytes of the hi (or only) activation tiles of a stage
   constexpr uint32_t B_TILE = (uint32_t)BN * 128u;          // bytes of the f16 weight tile of a stage
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n0 = blockIdx.x * BN, m0 = blockIdx.y * (128 * MT);
@@ -136,8 +133,6 @@ __global__ void __launch_bounds__((DQ_WARPS + 2) * 32, 1) gemm_q4k_tc_kernel(con
 #pragma unroll
         for (int mt = 0; mt < MT; mt++) {
           tma_load_2d(dst + (uint32_t)mt * 128u * 128u, &tmap_a, ((kb0 + ((kt >> 2) + rot_b) % bpr) * 4 + (kt & 3)) * BK, m0 + 128 * mt, full_a(s));
-          if constexpr (NPROD == 3)
-            tma_load_2d(dst + A_TILES + (uint32_t)mt * 128u * 128u, &tmap_a_lo, ((kb0 + ((kt >> 2) + rot_b) % bpr) * 4 + (kt & 3)) * BK, m0 + 128 * mt, full_a(s));
         }
       }
     }
@@ -161,9 +156,7 @@ __global__ void __launch_bounds__((DQ_WARPS + 2) * 32, 1) gemm_q4k_tc_kernel(con
           for (int mt = 0; mt < MT; mt++) {
             const uint64_t adesc = umma_desc_sw128(a_addr + (uint32_t)mt * 128u * 128u + (uint32_t)k16 * 32u);
             umma_f16(tmem_base + (uint32_t)(mt * BN), adesc, bdesc, idesc, acc);
-            if constexpr (NPROD >= 2) umma_f16(tmem_base + (uint32_t)(mt * BN), adesc, umma_desc_sw128(b_addr + B_TILE + (uint32_t)k16 * 32u), idesc, 1u);
-            if constexpr (NPROD == 3)
-              umma_f16(tmem_base + (uint32_t)(mt * BN), umma_desc_sw128(a_addr + A_TILES + (uint32_t)mt * 128u * 128u + (uint32_t)k16 * 32u), bdesc, idesc, 1u);
+            if constexpr (NPROD == 2) umma_f16(tmem_base + (uint32_t)(mt * BN), adesc, umma_desc_sw128(b_addr + B_TILE + (uint32_t)k16 * 32u), idesc, 1u);
           }
         }
         // both stages are free once these MMAs have read them
@@ -266,14 +259,14 @@ __global__ void __launch_bounds__((DQ_WARPS + 2) * 32, 1) gemm_q4k_tc_kernel(con
             const float wh0 = __fmaf_rn(s_hi, qh0, -m_hi), wh1 = __fmaf_rn(s_hi, qh1, -m_hi);
             lo[i] = tc_pack_hi(wl0, wl1);
             hi[i] = tc_pack_hi(wh0, wh1);
-            if constexpr (NPROD >= 2) { rlo[i] = tc_pack_lo(wl0, wl1, lo[i]); rhi[i] = tc_pack_lo(wh0, wh1, hi[i]); }
+            if constexpr (NPROD == 2) { rlo[i] = tc_pack_lo(wl0, wl1, lo[i]); rhi[i] = tc_pack_lo(wh0, wh1, hi[i]); }
           }
           // row r of an 8-row group: 16-byte chunk c lives at chunk (c ^ r) of the 128-byte line
           uint8_t *line = bt + (uint32_t)(grp0 + dw + j * DQ_WARPS) * 1024u + (uint32_t)r8 * 128u;
           const uint32_t off_lo = ((uint32_t)oct ^ (uint32_t)r8) << 4, off_hi = ((uint32_t)(oct + 4) ^ (uint32_t)r8) << 4;
           *reinterpret_cast<uint4 *>(line + off_lo) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
           *reinterpret_cast<uint4 *>(line + off_hi) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-          if constexpr (NPROD >= 2) {  // the residue tile, same layout, behind the f16 tile
+          if constexpr (NPROD == 2) {  // the residue tile, same layout, behind the f16 tile
             *reinterpret_cast<uint4 *>(line + B_TILE + off_lo) = make_uint4(rlo[0], rlo[1], rlo[2], rlo[3]);
             *reinterpret_cast<uint4 *>(line + B_TILE + off_hi) = make_uint4(rhi[0], rhi[1], rhi[2], rhi[3]);
           }
@@ -301,7 +294,7 @@ __global__ void __launch_bounds__((DQ_WARPS + 2) * 32, 1) gemm_q4k_tc_kernel(con
     if (go) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     {
       constexpr int ET = DQ_WARPS * 32;  // epilogue threads
-      static_assert(128 * (BN * (int)sizeof(OutT) + 16) <= MT * 128 * 128 * SA * (NPROD == 3 ? 2 : 1) + BN * 128 * SB * (NPROD >= 2 ? 2 : 1),
+      static_assert(128 * (BN * (int)sizeof(OutT) + 16) <= MT * 128 * 128 * SA + BN * 128 * SB * NPROD,
                     "the output tile of a pass must fit the idle operand rings");
       const int quad = warp & 3;         // the 32 TMEM lanes this warp may read
       const int half = dw >> 2;          // DQ_WARPS/4 warps share a quarter and split the column groups
@@ -393,8 +386,7 @@ __global__ void __launch_bounds__((DQ_WARPS + 2) * 32, 1) gemm_q4k_tc_kernel(con
 // PS = passes: 256-row MMAs per pair tile (output tile 256*PS x bn).  One pass halves the activation bytes
 // per stage, which buys twice as many stages for the same shared memory.
 template <int BNMAX, typename OutT, int SA, int SB, int CH, int PS, int NPROD = 1>
-__global__ void __launch_bounds__((BNMAX / 16 + 2) * 32, 1) gemm_q4k_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
-                                                                  const __grid_constant__ CUtensorMap tmap_a_lo, const uint8_t *__restrict__ W,
+__global__ void __launch_bounds__((BNMAX / 16 + 2) * 32, 1) gemm_q4k_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const uint8_t *__restrict__ W,
                                                                   OutT *__restrict__ C, int M, int N, int K, TcAlpha alpha,
                                                                   int *__restrict__ err, int wide_tiles, int bn_wide, int bn_narrow) {
   constexpr int HBMAX = BNMAX / 2, DQ_WARPS = HBMAX / 8;  // warps 2 .. 2+DQ_WARPS-1: one 8-row group of weights each, then the epilogue
@@ -407,7 +399,6 @@ __global__ void __launch_bounds__((BNMAX / 16 + 2) * 32, 1) gemm_q4k_tc2_kernel(
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const TcSmem L = tc_layout(HBMAX, SA, SB, PS, NPROD);
-  constexpr uint32_t A_TILES = (uint32_t)PS * 128u * 128u;  // bytes of the hi (or only) activation tiles of a stage
   constexpr uint32_t B_TILE = (uint32_t)HBMAX * 128u;       // bytes of this CTA's half of the f16 weight tile of a stage
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t rank = cluster_ctarank();
@@ -466,8 +457,6 @@ __global__ void __launch_bounds__((BNMAX / 16 + 2) * 32, 1) gemm_q4k_tc2_kernel(
 #pragma unroll
         for (int ps = 0; ps < PS; ps++) {
           tma_load_2d_2sm(dst + (uint32_t)ps * 128u * 128u, &tmap_a, ((kb0 + ((kt >> 2) + rot_b) % bpr) * 4 + (kt & 3)) * BK, m0 + ps * 256 + (int)rank * 128, bar0);
-          if constexpr (NPROD == 3)
-            tma_load_2d_2sm(dst + A_TILES + (uint32_t)ps * 128u * 128u, &tmap_a_lo, ((kb0 + ((kt >> 2) + rot_b) % bpr) * 4 + (kt & 3)) * BK, m0 + ps * 256 + (int)rank * 128, bar0);
         }
       }
     }
@@ -500,9 +489,7 @@ __global__ void __launch_bounds__((BNMAX / 16 + 2) * 32, 1) gemm_q4k_tc2_kernel(
           for (int ps = 0; ps < PS; ps++) {
             const uint64_t adesc = umma_desc_sw128(a_addr + (uint32_t)ps * 128u * 128u + (uint32_t)k16 * 32u);
             umma_f16_2sm(tmem_base + (uint32_t)(ps * BNMAX), adesc, bdesc, idesc, acc);
-            if constexpr (NPROD >= 2) umma_f16_2sm(tmem_base + (uint32_t)(ps * BNMAX), adesc, umma_desc_sw128(b_addr + B_TILE + (uint32_t)k16 * 32u), idesc, 1u);
-            if constexpr (NPROD == 3)
-              umma_f16_2sm(tmem_base + (uint32_t)(ps * BNMAX), umma_desc_sw128(a_addr + A_TILES + (uint32_t)ps * 128u * 128u + (uint32_t)k16 * 32u), bdesc, idesc, 1u);
+            if constexpr (NPROD == 2) umma_f16_2sm(tmem_base + (uint32_t)(ps * BNMAX), adesc, umma_desc_sw128(b_addr + B_TILE + (uint32_t)k16 * 32u), idesc, 1u);
           }
         }
         umma_commit_2sm(done(kt % SD));  // arrives on both CTAs' barrier: their stages of this step are free
@@ -574,12 +561,12 @@ __global__ void __launch_bounds__((BNMAX / 16 + 2) * 32, 1) gemm_q4k_tc2_kernel(
             const float wh0 = __fmaf_rn(s_hi, qh0, -m_hi), wh1 = __fmaf_rn(s_hi, qh1, -m_hi);
             lo[i] = tc_pack_hi(wl0, wl1);
             hi[i] = tc_pack_hi(wh0, wh1);
-            if constexpr (NPROD >= 2) { rlo[i] = tc_pack_lo(wl0, wl1, lo[i]); rhi[i] = tc_pack_lo(wh0, wh1, hi[i]); }
+            if constexpr (NPROD == 2) { rlo[i] = tc_pack_lo(wl0, wl1, lo[i]); rhi[i] = tc_pack_lo(wh0, wh1, hi[i]); }
           }
           uint8_t *line = smem + L.b + (uint32_t)s * L.stage_b + (uint32_t)dw * 1024u + (uint32_t)r8 * 128u;
           *reinterpret_cast<uint4 *>(line + (((uint32_t)oct ^ (uint32_t)r8) << 4)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
           *reinterpret_cast<uint4 *>(line + (((uint32_t)(oct + 4) ^ (uint32_t)r8) << 4)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-          if constexpr (NPROD >= 2) {  // the residue tile, same layout, behind this CTA's half of the f16 tile
+          if constexpr (NPROD == 2) {  // the residue tile, same layout, behind this CTA's half of the f16 tile
             *reinterpret_cast<uint4 *>(line + B_TILE + (((uint32_t)oct ^ (uint32_t)r8) << 4)) = make_uint4(rlo[0], rlo[1], rlo[2], rlo[3]);
             *reinterpret_cast<uint4 *>(line + B_TILE + (((uint32_t)(oct + 4) ^ (uint32_t)r8) << 4)) = make_uint4(rhi[0], rhi[1], rhi[2], rhi[3]);
           }
@@ -603,7 +590,7 @@ __global__ void __launch_bounds__((BNMAX / 16 + 2) * 32, 1) gemm_q4k_tc2_kernel(
     if (go) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     {
       constexpr int ET = DQ_WARPS * 32;  // epilogue threads
-      static_assert(128 * (BNMAX * (int)sizeof(OutT) + 16) <= PS * 128 * 128 * SA * (NPROD == 3 ? 2 : 1) + HBMAX * 128 * SB * (NPROD >= 2 ? 2 : 1),
+      static_assert(128 * (BNMAX * (int)sizeof(OutT) + 16) <= PS * 128 * 128 * SA + HBMAX * 128 * SB * NPROD,
                     "the output tile of a pass must fit the idle operand rings");
       const int quad = warp & 3, set = dw >> 2;  // DQ_WARPS / 4 sets of four warps share the 16-column groups
       const int groups = bn / 16;
@@ -808,13 +795,13 @@ static dp_status launch_scale_cast(dp_ctx *ctx, const float *A, __half *hi, __ha
 }
 
 template <int BN, int DQ_WARPS, typename OutT, int SA, int SB, int MT, int NPROD>
-dp_status launch_tc(dp_ctx *ctx, const CUtensorMap &tm, const CUtensorMap &tm_lo, const uint8_t *W, OutT *C, int M, int N, int K, TcAlpha alpha) {
+dp_status launch_tc(dp_ctx *ctx, const CUtensorMap &tm, const uint8_t *W, OutT *C, int M, int N, int K, TcAlpha alpha) {
   constexpr size_t smem = tc_layout(BN, SA, SB, MT, NPROD).total + 1024;
   static_assert(smem <= 227 * 1024, "rings exceed shared memory");
   auto kernel = gemm_q4k_tc_kernel<BN, DQ_WARPS, OutT, SA, SB, MT, NPROD>;
   DP_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   dim3 grid(N / BN, (M + 128 * MT - 1) / (128 * MT), alpha.k_splits > 1 ? alpha.k_splits : 1);
-  DP_LAUNCH(ctx, kernel, grid, (DQ_WARPS + 2) * 32, smem, tm, tm_lo, W, C, M, N, K, alpha, ctx->dev_status);
+  DP_LAUNCH(ctx, kernel, grid, (DQ_WARPS + 2) * 32, smem, tm, W, C, M, N, K, alpha, ctx->dev_status);
   return DP_OK;
 }
 
@@ -829,7 +816,7 @@ static int tc_k_splits(dp_ctx *ctx, int tiles, int K) {
 
 // two-SM MMA variant: clusters of two CTAs along x, pair tiles of 256 * PS rows
 template <typename OutT, int BNMAX, int SA, int SB, int CH, int PS, int NPROD>
-dp_status launch_tc_2sm(dp_ctx *ctx, const CUtensorMap &tm, const CUtensorMap &tm_lo, const uint8_t *W, OutT *C, int M, int N, int K, TcAlpha alpha,
+dp_status launch_tc_2sm(dp_ctx *ctx, const CUtensorMap &tm, const uint8_t *W, OutT *C, int M, int N, int K, TcAlpha alpha,
                         int tiles, int wide_tiles, int bn_wide, int bn_narrow) {
   constexpr size_t smem = tc_layout(BNMAX / 2, SA, SB, PS, NPROD).total + 1024;
   static_assert(smem <= 227 * 1024, "rings exceed shared memory");
@@ -847,7 +834,7 @@ dp_status launch_tc_2sm(dp_ctx *ctx, const CUtensorMap &tm, const CUtensorMap &t
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, tm, tm_lo, W, C, M, N, K, alpha, ctx->dev_status, wide_tiles, bn_wide, bn_narrow);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, tm, W, C, M, N, K, alpha, ctx->dev_status, wide_tiles, bn_wide, bn_narrow);
   ctx->launches++;
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return dp_fail(ctx, DP_ERR_CUDA, "launch of gemm_q4k_tc2_kernel failed: %s", cudaGetErrorString(e));
@@ -855,11 +842,11 @@ dp_status launch_tc_2sm(dp_ctx *ctx, const CUtensorMap &tm, const CUtensorMap &t
 }
 
 // Ring depths per number of products (a stage grows with the products, shared memory does not):
-//   two-SM, tiles up to 192 wide:  1: 4 + 8 (four K steps per synchronisation)   2: 3 + 4   3: 2 + 4
-//   two-SM, tiles up to 256 wide:  1: 3 + 4   2: 3 + 4   3: 2 + 3 (one K step per synchronisation)
-//   one-SM, 192 / 128 wide:        1: 3 + 3   2: 3 + 2 / 3 + 3   3: 2 + 2 / 2 + 3
+//   two-SM, tiles up to 192 wide:  1: 4 + 8 (four K steps per synchronisation)   2: 3 + 4
+//   two-SM, tiles up to 256 wide:  1: 3 + 4   2: 3 + 4
+//   one-SM, 192 / 128 wide:        1: 3 + 3   2: 3 + 2 / 3 + 3
 template <typename OutT, int NPROD>
-dp_status dispatch_tc(dp_ctx *ctx, int bn, const CUtensorMap &tm, const CUtensorMap &tm_lo, const uint8_t *W, OutT *C, int M, int N, int K, TcAlpha alpha) {
+dp_status dispatch_tc(dp_ctx *ctx, int bn, const CUtensorMap &tm, const uint8_t *W, OutT *C, int M, int N, int K, TcAlpha alpha) {
   // Two-SM kernel (tcgen05.mma.cta_group::2) for M > 256.  On 512 x 256 pair tiles its 256-wide MMAs fetch
   // 8 KB of operands per SM and 128 cycles instead of 10 KB per 96, and the tensor pipe runs about 1.3x
   // faster per SM.  It needs whole waves of 74 clusters to win (at M = 512, 48 uniform tiles of 256 columns
@@ -871,9 +858,8 @@ dp_status dispatch_tc(dp_ctx *ctx, int bn, const CUtensorMap &tm, const CUtensor
   // Measurements of the alternatives that were tried and dropped: profiles/gemm_q4k_tc__config1.md.
   if (M > 256 && alpha.k_splits > 1 && N % 256 == 0) {  // few pair tiles: uniform 256-wide tiles, several clusters per tile along K
     const int cols = N / 256;
-    if constexpr (NPROD == 1) return launch_tc_2sm<OutT, 256, 3, 4, 2, 2, 1>(ctx, tm, tm_lo, W, C, M, N, K, alpha, cols, 0, 256, 256);
-    else if constexpr (NPROD == 2) return launch_tc_2sm<OutT, 256, 3, 4, 2, 2, 2>(ctx, tm, tm_lo, W, C, M, N, K, alpha, cols, 0, 256, 256);
-    else return launch_tc_2sm<OutT, 256, 2, 3, 1, 2, 3>(ctx, tm, tm_lo, W, C, M, N, K, alpha, cols, 0, 256, 256);
+    if constexpr (NPROD == 1) return launch_tc_2sm<OutT, 256, 3, 4, 2, 2, 1>(ctx, tm, W, C, M, N, K, alpha, cols, 0, 256, 256);
+    else return launch_tc_2sm<OutT, 256, 3, 4, 2, 2, 2>(ctx, tm, W, C, M, N, K, alpha, cols, 0, 256, 256);
   }
   if (M > 256 && N % 16 == 0) {
     const int clusters = ctx->sm_count / 2, rows = (M + 511) / 512;
@@ -885,39 +871,31 @@ dp_status dispatch_tc(dp_ctx *ctx, int bn, const CUtensorMap &tm, const CUtensor
       const int n_wide = (N - cols * narrow) / 16;  // cols * narrow + 16 * n_wide == N, n_wide < cols
       const int wide = narrow + 16, widest = n_wide ? wide : narrow;
       if (narrow >= 128 && widest <= 192) {
-        if constexpr (NPROD == 1) return launch_tc_2sm<OutT, 192, 4, 8, 4, 2, 1>(ctx, tm, tm_lo, W, C, M, N, K, alpha, cols, n_wide, wide, narrow);
-        else if constexpr (NPROD == 2) return launch_tc_2sm<OutT, 192, 3, 4, 2, 2, 2>(ctx, tm, tm_lo, W, C, M, N, K, alpha, cols, n_wide, wide, narrow);
-        else return launch_tc_2sm<OutT, 192, 2, 4, 2, 2, 3>(ctx, tm, tm_lo, W, C, M, N, K, alpha, cols, n_wide, wide, narrow);
+        if constexpr (NPROD == 1) return launch_tc_2sm<OutT, 192, 4, 8, 4, 2, 1>(ctx, tm, W, C, M, N, K, alpha, cols, n_wide, wide, narrow);
+        else return launch_tc_2sm<OutT, 192, 3, 4, 2, 2, 2>(ctx, tm, W, C, M, N, K, alpha, cols, n_wide, wide, narrow);
       }
       if (narrow >= 128 && widest <= 256) {
-        if constexpr (NPROD == 1) return launch_tc_2sm<OutT, 256, 3, 4, 2, 2, 1>(ctx, tm, tm_lo, W, C, M, N, K, alpha, cols, n_wide, wide, narrow);
-        else if constexpr (NPROD == 2) return launch_tc_2sm<OutT, 256, 3, 4, 2, 2, 2>(ctx, tm, tm_lo, W, C, M, N, K, alpha, cols, n_wide, wide, narrow);
-        else return launch_tc_2sm<OutT, 256, 2, 3, 1, 2, 3>(ctx, tm, tm_lo, W, C, M, N, K, alpha, cols, n_wide, wide, narrow);
+        if constexpr (NPROD == 1) return launch_tc_2sm<OutT, 256, 3, 4, 2, 2, 1>(ctx, tm, W, C, M, N, K, alpha, cols, n_wide, wide, narrow);
+        else return launch_tc_2sm<OutT, 256, 3, 4, 2, 2, 2>(ctx, tm, W, C, M, N, K, alpha, cols, n_wide, wide, narrow);
       }
     }
   }
   // one-SM kernel; up to 128 rows (batched decode steps) one 128-row accumulator per CTA, else two
   if (M <= 128) {
     if constexpr (NPROD == 1) {
-      if (bn == 192) return launch_tc<192, 12, OutT, 4, 4, 1, 1>(ctx, tm, tm_lo, W, C, M, N, K, alpha);
-      return launch_tc<128, 8, OutT, 4, 4, 1, 1>(ctx, tm, tm_lo, W, C, M, N, K, alpha);
+      if (bn == 192) return launch_tc<192, 12, OutT, 4, 4, 1, 1>(ctx, tm, W, C, M, N, K, alpha);
+      return launch_tc<128, 8, OutT, 4, 4, 1, 1>(ctx, tm, W, C, M, N, K, alpha);
     } else if constexpr (NPROD == 2) {
-      if (bn == 192) return launch_tc<192, 12, OutT, 4, 3, 1, 2>(ctx, tm, tm_lo, W, C, M, N, K, alpha);
-      return launch_tc<128, 8, OutT, 4, 4, 1, 2>(ctx, tm, tm_lo, W, C, M, N, K, alpha);
-    } else {
-      if (bn == 192) return launch_tc<192, 12, OutT, 3, 2, 1, 3>(ctx, tm, tm_lo, W, C, M, N, K, alpha);
-      return launch_tc<128, 8, OutT, 3, 3, 1, 3>(ctx, tm, tm_lo, W, C, M, N, K, alpha);
+      if (bn == 192) return launch_tc<192, 12, OutT, 4, 3, 1, 2>(ctx, tm, W, C, M, N, K, alpha);
+      return launch_tc<128, 8, OutT, 4, 4, 1, 2>(ctx, tm, W, C, M, N, K, alpha);
     }
   }
   if constexpr (NPROD == 1) {
-    if (bn == 192) return launch_tc<192, 12, OutT, 3, 3, 2, 1>(ctx, tm, tm_lo, W, C, M, N, K, alpha);
-    return launch_tc<128, 8, OutT, 3, 3, 2, 1>(ctx, tm, tm_lo, W, C, M, N, K, alpha);
+    if (bn == 192) return launch_tc<192, 12, OutT, 3, 3, 2, 1>(ctx, tm, W, C, M, N, K, alpha);
+    return launch_tc<128, 8, OutT, 3, 3, 2, 1>(ctx, tm, W, C, M, N, K, alpha);
   } else if constexpr (NPROD == 2) {
-    if (bn == 192) return launch_tc<192, 12, OutT, 3, 2, 2, 2>(ctx, tm, tm_lo, W, C, M, N, K, alpha);
-    return launch_tc<128, 8, OutT, 3, 3, 2, 2>(ctx, tm, tm_lo, W, C, M, N, K, alpha);
-  } else {
-    if (bn == 192) return launch_tc<192, 12, OutT, 2, 2, 2, 3>(ctx, tm, tm_lo, W, C, M, N, K, alpha);
-    return launch_tc<128, 8, OutT, 2, 3, 2, 3>(ctx, tm, tm_lo, W, C, M, N, K, alpha);
+    if (bn == 192) return launch_tc<192, 12, OutT, 3, 2, 2, 2>(ctx, tm, W, C, M, N, K, alpha);
+    return launch_tc<128, 8, OutT, 3, 3, 2, 2>(ctx, tm, W, C, M, N, K, alpha);
   }
 }
 
@@ -946,8 +924,7 @@ static dp_status gemm_q4k_tc_impl(dp_ctx *ctx, const uint8_t *W, const void *A, 
                                   int N, int K, float alpha, int mode, bool *handled, dpk_tc_fuse *fuse = nullptr) {
   // mode 0: A as given (f32 is cast to f16), weights rounded to f16: one product per K step.
   //      1: f32 rows scaled into f16 range, weights rounded to f16: one product.
-  //      2: as 1, three products per K step into the one accumulator, A_hi.W_hi + A_hi.W_lo + A_lo.W_hi with the f16
-  //         rounding residues of A and W: the f32-exact product to about 2^-21 of each term (f32 output only).
+  //      2: f32 rows, the f32-exact product: integer weight tiles (gemm_q4k_int.cu).
   //      3: f16 A, two products A.W_hi + A.W_lo: the product with weights kept to f32 accuracy (what the
   //         reference's rule-selected kernel for f16 activations computes, fused_matmul_q4_batched_f16a.wgsl:107);
   //         an f16 output is rounded once, from the f32 accumulator.
@@ -959,36 +936,28 @@ static dp_status gemm_q4k_tc_impl(dp_ctx *ctx, const uint8_t *W, const void *A, 
   if (M < 1 || (mode == 3 && a_dtype != DP_F16)) return DP_OK;
   const bool tiled = K % QK_K == 0 && N % 128 == 0, exact = (mode == 2 && a_dtype == DP_F32) || mode == 3;
   // an RMSNorm folded into the activation conversion: row-scaled f32 rows of 1024..4096 values on the kernels below only
-  if (fuse && fuse->norm_w && !(row_scaled && a_dtype == DP_F32 && c_dtype == DP_F32 && M > 64 && K % 4 == 0 && K >= 1024 && K <= 4096 &&
+  if (fuse && fuse->norm_w && !(row_scaled && a_dtype == DP_F32 && c_dtype == DP_F32 && K % 4 == 0 && K >= 1024 && K <= 4096 &&
                                  ((uintptr_t)fuse->norm_w & 15) == 0 && ((uintptr_t)A & 15) == 0))
     return DP_OK;
-  // up to 64 rows, f32 out, exact weights (modes 2 and 3): the small-batch kernel (gemm_q4k_tc_rows.cu)
-  if (M <= 64 && c_dtype == DP_F32 && exact && tiled) {
-    DP_TRY(dpk_gemm_q4k_tc_rows(ctx, W, A, a_dtype, (float *)C, M, N, K, alpha, handled));
-    if (*handled) return DP_OK;
-  }
-  if (M < 32 && (a_dtype == DP_F32 || !tiled)) return DP_OK;  // few rows on a shape that kernel does not tile: the CUDA-core kernel
-  // Exact weights: the integer-tile kernel (gemm_q4k_int.cu: one product less per K step, any shape) against the tiles of
-  // dequantised weights below, which lose less between K steps.  Measured, us, dequantised -> integer tiles:
-  //   f32 rows, M x N x K   65 x 24576 x 4096 87 -> 74, 512 x 6144 x 4096 84 -> 69, 1024 x 4096 x 4096 99 -> 93, 2048 x 1024 x 3072 66 -> 53, but
-  //                         512 x 24576 x 4096 207 -> 221, 1024 x 6144 x 4096 111 -> 120, 512 x 4096 x 12288 122 -> 131, 2048 x 4096 x 4096 143 -> 152
-  //   f16 rows              128 x 12288 x 4096 79 -> 43, 256 x 4096 x 4096 74 -> 43, 512 x 4096 x 4096 73 -> 53, but 512 x 12288 x 4096 75 -> 88
-  // so it takes what fills less than half a wave of the others' 512 x 256 pair tiles and has K up to 8192, and up to 256 rows at
-  // any N and K: there 40 to 390 % of its speed is gained with most shapes of f16 rows and up to 50 % with most of f32 rows (16 %
-  // lost at worst: 128 x 6144 x 4096 f32 37 -> 44, 100 x 24576 x 4096 f32 87 -> 102; f16 with K of 1024 and less 12 -> 15, 18 -> 21,
-  // 256 x 24576 x 4096 f16 93 -> 103), and everywhere the accuracy (3.7e-6 to 2.2e-5 -> 9e-7 for f32 rows, 4e-7 for f16 rows) and
-  // the range: a weight beyond f16's is an infinity in the others' tiles.  Very small weights
-  // stay with the one launch that needs no pass over the rows (33 x 256 x 256: 9 against 17 us).  Shapes the others do not
-  // tile ran on CUDA cores (1000 x 1000 x 1000: f32 rows 105 -> 30, f16 rows 102 -> 27 us); they still do where that is over within about 15 us, where the result
-  // is f32 and K below 640 (error of the f32 FMAs 4.1e-7 at K = 512, of the integer tiles 4.8e-7; 5.7e-7 and 4.6e-7 at 1024), and
-  // with an alpha that a row's scale might carry out of f32's range.
-  // fuse->exact_weights (rows of several prompts, which were multiplied with exact weights one by one): always.
+  if (M < 2 || (M < 32 && !tiled)) return DP_OK;  // one row, or few on a shape that is not tiled: the CUDA-core kernels
+  // Exact weights: the integer-tile kernel (gemm_q4k_int.cu), whatever the size: one product less per K step than the tiles of
+  // dequantised weights below, 4 to 20 times less error (f32 rows 3.7e-6 to 2.2e-5 -> 9e-7, f16 rows 4e-7), and weights beyond
+  // f16's range.  A whole call, us, what ran before (two products for f16 rows, three for f32 rows; up to 64 f32 rows a kernel of their
+  // own) -> integer tiles, M x N x K:
+  //   f32 rows  2 x 24576 x 4096 66 -> 53, 64 x 24576 x 4096 80 -> 60, 64 x 4096 x 12288 54 -> 43, 384 x 4096 x 12288 131 -> 95, 512 x 24576 x 4096 210 ->
+  //             180, 1024 x 6144 x 4096 115 -> 105, 2048 x 4096 x 4096 155 -> 135, 2048 x 24576 x 4096 763 -> 614, 2048 x 3072 x 1024 45 -> 46
+  //   f16 rows  384 x 6144 x 4096 40 -> 40, 512 x 12288 x 4096 80 -> 70, 512 x 4096 x 12288 221 -> 156, 2048 x 24576 x 4096 502 -> 398
+  // The two products stay for f16 rows where the pass over the rows and a unit's fixed cost weigh more: K up to 1024 with more than half a
+  // wave of the others' 512 x 256 pair tiles (2048 x 3072 x 1024 27 -> 37), and very small weights (32 x 256 x 1024 16 -> 18).
+  // Shapes the others do not tile ran on CUDA cores (1000 x 1000 x 1000: f32 rows 105 -> 30, f16 rows 102 -> 27 us); they still do where
+  // that is over within about 15 us, where the result is f32 and K below 640 (error of the f32 FMAs 4.1e-7 at K = 512, of the integer
+  // tiles 4.8e-7; 5.7e-7 and 4.6e-7 at 1024), and with an alpha that a row's scale might carry out of f32's range.
   if (exact && (c_dtype == DP_F32 || c_dtype == DP_F16)) {
     const long pair_tiles = (long)((M + 511) / 512) * ((N + 255) / 256);
-    const bool few = M <= 256 || (pair_tiles * 2 <= ctx->sm_count / 2 && K <= 8192);
+    const bool few = M <= 256 || pair_tiles * 2 <= ctx->sm_count / 2;
     const float size = fabsf(alpha);
     const bool whole = (double)M * N * K >= (double)(1l << 27) && (K >= 640 || c_dtype == DP_F16) && (size == 0.0f || (size >= 0x1p-60f && size <= 0x1p60f));
-    const bool take = tiled ? (few && (long)N * K >= (1l << 19)) || (fuse && fuse->exact_weights) : whole;
+    const bool take = tiled ? a_dtype == DP_F32 || ((few || K > 1024) && (long)N * K >= (1l << 19)) : whole;
     if (take) {
       DP_TRY(dpk_gemm_q4k_int(ctx, W, A, a_dtype, C, c_dtype, M, N, K, alpha, handled, fuse));
       if (*handled) return DP_OK;
@@ -1000,19 +969,16 @@ static dp_status gemm_q4k_tc_impl(dp_ctx *ctx, const uint8_t *W, const void *A, 
   if (!encode) return DP_OK;
   const __half *a16 = (const __half *)A;
   // The f16 copies of f32 activations live in one scratch allocation of the context, reused in stream order.
-  const __half *a_lo = nullptr;
   const float *scales = nullptr;
   if (a_dtype == DP_F32) {
-    if (mode == 2 && c_dtype != DP_F32) return DP_OK;
+    if (mode == 2) return DP_OK;
     const size_t a_bytes = ((size_t)M * K * 2 + 255) / 256 * 256;
-    DP_TRY(dp_scratch(ctx, &ctx->gemm_scratch, 2 * a_bytes + (size_t)M * 4, "matmul_a_f16"));
+    DP_TRY(dp_scratch(ctx, &ctx->gemm_scratch, a_bytes + (size_t)M * 4, "matmul_a_f16"));
     char *base = (char *)ctx->gemm_scratch->dptr;
     a16 = (const __half *)base;
     if (row_scaled) {
-      if (mode == 2) a_lo = (const __half *)(base + a_bytes);
-      scales = (const float *)(base + 2 * a_bytes);
-      DP_TRY(launch_scale_cast(ctx, (const float *)A, (__half *)base, mode == 2 ? (__half *)(base + a_bytes) : (__half *)nullptr,
-                               (float *)(base + 2 * a_bytes), M, K, fuse ? fuse->norm_w : nullptr, fuse ? fuse->eps : 0.0f));
+      scales = (const float *)(base + a_bytes);
+      DP_TRY(launch_scale_cast(ctx, (const float *)A, (__half *)base, nullptr, (float *)(base + a_bytes), M, K, fuse ? fuse->norm_w : nullptr, fuse ? fuse->eps : 0.0f));
     } else {
       size_t n = (size_t)M * K, grid = (n + 255) / 256;
       if (grid > (size_t)ctx->sm_count * 16) grid = (size_t)ctx->sm_count * 16;
@@ -1021,16 +987,13 @@ static dp_status gemm_q4k_tc_impl(dp_ctx *ctx, const uint8_t *W, const void *A, 
   } else if (a_dtype != DP_F16) {
     return DP_OK;
   }
-  CUtensorMap tm, tm_lo;
+  CUtensorMap tm;
   const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)M};
   const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
   const cuuint32_t box[2] = {BK, 128};
   const cuuint32_t estr[2] = {1, 1};
   CUresult r = encode(&tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void *)a16, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                       CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r == CUDA_SUCCESS)  // (without a lo half the second map is a copy of the first; the kernel then never uses it)
-    r = encode(&tm_lo, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void *)(a_lo ? a_lo : a16), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   dp_status st = DP_OK;
   TcAlpha ta = {alpha, scales, 1, 0};
   // few output tiles (one-SM kernel, f32 output): split K over several CTAs per tile, partial tiles in a scratch
@@ -1076,9 +1039,8 @@ static dp_status gemm_q4k_tc_impl(dp_ctx *ctx, const uint8_t *W, const void *A, 
   if (r != CUDA_SUCCESS) {
     st = dp_fail(ctx, DP_ERR_CUDA, "matmul: cuTensorMapEncodeTiled failed (%d) for A[%d,%d]", (int)r, M, K);
   } else if (c_dtype == DP_F32) {
-    if (mode == 2) st = dispatch_tc<float, 3>(ctx, bn, tm, tm_lo, W, cdst, M, N, K, ta);
-    else if (mode == 3) st = dispatch_tc<float, 2>(ctx, bn, tm, tm_lo, W, cdst, M, N, K, ta);
-    else st = dispatch_tc<float, 1>(ctx, bn, tm, tm_lo, W, cdst, M, N, K, ta);
+    if (mode == 3) st = dispatch_tc<float, 2>(ctx, bn, tm, W, cdst, M, N, K, ta);
+    else st = dispatch_tc<float, 1>(ctx, bn, tm, W, cdst, M, N, K, ta);
     if (st == DP_OK && ta.k_splits > 1) {
       const size_t n = (size_t)M * N;
       size_t grid = (n / 4 + 255) / 256;
@@ -1086,8 +1048,8 @@ static dp_status gemm_q4k_tc_impl(dp_ctx *ctx, const uint8_t *W, const void *A, 
       DP_LAUNCH(ctx, splitk_reduce_kernel, (unsigned)grid, 256, 0, (const float *)cdst, c_final, n, ta.k_splits, red_residual);
     }
   } else if (c_dtype == DP_F16) {
-    if (mode == 3) st = dispatch_tc<__half, 2>(ctx, bn, tm, tm_lo, W, (__half *)C, M, N, K, ta);
-    else st = dispatch_tc<__half, 1>(ctx, bn, tm, tm_lo, W, (__half *)C, M, N, K, ta);
+    if (mode == 3) st = dispatch_tc<__half, 2>(ctx, bn, tm, W, (__half *)C, M, N, K, ta);
+    else st = dispatch_tc<__half, 1>(ctx, bn, tm, W, (__half *)C, M, N, K, ta);
   } else {
     st = dp_fail(ctx, DP_ERR_INVALID, "matmul: unsupported output dtype");
   }
@@ -1108,11 +1070,9 @@ dp_status dpk_gemm_q4k_tc(dp_ctx *ctx, const uint8_t *W, const void *A, dp_dtype
   return gemm_q4k_tc_impl(ctx, W, A, a_dtype, C, c_dtype, M, N, K, alpha, (!f16_weights && a_dtype == DP_F16) ? 3 : 0, handled);
 }
 
-// f32 activations of any range on the tensor-core kernel: every row is scaled into f16 range by a power
-// of two and scaled back in the epilogue.  passes == 1: activations and weights rounded to f16 (11-bit
-// significands, what the reference's tiled f16 prefill kernel computes).  passes == 3: the rounding
-// residues of both are multiplied in as well (three products per K step in one kernel), which gives the
-// f32-exact product to f32 accuracy.
+// f32 activations of any range on the tensor cores: every row is scaled into f16 range by a power of two and scaled back in
+// the epilogue.  passes == 1: activations and weights rounded to f16 (11-bit significands, what the reference's tiled f16
+// prefill kernel computes).  passes == 3: the f32-exact product to f32 accuracy, on integer weight tiles.
 dp_status dpk_gemm_q4k_tc_rowscaled(dp_ctx *ctx, const uint8_t *W, const float *A, float *C, int M, int N, int K, float alpha, int passes,
                                     bool *handled, dpk_tc_fuse *fuse) {
   if (fuse) fuse->silu_done = fuse->residual_done = false;

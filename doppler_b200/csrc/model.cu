@@ -715,12 +715,9 @@ static dp_status q4k_linear(dp_model *m, const uint8_t *W, const float *x, float
   // Several rows run on the tensor-core kernels: each activation row is scaled into f16 range by a power of two (FFN
   // intermediates of a random-init model reach 1e7, far outside f16) and scaled back in the epilogue.  Default: the f32
   // product (the reference's rule for f32 activations, matmul.rules.json:15-22), with integer weight tiles and the rows
-  // as two f16 halves (gemm_q4k_int.cu, gemm_q4k_tc_rows.cu) or, on full waves, in three passes A_hi.W_hi + A_lo.W_hi +
-  // A_hi.W_lo with the f16 rounding residues of activations and weights; rows of several prompts (exact_weights) always with
-  // integer tiles, to the accuracy that the prompts have one by one.  DP_PREFILL_TC=1: one pass, activations and weights
-  // rounded to f16 as in the reference's tiled f16 prefill kernel (fused_matmul_q4_prefill_tiled_f16.wgsl), about 1e-3 of
-  // the output's rms away from the exact product; DP_PREFILL_TC=0 and few rows of shapes those kernels do not take: the
-  // f32-exact CUDA-core kernel.
+  // as two f16 halves (gemm_q4k_int.cu).  DP_PREFILL_TC=1: one pass, activations and weights rounded to f16 as in the
+  // reference's tiled f16 prefill kernel (fused_matmul_q4_prefill_tiled_f16.wgsl), about 1e-3 of the output's rms away from the
+  // exact product; DP_PREFILL_TC=0 and few rows of shapes that are not tiled: the f32-exact CUDA-core kernel.
   static int prefill_tc = -1;
   if (prefill_tc < 0) { const char *e = getenv("DP_PREFILL_TC"); prefill_tc = e ? atoi(e) : 3; }
   bool handled = false;
@@ -869,26 +866,6 @@ static bool tp_exchange_decode_ok(dp_model *m, const DecodeGroup &g) {
   return dpk_attention_uses_tc(m->ctx, ap);
 }
 
-// 2..64 rows on one GPU: a projection on the small-batch tensor-core kernel with the operation that precedes it in
-// the layer (RMSNorm, silu(gate)*up) folded into that kernel's pre-pass and the residual added by its epilogue.
-// *handled stays false when the kernel does not take the shape or a fallback switch is set; the caller then runs
-// the separate kernels.
-static dp_status rows_linear_fused(dp_model *m, const uint8_t *W, const float *A, float *C, int M, int N, int K, const dpk_rows_fuse &fuse,
-                                   bool *handled) {
-  *handled = false;
-  static int on = -1;
-  if (on < 0) {
-    const char *a = getenv("DP_GEMM_TC"), *b = getenv("DP_PREFILL_TC");
-    on = ((a && atoi(a) == 0) || (b && atoi(b) != 3)) ? 0 : 1;
-  }
-  // (up to 32 rows: beyond, one block per row is too little parallelism for the folded operations and the separate
-  // kernels overlap with the projections' tails; measured on the 9B shapes, batch 16: 7.37 -> 6.63 ms per step,
-  // batch 64: 9.18 -> 9.36 ms with everything folded, 9.51 ms with the residual alone; a 1024-token prefill with the
-  // folded pre-pass in front of the prefill GEMM: 39.4 -> 41.5 ms)
-  if (!on || M < 2 || M > 32 || m->cfg.tp_size != 1) return DP_OK;
-  return dpk_gemm_q4k_tc_rows(m->ctx, W, A, DP_F32, C, M, N, K, 1.0f, handled, &fuse);
-}
-
 static dp_status run_layers(dp_model *m, int tokens, bool decode, int seq, int start_pos) {
   if (m->stack) return dp_stack_run_layers(m, tokens, decode, seq, start_pos);
   dp_ctx *ctx = m->ctx;
@@ -911,11 +888,6 @@ static dp_status run_layers(dp_model *m, int tokens, bool decode, int seq, int s
     bool done = false;
     if (single) {
       DP_TRY(dpk_gemv_q4k_tma_fused(ctx, (const uint8_t *)L.qkv->dptr, SRC_RMSNORM, m->h, L.in_norm, c.eps, 0, 0, m->qkv, nqkv, H, nullptr, &done));
-    }
-    if (!done && !single) {
-      dpk_rows_fuse f;
-      f.pre = DPK_ROWS_PRE_RMSNORM; f.norm_w = L.in_norm; f.eps = c.eps;
-      DP_TRY(rows_linear_fused(m, (const uint8_t *)L.qkv->dptr, m->h, m->qkv, tokens, nqkv, H, f, &done));
     }
     if (!done) {
       const bool emit = single && H % QK_K == 0 && H <= 8192 && dpk_gemv_q4k_fast_ok(nqkv, H);
@@ -989,11 +961,6 @@ static dp_status run_layers(dp_model *m, int tokens, bool decode, int seq, int s
       bool fused_o = false;
       if (single)  // one split (short sequences): the projection builds its digits out of the attention's rows itself
         DP_TRY(dpk_gemv_q4k_tma_fused(ctx, (const uint8_t *)L.o->dptr, SRC_PLAIN, m->att, nullptr, 0.0f, 0, 0, o_dst, H, m->qdim, o_res, &fused_o));
-      if (!fused_o && p == 1) {  // h += o_proj(att) in the projection's epilogue
-        dpk_rows_fuse f;
-        f.residual = m->h;
-        DP_TRY(rows_linear_fused(m, (const uint8_t *)L.o->dptr, m->att, m->h, tokens, H, m->qdim, f, &fused_o));
-      }
       if (!fused_o) DP_TRY(q4k_linear(m, (const uint8_t *)L.o->dptr, m->att, o_dst, tokens, H, m->qdim, o_res));
     }
     // ---- exchange after o_proj (tensor parallel) and the post-attention norm ----
@@ -1014,11 +981,6 @@ static dp_status run_layers(dp_model *m, int tokens, bool decode, int seq, int s
       if (!done)
         DP_TRY(dpk_gemv_q4k_tma_fused(ctx, (const uint8_t *)L.gateup->dptr, SRC_RMSNORM, m->h, L.post_norm, c.eps, 0, 0, m->gu, 2 * m->inter, H,
                                       nullptr, &done));
-    }
-    if (!done && !single) {
-      dpk_rows_fuse f;
-      f.pre = DPK_ROWS_PRE_RMSNORM; f.norm_w = L.post_norm; f.eps = c.eps;
-      DP_TRY(rows_linear_fused(m, (const uint8_t *)L.gateup->dptr, m->h, m->gu, tokens, 2 * m->inter, H, f, &done));
     }
     if (!done) {
       const bool emit = single && H % QK_K == 0 && H <= 8192 && dpk_gemv_q4k_fast_ok(2 * m->inter, H);
@@ -1042,11 +1004,6 @@ static dp_status run_layers(dp_model *m, int tokens, bool decode, int seq, int s
       if (!done) return dp_fail(ctx, DP_ERR_STATE, "decode schedule: down_proj cannot read the fused silu(gate) * up vector");
     } else if (single && m->inter % QK_K == 0)
       DP_TRY(dpk_gemv_q4k_tma_fused(ctx, (const uint8_t *)L.down->dptr, SRC_SILU, m->gu, nullptr, 0.0f, 0, 0, d_dst, H, m->inter, d_res, &done));
-    if (!done && !single && p == 1 && !act_rows_ready) {  // silu(gate) * up in the pre-pass, h += down_proj(...) in the epilogue
-      dpk_rows_fuse f;
-      f.pre = DPK_ROWS_PRE_SILU; f.residual = m->h;
-      DP_TRY(rows_linear_fused(m, (const uint8_t *)L.down->dptr, m->gu, m->h, tokens, H, m->inter, f, &done));
-    }
     if (!done) {
       const bool emit = single && m->inter % QK_K == 0 && dpk_gemv_q4k_fast_ok(H, m->inter);
       if (emit) {

@@ -106,6 +106,45 @@ __device__ __forceinline__ void tma_load_2d_2sm(uint32_t dst, const CUtensorMap 
                : "memory");
 }
 
+// ---- issue by a converged warp ----
+// The warps that issue MMAs compete for their scheduler with busy ones, so an MMA must be few instructions.  Its operands live in
+// uniform registers only where the compiler takes the warp for converged and the values for uniform: the warp's number and the
+// tensor-memory address come from one lane (__shfl_sync), so does what decides a wait, the whole warp runs the loop, and the
+// elected lane issues.  Out of a branch that one lane takes an MMA costs 54 cycles on an idle SM and 100 to 200 on a busy one,
+// this way 28 and 33.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+  for (uint32_t i = 0; i < (1u << 20); i++) {
+    if (__shfl_sync(0xffffffffu, mbar_try_wait(bar, parity), 0)) return true;
+    if ((i & 63u) == 63u && __shfl_sync(0xffffffffu, *abort_flag, 0)) return false;
+  }
+  *abort_flag = 1;
+  return false;
+}
+// the four MMAs of a K step of 64, both operands in shared memory; PAIR: of two CTAs
+template <bool PAIR>
+__device__ __forceinline__ void umma_step_warp(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+#define UMMA_STEP(G)                                                                                                                                  \
+  asm volatile("{\n .reg .pred p, q, t;\n .reg .b64 a1, a2, a3, b1, b2, b3;\n setp.ne.b32 p, %4, 0;\n setp.eq.u32 t, 0, 0;\n elect.sync _|q, 0xffffffff;\n" \
+               " add.s64 a1, %1, 2;\n add.s64 a2, %1, 4;\n add.s64 a3, %1, 6;\n add.s64 b1, %2, 2;\n add.s64 b2, %2, 4;\n add.s64 b3, %2, 6;\n"                    \
+               " @q tcgen05.mma.cta_group::" G ".kind::f16 [%0], %1, %2, %3, p;\n @q tcgen05.mma.cta_group::" G ".kind::f16 [%0], a1, b1, %3, t;\n"           \
+               " @q tcgen05.mma.cta_group::" G ".kind::f16 [%0], a2, b2, %3, t;\n @q tcgen05.mma.cta_group::" G ".kind::f16 [%0], a3, b3, %3, t;\n}\n" ::"r"(     \
+                   tmem_d),                                                                                                                            \
+               "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)                                                                                     \
+               : "memory")
+  if constexpr (PAIR) UMMA_STEP("2");
+  else UMMA_STEP("1");
+#undef UMMA_STEP
+}
+template <bool PAIR>
+__device__ __forceinline__ void umma_commit_warp(uint32_t bar) {  // by the same lane; PAIR: on this barrier offset in both CTAs
+  if constexpr (PAIR)
+    asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n @q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n}\n" ::"r"(bar),
+                 "h"((uint16_t)3)
+                 : "memory");
+  else
+    asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(bar) : "memory");
+}
+
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"

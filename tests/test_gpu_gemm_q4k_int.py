@@ -66,6 +66,14 @@ def test_edges(dev, m, n, k, act, out):
     assert np.array_equal(got, run(dev, b, n, k, a, out, alpha=0.5))  # nothing depends on timing
 
 
+@pytest.mark.parametrize("act,out", [("f32", "f32"), ("f16", "f32")])
+@pytest.mark.parametrize("m,n,k", [(2, 2048, 256), (3, 384, 1536), (16, 1024, 768), (17, 512, 1280), (31, 4096, 1792), (32, 256, 2048), (33, 640, 2304), (48, 128, 4352), (64, 1024, 6400),
+                                   (64, 4096, 12288), (600, 2048, 1792), (2000, 1024, 2560)])
+def test_few_rows_and_sum_units(dev, m, n, k, act, out):
+    """From two rows on, every tile width; sum units of one to eight super-blocks, even and odd, in both orders of the products."""
+    test_edges(dev, m, n, k, act, out)
+
+
 @pytest.mark.parametrize("m,n,k", [(1024, 600, 256), (300, 2049, 512), (1024, 600, 640), (300, 2049, 1024), (130, 4095, 2560), (70, 1023, 3100), (768, 513, 12288)])
 def test_untiled_f32_rows_keep_the_accuracy_of_f32_sums(dev, m, n, k):
     """Shapes no tile divides: no further from 64 bits than f32 FMAs in order of K, the general path, are (mean over the outputs)."""

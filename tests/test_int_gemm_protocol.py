@@ -133,3 +133,128 @@ def test_row_scales_are_ordered(sb):
 def test_the_model_sees_a_missing_order():
     with pytest.raises(AssertionError, match="without an order"):
         Pair(4, 24, False).run(random.Random(0))
+
+
+# ---- two sets of builders, several accumulators ----
+BARS, SCALES2 = 16, 8
+
+
+class PairOfSets(Pair):
+    """Four groups a unit; builders of even and of odd units, each unit's groups by two of its set's warps; `accs` accumulators
+    handed back by the drains; packed blocks in a ring of `sp` stages that completes out of order."""
+
+    def __init__(self, sb, accs, sp, units):
+        self.sb, self.accs, self.sp, self.units, self.own = sb, accs, sp, units, True
+        self.full = [Barrier(0, 2) for _ in range(BARS)]  # one warp of either CTA
+        self.done = [[Barrier(c, 1) for _ in range(BARS)] for c in (0, 1)]
+        self.scaled = [[Barrier(c, 1) for _ in range(SCALES2)] for c in (0, 1)]
+        self.packed = [[Barrier(c, 1) for _ in range(sp)] for c in (0, 1)]
+        self.free = [[Barrier(c, 2) for _ in range(sp)] for c in (0, 1)]
+        self.empty = [Barrier(0, 2) for _ in range(accs)]
+        self.clocks, self.written, self.read = {}, {}, {}
+        self.landing = {0: [], 1: []}
+        self.stage = {0: {}, 1: {}}
+
+    def packer(self, cta):
+        me = (cta, "packer")
+        for n in range(self.units):
+            if n >= self.sp:
+                yield from self.wait(me, self.free[cta][n % self.sp], n // self.sp - 1)
+            self.landing[cta].append(n)
+            yield
+
+    def memory(self, cta, rng):
+        """copies land in any order"""
+        for _ in range(self.units):
+            while not self.landing[cta]:
+                yield
+            n = self.landing[cta].pop(rng.randrange(len(self.landing[cta])))
+            self.stage[cta][n % self.sp] = n
+            self.packed[cta][n % self.sp].arrive(None)
+            yield
+
+    def builder(self, cta, odd, half):
+        me = (cta, "builder", odd, half)
+        for n in range(odd, self.units, 2):
+            yield from self.wait(me, self.packed[cta][n % self.sp], n // self.sp)
+            assert self.stage[cta].get(n % self.sp) == n, "another unit's packed block"
+            if half == 0:
+                assert n < SCALES2 or (cta, n - SCALES2) in self.read, "slot overwritten before it is read"
+                self.written[cta, n % SCALES2] = (n, me, self.tick(me)[me])
+            yield
+            for h in (0, 1):
+                g = 4 * n + 2 * half + h
+                if g >= self.sb:
+                    yield from self.wait(me, self.done[cta][(g - self.sb) % BARS], (g - self.sb) // BARS)
+                    assert g - self.sb in self.finished, "a group of weights overwritten before it is multiplied"
+                if h == 1:
+                    self.arrive(me, self.free[cta][n % self.sp])
+                    if half == 0:
+                        self.arrive(me, self.scaled[cta][n % SCALES2])
+                self.built.setdefault(g, set()).add(cta)
+                self.arrive(me, self.full[g % BARS])
+                yield
+
+    def mma(self, mine):
+        me = (0, "mma", mine)
+        for n in range(mine, self.units, 2):
+            if n >= self.accs:
+                yield from self.wait(me, self.empty[n % self.accs], n // self.accs - 1)
+                assert all((c, n - self.accs) in self.read for c in (0, 1)), "an accumulator overwritten before it is read"
+            for g in range(4 * n, 4 * n + 4):
+                yield from self.wait(me, self.full[g % BARS], g // BARS)
+                assert self.built[g] == {0, 1}, "multiplied before it is built"
+                self.commits.append(g)
+                yield
+
+    def tensor_core(self):
+        for _ in range(4 * self.units):
+            while not self.commits:
+                yield
+            g = self.commits.pop(0)
+            self.finished.add(g)
+            for c in (0, 1):
+                self.done[c][g % BARS].arrive(None)
+            yield
+
+    def drain(self, cta):
+        me = (cta, "drain")
+        for n in range(self.units):
+            yield from self.wait(me, self.scaled[cta][n % SCALES2], n // SCALES2)
+            yield from self.wait(me, self.done[cta][(4 * n + 3) % BARS], (4 * n + 3) // BARS)
+            assert 4 * n + 3 in self.finished
+            unit, writer, at = self.written[cta, n % SCALES2]
+            assert unit == n
+            assert self.tick(me).get(writer, 0) >= at, "row scale read without an order after its write"
+            yield
+            self.read[cta, n] = True
+            self.arrive(me, self.empty[n % self.accs])
+
+    def run(self, rng):
+        self.commits, self.finished, self.built = [], set(), {}
+        roles = [self.builder(c, o, h) for c in (0, 1) for o in (0, 1) for h in (0, 1)]
+        roles += [self.packer(0), self.packer(1), self.memory(0, rng), self.memory(1, rng), self.mma(0), self.mma(1), self.tensor_core(), self.drain(0), self.drain(1)]
+        weight = [10.0 ** rng.uniform(-2, 0) for _ in roles]
+        for _ in range(600000):
+            if not roles:
+                return
+            i = rng.choices(range(len(roles)), weight)[0]
+            try:
+                next(roles[i])
+            except StopIteration:
+                del roles[i], weight[i]
+        raise AssertionError("a wait hangs")
+
+
+@pytest.mark.parametrize("sb,accs", [(8, 4), (7, 3), (8, 2), (6, 2), (4, 2)])
+@pytest.mark.parametrize("sp", [2, 4])
+def test_sets_of_builders(sb, accs, sp):
+    for seed in range(25):
+        PairOfSets(sb, accs, sp, 41).run(random.Random(seed))
+
+
+def test_an_odd_ring_of_packed_blocks_is_caught():
+    """With three stages a set of builders takes a stage's barrier for that of its own unit while the other set's copy is under way."""
+    with pytest.raises(AssertionError):
+        for seed in range(200):
+            PairOfSets(8, 4, 3, 41).run(random.Random(seed))
