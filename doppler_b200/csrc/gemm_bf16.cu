@@ -7,6 +7,12 @@
 // TMEM, four epilogue warps) with two accumulators in tensor memory, so the next tile's products run under this
 // tile's stores.  K tails and rows beyond M or N are zero filled by TMA.  Every wait is bounded.
 //
+// Bound by what the SMs fetch from L2 (a tile of 128 x 256 takes 48 KB per K step of 512 cycles of MMAs): with PAIR a
+// cluster of two CTAs owns 256 features (cta_group::2) and each brings its 128 weight rows and half of the activation rows,
+// 32 KB.  The products of a prompt of 2048 tokens (the ten of four 4096-wide Fenorax layers): 1777 us with the MMAs out of a
+// branch of one lane, 1575 from a converged warp (umma.cuh), 1452 in pairs; of 1500 tokens (22 of four Virolorn layers) 1753, 1483, 1436;
+// of 40 tokens at width 1024 129 -> 97.
+//
 // dpk_gemm_f16_tc: the same kernel with f16 operands and an f16 result.
 //
 // Optional decay: exp(-rate softplus(c + bias)) of every product is stored instead of the product.
@@ -53,6 +59,7 @@ __device__ __forceinline__ uint32_t idesc_16(int M, int N, bool f16) {  // D = f
   return (1u << 4) | (f16 ? 0u : (1u << 7) | (1u << 10)) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
+template <bool PAIR>
 __global__ void __launch_bounds__(BT_THREADS, 1) gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_a,
                                                                      const TcArgs a, int *__restrict__ err) {
   extern __shared__ uint8_t bt_raw[];
@@ -61,9 +68,11 @@ __global__ void __launch_bounds__(BT_THREADS, 1) gemm_bf16_tc_kernel(const __gri
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_word;
   volatile int *abort_flag = &abort_word;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int S = a.stages;
-  const uint32_t stage_bytes = BT_W_TILE + (uint32_t)a.bn * 128u;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
+  const int owner = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, owners = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
+  const int S = a.stages, rows = PAIR ? a.bn / 2 : a.bn, features = PAIR ? 256 : 128;  // activation rows of this CTA, features of a tile
+  const uint32_t stage_bytes = BT_W_TILE + (uint32_t)rows * 128u;
   const uint32_t bar0 = smem_u32(bars);
   auto full = [&](int s) { return bar0 + 8u * (uint32_t)s; };
   auto empty = [&](int s) { return bar0 + 8u * (uint32_t)(BT_MAX_STAGES + s); };
@@ -71,72 +80,87 @@ __global__ void __launch_bounds__(BT_THREADS, 1) gemm_bf16_tc_kernel(const __gri
   auto acc_empty = [&](int b) { return bar0 + 8u * (uint32_t)(2 * BT_MAX_STAGES + 2 + b); };
   const int tiles = a.tiles_n * a.tiles_m, ksteps = (a.K + BK - 1) / BK;
 
-  pdl_launch();
+  if constexpr (!PAIR) pdl_launch();  // (a launch of clusters is not made programmatic)
   pdl_wait();
   if (tid == 0) {
     for (int s = 0; s < S; s++) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
-    for (int b = 0; b < 2; b++) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 4); }
+    for (int b = 0; b < 2; b++) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), PAIR ? 8 : 4); }
     abort_word = 0;
     mbar_fence_init();
   }
   if (warp == 2) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"((uint32_t)a.tmem_cols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if constexpr (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"((uint32_t)a.tmem_cols) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"((uint32_t)a.tmem_cols) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if constexpr (PAIR) cluster_sync_all();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(&tmem_slot);
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t *>(&tmem_slot), 0);
 
   if (warp == 0) {
     if (lane == 0) {
-      uint32_t it = 0;
+      uint32_t it = 0, round = 0;
+      int s = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-        const int n0 = (tile / a.tiles_m) * 128, m0 = (tile % a.tiles_m) * a.bn;
+      for (int tile = owner; tile < tiles && ok; tile += owners) {
+        const int n0 = (tile / a.tiles_m) * features + (int)rank * 128, m0 = (tile % a.tiles_m) * a.bn + (int)rank * rows;
         for (int k = 0; k < ksteps; k++, it++) {
-          const int s = (int)(it % (uint32_t)S);
-          if (it >= (uint32_t)S && !mbar_wait_bounded(empty(s), ((it / (uint32_t)S) - 1u) & 1u, abort_flag)) { ok = false; break; }
-          mbar_expect_tx(full(s), stage_bytes);
+          if (round > 0 && !mbar_wait_bounded(empty(s), (round - 1u) & 1u, abort_flag)) { ok = false; break; }
           const uint32_t dst = smem_u32(smem) + (uint32_t)s * stage_bytes;
-          tma_load_2d(dst, &tmap_w, k * BK, n0, full(s));
-          tma_load_2d(dst + BT_W_TILE, &tmap_a, k * BK, m0, full(s));
+          if constexpr (PAIR) {  // both CTAs' bytes are counted on CTA 0's barrier
+            if (rank == 0) mbar_expect_tx(full(s), 2u * stage_bytes);
+            const uint32_t there = mapa_shared(full(s), 0u);
+            tma_load_2d_2sm(dst, &tmap_w, k * BK, n0, there);
+            tma_load_2d_2sm(dst + BT_W_TILE, &tmap_a, k * BK, m0, there);
+          } else {
+            mbar_expect_tx(full(s), stage_bytes);
+            tma_load_2d(dst, &tmap_w, k * BK, n0, full(s));
+            tma_load_2d(dst + BT_W_TILE, &tmap_a, k * BK, m0, full(s));
+          }
+          if (++s == S) { s = 0; round++; }
         }
       }
       // no copy may still be in flight when the CTA ends, also where a wait gave up
       const uint32_t held = it < (uint32_t)S ? it : (uint32_t)S;
-      for (uint32_t i = it - held; i < it; i++)
+      for (uint32_t i = it - held; i < it && rank == 0; i++)
         for (uint32_t poll = 0; poll < (1u << 20) && !mbar_try_wait(full((int)(i % (uint32_t)S)), (i / (uint32_t)S) & 1u); poll++) {}
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = idesc_16(128, a.bn, a.C16 != nullptr);
-      uint32_t it = 0, n = 0;
+    if (rank == 0) {
+      const uint32_t idesc = idesc_16(features, a.bn, a.C16 != nullptr);
+      const uint64_t first = umma_desc_sw128(smem_u32(smem));
+      uint32_t n = 0, round = 0;
+      int s = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, n++) {
+      for (int tile = owner; tile < tiles && ok; tile += owners, n++) {
         const int b = (int)(n & 1u);
-        if (n >= 2 && !mbar_wait_bounded(acc_empty(b), ((n >> 1) - 1u) & 1u, abort_flag)) break;
+        if (n >= 2 && !mbar_wait_warp(acc_empty(b), ((n >> 1) - 1u) & 1u, abort_flag)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t acc = tmem + (uint32_t)(b * a.bn);
-        for (int k = 0; k < ksteps; k++, it++) {
-          const int s = (int)(it % (uint32_t)S);
-          if (!mbar_wait_bounded(full(s), (it / (uint32_t)S) & 1u, abort_flag)) { ok = false; break; }
+        for (int k = 0; k < ksteps; k++) {
+          if (!mbar_wait_warp(full(s), round & 1u, abort_flag)) { ok = false; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t w_addr = smem_u32(smem) + (uint32_t)s * stage_bytes, x_addr = w_addr + BT_W_TILE;
-#pragma unroll
-          for (int k16 = 0; k16 < BK / 16; k16++)
-            umma_f16(acc, umma_desc_sw128(w_addr + (uint32_t)k16 * 32u), umma_desc_sw128(x_addr + (uint32_t)k16 * 32u), idesc, (k > 0 || k16 > 0) ? 1u : 0u);
-          umma_commit(empty(s));
+          const uint64_t w = first + (uint64_t)((uint32_t)s * (stage_bytes >> 4));
+          umma_step_warp<PAIR>(acc, w, w + (BT_W_TILE >> 4), idesc, k);
+          umma_commit_warp<PAIR>(empty(s));
+          if (++s == S) { s = 0; round++; }
         }
-        if (ok) umma_commit(acc_full(b));
+        if (ok) umma_commit_warp<PAIR>(acc_full(b));
       }
     }
   } else if (warp >= 4) {
     const int quad = warp & 3;
+    const uint32_t acc_empty0 = PAIR ? mapa_shared(acc_empty(0), 0u) : 0u;
     uint32_t n = 0;
-    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, n++) {
+    for (int tile = owner; tile < tiles; tile += owners, n++) {
       const int b = (int)(n & 1u);
-      const int n0 = (tile / a.tiles_m) * 128, m0 = (tile % a.tiles_m) * a.bn;
+      const int n0 = (tile / a.tiles_m) * features + (int)rank * 128, m0 = (tile % a.tiles_m) * a.bn;
       const bool ready = mbar_wait_bounded(acc_full(b), (n >> 1) & 1u, abort_flag);
       if (!__all_sync(0xffffffffu, ready)) break;  // tcgen05.ld is warp-wide: together or not at all
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -180,12 +204,20 @@ __global__ void __launch_bounds__(BT_THREADS, 1) gemm_bf16_tc_kernel(const __gri
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) mbar_arrive(acc_empty(b));
+      if (lane == 0) {
+        if constexpr (PAIR) asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(acc_empty0 + 8u * (uint32_t)b) : "memory");
+        else mbar_arrive(acc_empty(b));
+      }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 2) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)a.tmem_cols) : "memory");
+  if constexpr (PAIR) {
+    cluster_sync_all();  // neither CTA frees tensor memory or leaves while the peer still uses the pair's resources
+    if (warp == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)a.tmem_cols) : "memory");
+  } else {
+    if (warp == 2) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)a.tmem_cols) : "memory");
+  }
   if (abort_word && tid == 0) atomicExch(err, 2);
 }
 
@@ -195,17 +227,25 @@ GluArgs glu_args(const GluOut *g) {
   return a;
 }
 
-// activation rows per tile: the width with the least (waves x (products of a tile + its fixed cost))
-int pick_rows(dp_ctx *ctx, int M, int tiles_n) {
-  int best = 16;
+// Activation rows per tile, and whether two SMs share one: the least estimated time in cycles.  A K step takes its MMAs (two
+// cycles per activation row) or what it fetches from L2, at some 44 bytes a cycle and SM.
+struct TilePick {
+  int bn;
+  bool pair;
+};
+TilePick pick_tile(dp_ctx *ctx, int M, int N, int ksteps, bool may_pair) {
+  TilePick best = {16, false};
   double best_cost = -1.0;
-  for (int bn = 16; bn <= 256; bn += 16) {
-    const long tiles = (long)tiles_n * ((M + bn - 1) / bn);
-    const long waves = (tiles + ctx->sm_count - 1) / ctx->sm_count;
-    // tiles narrower than 128 rows are paced by the weight operand's shared-memory reads, not by the products
-    const double cost = (double)waves * ((bn < 128 ? 128 : bn) + 16);
-    if (best_cost < 0 || cost < best_cost) { best = bn; best_cost = cost; }
-  }
+  for (int pair = 0; pair <= (may_pair ? 1 : 0); pair++)
+    for (int bn = 16; bn <= 256; bn += 16) {
+      const long tiles = (long)((N + (pair ? 255 : 127)) / (pair ? 256 : 128)) * ((M + bn - 1) / bn), owners = pair ? ctx->sm_count / 2 : ctx->sm_count;
+      const long waves = (tiles + owners - 1) / owners;
+      const double fetch = (16384.0 + 128.0 * (pair ? bn / 2 : bn)) / 44.0, step = fetch > 2.0 * bn ? fetch : 2.0 * bn;
+      // (a pair's advantage counts by less than its bytes: it gains 8 % on the largest products, and loses 3 to 8 % on those of a few
+      // microseconds, 301 -> 311 us for 1500 tokens at width 1024)
+      const double cost = ((double)waves * (ksteps * step + 1500.0) + 12.0 * bn) * (pair ? 1.3 : 1.0);
+      if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = {bn, pair != 0}; }
+    }
   return best;
 }
 
@@ -215,10 +255,13 @@ dp_status launch_tc(dp_ctx *ctx, const void *W, int w_stride, const void *A, int
   DP_CHECK(ctx, w_stride % 8 == 0 && a_stride % 8 == 0 && K <= w_stride && K <= a_stride && M > 0 && N > 0 && K > 0, "gemm (bf16): bad shape or stride");
   EncodeTiledFn encode = get_encode();
   if (!encode) return dp_fail(ctx, DP_ERR_CUDA, "gemm (bf16): cuTensorMapEncodeTiled is not available");
-  a.tiles_n = (N + 127) / 128;
-  a.bn = pick_rows(ctx, M, a.tiles_n);
+  // (in a decode step's graph kernels launch their dependents early; those keep to launches without clusters)
+  const TilePick pick = pick_tile(ctx, M, N, (K + BK - 1) / BK, !ctx->pdl && ctx->sm_count >= 2);
+  a.bn = pick.bn;
+  a.tiles_n = (N + (pick.pair ? 255 : 127)) / (pick.pair ? 256 : 128);
   a.tiles_m = (M + a.bn - 1) / a.bn;
-  const uint32_t stage_bytes = BT_W_TILE + (uint32_t)a.bn * 128u;
+  const int rows = pick.pair ? a.bn / 2 : a.bn;
+  const uint32_t stage_bytes = BT_W_TILE + (uint32_t)rows * 128u;
   const size_t budget = ctx->smem_optin - 2048;
   int stages = (int)((budget - 1024) / stage_bytes);
   if (stages > BT_MAX_STAGES) stages = BT_MAX_STAGES;
@@ -230,20 +273,45 @@ dp_status launch_tc(dp_ctx *ctx, const void *W, int w_stride, const void *A, int
   const cuuint32_t estr[2] = {1, 1};
   const cuuint64_t wd[2] = {(cuuint64_t)K, (cuuint64_t)N}, ad[2] = {(cuuint64_t)K, (cuuint64_t)M};
   const cuuint64_t ws[1] = {(cuuint64_t)w_stride * 2}, as[1] = {(cuuint64_t)a_stride * 2};
-  const cuuint32_t wb[2] = {BK, 128}, ab[2] = {BK, (cuuint32_t)a.bn};
+  const cuuint32_t wb[2] = {BK, 128}, ab[2] = {BK, (cuuint32_t)rows};
   CUresult r = encode(&tw, type, 2, (void *)W, wd, ws, wb, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r == CUDA_SUCCESS)
     r = encode(&ta, type, 2, (void *)A, ad, as, ab, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return dp_fail(ctx, DP_ERR_CUDA, "gemm (bf16): cuTensorMapEncodeTiled failed (%d) for [%d,%d] x [%d,%d]", (int)r, M, K, N, K);
+  const size_t smem = (size_t)stages * stage_bytes + 1024;
+  const int tiles = a.tiles_n * a.tiles_m;
+  if (!pick.pair) {
+    static dp_per_device_once attr;
+    if (attr.pending(ctx->device)) {
+      DP_CUDA(ctx, cudaFuncSetAttribute(gemm_bf16_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
+      attr.done(ctx->device);
+    }
+    DP_LAUNCH(ctx, gemm_bf16_tc_kernel<false>, tiles < ctx->sm_count ? tiles : ctx->sm_count, BT_THREADS, smem, tw, ta, a, ctx->dev_status);
+    return DP_OK;
+  }
   static dp_per_device_once attr;
   if (attr.pending(ctx->device)) {
-    DP_CUDA(ctx, cudaFuncSetAttribute(gemm_bf16_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
+    DP_CUDA(ctx, cudaFuncSetAttribute(gemm_bf16_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
     attr.done(ctx->device);
   }
-  const int tiles = a.tiles_n * a.tiles_m, grid = tiles < ctx->sm_count ? tiles : ctx->sm_count;
-  DP_LAUNCH(ctx, gemm_bf16_tc_kernel, grid, BT_THREADS, (size_t)stages * stage_bytes + 1024, tw, ta, a, ctx->dev_status);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * (unsigned)(tiles < ctx->sm_count / 2 ? tiles : ctx->sm_count / 2));
+  cfg.blockDim = dim3(BT_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute cluster[1];
+  cluster[0].id = cudaLaunchAttributeClusterDimension;
+  cluster[0].val.clusterDim.x = 2;
+  cluster[0].val.clusterDim.y = 1;
+  cluster[0].val.clusterDim.z = 1;
+  cfg.attrs = cluster;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_bf16_tc_kernel<true>, tw, ta, a, ctx->dev_status);
+  ctx->launches++;
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e != cudaSuccess) return dp_fail(ctx, DP_ERR_CUDA, "launch of gemm_bf16_tc_kernel failed: %s", cudaGetErrorString(e));
   return DP_OK;
 }
 
