@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) gemm_bf16w_f32_tc_kernel(const 
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_word;
   volatile int *abort_flag = &abort_word;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const uint32_t S = (uint32_t)a.stages, x_tile = (uint32_t)a.bn * 128u, stage_bytes = FX_W_TILE + 3u * x_tile;
   const uint32_t bar0 = smem_u32(bars);
   auto full = [&](uint32_t s) { return bar0 + 8u * s; };                       // stages <= FX_BUFS
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) gemm_bf16w_f32_tc_kernel(const 
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(&tmem_slot);
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t *>(&tmem_slot), 0);
 
   if (warp == 0) {
     if (lane == 0) {
@@ -119,11 +119,9 @@ __global__ void __launch_bounds__(FX_THREADS, 1) gemm_bf16w_f32_tc_kernel(const 
           mbar_expect_tx(full(s), stage_bytes);
           const uint32_t dst = smem_u32(smem) + s * stage_bytes;
           tma_load_2d(dst, &tmap_w, k * BK, n0, full(s));
-          for (int t = 0; t < 3; t++)
-            asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
-                             dst + FX_W_TILE + (uint32_t)t * x_tile),
-                         "l"(&tmap_a), "r"(k * BK), "r"(m0), "r"(t), "r"(full(s))
-                         : "memory");
+          asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst + FX_W_TILE),
+                       "l"(&tmap_a), "r"(k * BK), "r"(m0), "r"(0), "r"(full(s))  // all three terms
+                       : "memory");
         }
       }
       // no copy may still be in flight when the CTA ends, also where a wait gave up
@@ -132,26 +130,23 @@ __global__ void __launch_bounds__(FX_THREADS, 1) gemm_bf16w_f32_tc_kernel(const 
         for (uint32_t poll = 0; poll < (1u << 20) && !mbar_try_wait(full(i % S), (i / S) & 1u); poll++) {}
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(a.bn >> 3) << 17) | (128u >> 4 << 24);  // D = f32, A = B = bf16, K-major
-      uint32_t it = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-        for (int k = 0; k < ksteps; k++, it++) {
-          const uint32_t s = it % S, b = it % FX_BUFS;
-          if (it >= FX_BUFS && !mbar_wait_bounded(drained(b), ((it / FX_BUFS) - 1u) & 1u, abort_flag)) { ok = false; break; }
-          if (!mbar_wait_bounded(full(s), (it / S) & 1u, abort_flag)) { ok = false; break; }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t w_addr = smem_u32(smem) + s * stage_bytes, acc = tmem + b * (uint32_t)a.bn;
-#pragma unroll
-          for (int t = 2; t >= 0; t--) {
-            const uint32_t x_addr = w_addr + FX_W_TILE + (uint32_t)t * x_tile;
-#pragma unroll
-            for (int k16 = 0; k16 < BK / 16; k16++)
-              umma_f16(acc, umma_desc_sw128(w_addr + (uint32_t)k16 * 32u), umma_desc_sw128(x_addr + (uint32_t)k16 * 32u), idesc, (t < 2 || k16 > 0) ? 1u : 0u);
-          }
-          umma_commit(done(b));  // the stage is free, the step's sums are complete
-        }
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(a.bn >> 3) << 17) | (128u >> 4 << 24);  // D = f32, A = B = bf16, K-major
+    const uint64_t first = umma_desc_sw128(smem_u32(smem));
+    uint32_t it = 0, s = 0, round = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+      for (int k = 0; k < ksteps; k++, it++) {
+        const uint32_t b = it % FX_BUFS;
+        if (it >= FX_BUFS && !mbar_wait_warp(drained(b), ((it / FX_BUFS) - 1u) & 1u, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(full(s), round & 1u, abort_flag)) { ok = false; break; }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint64_t w = first + (uint64_t)(s * (stage_bytes >> 4)), x = w + (FX_W_TILE >> 4);
+        const uint32_t acc = tmem + b * (uint32_t)a.bn;
+        umma_step_warp<false>(acc, w, x + 2u * (x_tile >> 4), idesc, 0u);
+        umma_step_warp<false>(acc, w, x + (x_tile >> 4), idesc, 1u);
+        umma_step_warp<false>(acc, w, x, idesc, 1u);
+        umma_commit_warp<false>(done(b));  // the stage is free, the step's sums are complete
+        if (++s == S) { s = 0; round++; }
       }
     }
   } else if (warp >= 4) {
@@ -250,7 +245,7 @@ dp_status dpk_gemm_bf16w_f32(dp_ctx *ctx, const __nv_bfloat16 *W, int w_stride, 
   const cuuint32_t estr[3] = {1, 1, 1};
   const cuuint64_t wd[2] = {(cuuint64_t)K, (cuuint64_t)N}, ad[3] = {(cuuint64_t)K, (cuuint64_t)M, 3};
   const cuuint64_t ws[1] = {(cuuint64_t)w_stride * 2}, as[2] = {(cuuint64_t)kp * 2, (cuuint64_t)plane * 2};
-  const cuuint32_t wb[2] = {BK, 128}, ab[3] = {BK, (cuuint32_t)a.bn, 1};
+  const cuuint32_t wb[2] = {BK, 128}, ab[3] = {BK, (cuuint32_t)a.bn, 3};
   CUresult r = encode(&tw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void *)W, wd, ws, wb, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r == CUDA_SUCCESS)
