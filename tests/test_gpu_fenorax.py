@@ -260,6 +260,8 @@ LARGE = {
     "ssm 32 x 64": config([mamba(heads=90, vdim=64, state=32, groups=2, norm_groups=2)], width=128),
     "ssm 64 x 64": config([mamba(heads=90, vdim=64, state=64, groups=2, norm_groups=2)], width=128),
     "ssm 128 x 32": config([mamba(heads=48, vdim=64, state=128, groups=2, norm_groups=2)], width=128),
+    # products in tiles of two SMs (their 16400 features and 327 rows end inside a tile)
+    "two SMs a tile": config([attention(heads=2, kv_heads=1, dim=32, vdim=32, chunk=50, mlp={"kind": "dense", "ff": 8200, "limit": 1.0})], width=1024),
     # products whose rows and columns do not fill a tile
     "wide": config([attention(heads=4, kv_heads=4, dim=72, vdim=56, mlp={"kind": "dense", "ff": 700, "limit": 1.0})], width=264, groups=3, vocab=600),
 }
