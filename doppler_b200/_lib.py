@@ -179,6 +179,7 @@ SIGNATURES = {
     "dp_model_prefill_many": (_i, [_vp, _i, _vp, _vp, _vp, _vp]),
     "dp_model_prefill": (_i, [_vp, _i, _vp, _i, C.POINTER(C.c_int32)]),
     "dp_model_decode": (_i, [_vp, _i, _vp, _i, _vp]),
+    "dp_model_advance": (_i, [_vp, C.c_int32]),
     "dp_model_extend": (_i, [_vp, _i, _vp, _i, _vp, _i, _vp]),
     "dp_model_release": (_i, [_vp, _i]),
     "dp_model_create_stack": (_i, [_vp, C.POINTER(StackCfg), C.POINTER(LayerCfg), C.POINTER(_vp)]),

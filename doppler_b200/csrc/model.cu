@@ -135,6 +135,15 @@ __global__ void advance_kernel(int *pos, int *kvlen, const int *tok, int *step, 
 }
 
 
+// after a step of one sequence without logits
+__global__ void step_on_kernel(int *pos, int *kvlen, unsigned *ticket) {
+  pdl_launch();
+  pdl_wait();
+  *pos += 1;
+  *kvlen += 1;
+  *ticket += 1u;
+}
+
 // The end of a decode step of one sequence in one launch: greedy token (ties to the lower index, as sample.wgsl:311-408),
 // token record, position.  Three dependent launches of a few hundred threads each (two argmax phases, advance_kernel) were
 // 8 us of every step; the block that finishes last does what the second and third did.  `arrived` is 0 before and after.
@@ -1090,6 +1099,13 @@ static dp_status wanted_rows(dp_model *m, const char *op, const int32_t *want, i
   return DP_OK;
 }
 
+// Before a pass overwrites the hidden row of a step without logits: its logits, unless the pass has logits of its own
+static dp_status settle_head(dp_model *m, bool replaced) {
+  if (!m->head_pending) return DP_OK;
+  m->head_pending = false;
+  return replaced ? DP_OK : run_logits(m, m->h, 1);
+}
+
 // One portion of a sequence: `n` tokens that follow what the sequence holds already, in blocks of at most m->T rows.
 // want: ascending places among the n tokens whose logits are copied to `logits` [n_want][vocabulary share].
 // next_token (optional): the greedy token after the last one.
@@ -1104,6 +1120,7 @@ static dp_status run_portion(dp_model *m, const char *op, int seq, const int32_t
   for (int i = 0; i < n_want; i++)
     DP_CHECK(ctx, want[i] >= 0 && want[i] < n && (i == 0 || want[i] > want[i - 1]), "%s: wanted place %d is not an ascending place among the %d tokens", op, want[i], n);
   if (m->stack) DP_TRY(dp_stack_ready(m));
+  DP_TRY(settle_head(m, n_want > 0 || next_token));
   dp_buf ids = nullptr;
   DP_TRY(dp_buf_acquire(ctx, (size_t)m->T * 4, "prefill_token_ids", &ids));
   dp_status st = DP_OK;
@@ -1182,6 +1199,7 @@ static dp_status run_packed(dp_model *m, const int32_t *seqs, const int32_t *con
   DP_TRY(dp_buf_acquire(ctx, host.size() * 4, "packed_rows", &buf));
   const int *dev = (const int *)buf->dptr;
   const PackedRows packed = {dev + rows, dev + 2 * rows, (const int4 *)(dev + spans_at), n, longest};
+  m->head_pending = false;  // its logits are replaced
   auto run = [&]() -> dp_status {
     DP_TRY(dp_buf_upload(ctx, buf, host.data(), 0, host.size() * 4));
     DP_TRY(embed_rows(m, dev, rows, false));
@@ -1294,9 +1312,10 @@ extern "C" dp_status dp_model_decode(dp_model *m, int batch, const int32_t *firs
     DP_CHECK(ctx, m->seq_len[b] + steps <= c.max_seq, "decode: sequence %d would exceed max_seq %d", b, c.max_seq);
   }
   if (m->stack) DP_TRY(dp_stack_ready(m));
+  m->head_pending = false;  // its logits are replaced
   if (m->out_tokens_cap < steps * batch) {
     if (m->out_tokens) { dp_buf_release(ctx, m->out_tokens); m->out_tokens = nullptr; }
-    for (int i = 0; i < 2; i++) if (m->graph[i]) { dp_graph_destroy(m->graph[i]); m->graph[i] = nullptr; }
+    if (m->graph[0]) { dp_graph_destroy(m->graph[0]); m->graph[0] = nullptr; }
     if (m->pin_out) { cudaFreeHost(m->pin_out); m->pin_out = nullptr; }
     m->out_tokens_cap = 0;
     DP_TRY(dp_buf_acquire(ctx, (size_t)steps * batch * 4, "decode_out_tokens", &m->out_tokens));
@@ -1340,9 +1359,57 @@ extern "C" dp_status dp_model_decode(dp_model *m, int batch, const int32_t *firs
   return DP_OK;
 }
 
+// One token of sequence 0 whose logits nobody asked for: a decode step without the table's product and the pick (65 MB of 126
+// that a step of an eight-layer Fenorax decoder of width 1024 reads, 262 of 1390 MB of a four-layer Virolorn of width 4096).
+extern "C" dp_status dp_model_advance(dp_model *m, int32_t token) {
+  if (!m) return DP_ERR_INVALID;
+  dp_ctx *ctx = m->ctx;
+  const dp_model_cfg &c = m->cfg;
+  DP_CHECK(ctx, c.tp_size == 1, "advance: a sharded model decodes");
+  DP_CHECK(ctx, token >= 0 && token < c.vocab, "advance: token id %d outside the vocabulary", token);
+  DP_CHECK(ctx, m->seq_len[0] + 1 <= c.max_seq, "advance: sequence 0 would exceed max_seq %d", c.max_seq);
+  if (m->stack) DP_TRY(dp_stack_ready(m));
+  if (!m->pin_state) DP_CUDA(ctx, cudaMallocHost(&m->pin_state, 4096 + 16));
+  int *st = m->pin_state;
+  memset(st, 0, 4096);
+  st[0] = m->seq_len[0]; st[256] = m->seq_len[0] + 1; st[512] = token;
+  DP_CUDA(ctx, cudaMemcpyAsync(m->state->dptr, st, 4096, cudaMemcpyHostToDevice, ctx->stream));
+  if (!m->graph[1]) {
+    dp_recorder *rec = nullptr;
+    DP_TRY(dp_recorder_begin(ctx, "step_without_logits", 1, &rec));
+    ctx->pdl = getenv("DP_PDL") ? atoi(getenv("DP_PDL")) != 0 : true;
+    m->recording_decode = true;
+    dp_status s = embed_rows(m, m->d_tok, 1, true);
+    if (s == DP_OK) s = run_layers(m, 1, true, 0, 0);
+    if (s == DP_OK && m->stack) s = dp_stack_hidden(m);
+    if (s == DP_OK) s = [&]() -> dp_status {
+        DP_LAUNCH(ctx, step_on_kernel, 1, 1, 0, m->d_pos, m->d_kvlen, m->d_ticket);
+        return DP_OK;
+      }();
+    m->recording_decode = false;
+    ctx->pdl = false;
+    if (s != DP_OK) { std::string keep = ctx->err; dp_recorder_abort(rec); ctx->err = keep; return s; }
+    DP_TRY(dp_recorder_finish_graph(rec, &m->graph[1]));
+  }
+  DP_CUDA(ctx, cudaEventRecord(m->ev0, ctx->stream));
+  DP_TRY(dp_graph_launch(m->graph[1]));
+  DP_CUDA(ctx, cudaEventRecord(m->ev1, ctx->stream));
+  DP_CUDA(ctx, cudaMemcpyAsync(st + 1024, ctx->dev_status, 4, cudaMemcpyDeviceToHost, ctx->stream));
+  DP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  float ms = 0;
+  DP_CUDA(ctx, cudaEventElapsedTime(&ms, m->ev0, m->ev1));
+  m->last_ms = ms;
+  m->h_last = m->h;
+  if (st[1024]) DP_TRY(dp_take_dev_status(ctx));
+  m->head_pending = true;
+  m->seq_len[0] += 1;
+  return DP_OK;
+}
+
 extern "C" dp_status dp_model_read_logits(dp_model *m, float *host, int n) {
   if (!m || !host) return DP_ERR_INVALID;
   DP_CHECK(m->ctx, n > 0 && n <= m->cfg.max_batch * m->vocab_l, "readLogits: %d values requested, %d available", n, m->cfg.max_batch * m->vocab_l);
+  DP_TRY(settle_head(m, false));
   DP_CUDA(m->ctx, cudaMemcpyAsync(host, m->logits, (size_t)n * 4, cudaMemcpyDeviceToHost, m->ctx->stream));
   DP_CUDA(m->ctx, cudaStreamSynchronize(m->ctx->stream));
   return DP_OK;
@@ -1362,6 +1429,7 @@ extern "C" dp_status dp_model_bench_gemv(dp_model *m, int reps, double *ms_total
   const dp_model_cfg &c = m->cfg;
   DP_CHECK(ctx, reps > 0, "bench_gemv: reps must be positive");
   DP_CHECK(ctx, !m->stack, "bench_gemv: the model holds no Q4_K matrices");
+  DP_TRY(settle_head(m, false));
   const int H = c.hidden;
   struct Shape { int N, K; };
   const Shape sh[4] = {{m->qdim + 2 * m->kvdim, H}, {H, m->qdim}, {2 * m->inter, H}, {H, m->inter}};

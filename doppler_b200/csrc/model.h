@@ -51,13 +51,14 @@ struct dp_model {
   bool fuse_qk = true;  // decode: QK norm + RoPE + KV append inside the attention kernel
   std::vector<int> seq_len;
   const PackedRows *packed = nullptr;  // set while run_layers runs such a pass
-  dp_graph *graph[2] = {nullptr, nullptr};
+  dp_graph *graph[2] = {nullptr, nullptr};  // a decode step; a step of one sequence without logits
   int graph_batch[2] = {0, 0};
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   double last_ms = 0;
   size_t weight_bytes = 0;
   int allreduce_mode = 0;
   dp_stack *stack = nullptr;  // a decoder described layer by layer (stack.cu): its weights, sequence state and activations
+  bool head_pending = false;  // the last pass was a step without logits: dp_model_read_logits computes them from m->h
   bool final_norm_done = false;  // set by run_layers when the exchange kernel already applied the final RMSNorm
 };
 
@@ -70,6 +71,7 @@ dp_status dp_stack_ready(dp_model *m);  // every tensor loaded
 dp_status dp_stack_embed(dp_model *m, const int *ids, int rows, bool decode);
 dp_status dp_stack_run_layers(dp_model *m, int rows, bool decode, int seq, int start_pos);
 dp_status dp_stack_logits(dp_model *m, const float *hrow, int rows);
+dp_status dp_stack_hidden(dp_model *m);  // m->h of a decode row, where the logits' product would have completed it
 // logits of rows at[0..n) of m->h, 2 to dp_stack_wanted_rows of them (0: none), in the activations of the portion that has run
 constexpr int DP_WANTED_ROWS = 32;
 int dp_stack_wanted_rows(dp_model *m);

@@ -1077,6 +1077,14 @@ dp_status dp_stack_logits(dp_model *m, const float *hrow, int rows) {
   return product(m, s->embed, s->a, st, m->logits, rows);
 }
 
+dp_status dp_stack_hidden(dp_model *m) {
+  dp_stack *s = m->stack;
+  if (s->pending < 0) return DP_OK;
+  const int cur = s->pending;
+  s->pending = -1;
+  return dpk_stream_sum(m->ctx, s->x[cur], s->y, s->pending_end, s->cfg.streams, s->cfg.width, m->h, 1);
+}
+
 int dp_stack_wanted_rows(dp_model *m) {
   dp_stack *s = m->stack;
   if (!dpk_head_rows_ok(s->cfg.width)) return 0;

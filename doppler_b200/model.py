@@ -58,6 +58,10 @@ class Runner:
                                                           out.ctypes.data_as(C.c_void_p)))
         return out
 
+    def advance(self, token: int):
+        """One token of sequence 0 whose logits are not wanted (``read_logits`` still gives them if it is called next)."""
+        self.device.check(self.device.lib.dp_model_advance(self.h, token))
+
     @property
     def last_decode_ms(self) -> float:
         return float(self.device.lib.dp_model_last_decode_ms(self.h))
