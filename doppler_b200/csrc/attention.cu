@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(ATT_THREADS, LPK == 16 ? 2 : 1) attn_split_ker
 // the head's size; against 16 for all sizes up to 512 the kernel takes, in us (f16 unless it says f32):
 //   32 sequences of 2048 keys, 16 heads of 128 / 160 / 192 / 256: 586 -> 268, 695 -> 290, 768 -> 384, 1006 -> 430
 //   4 sequences of 8192 keys, 32 heads: 468 -> 410, 573 -> 451, 629 -> 605, 812 -> 676
-//   700-token portion, 16 heads, f32: 774 -> 414, 1045 -> 428, 1049 -> 686, 1059 -> 698
+//   700-token portion, 16 heads, f32: 774 -> 414, 1045 -> 428, 1049 -> 686, 1059 -> 698 (attention_rows.cu since)
 // (5 because heads of 129 to 160 would be up to 6 % slower with 8 than with 16).  Two keys at a time pay up to 128 values
 // only, where the registers of both fit beside enough warps; beyond, the loop is left alone (256 values, 4 x 8192 keys, two at
 // a time: 1275 us; 512 values: 2962 against 1182).
@@ -320,6 +320,12 @@ bool dpk_attention_latent_eligible(dp_ctx *ctx, const dpk_attn_params &p);
 int dpk_attention_latent_splits(dp_ctx *ctx, const dpk_attn_params &p);
 dp_status dpk_attention_latent(dp_ctx *ctx, const dpk_attn_params &p, float *scratch, int splits);
 
+// several query rows in f32 arithmetic (attention_rows.cu)
+bool dpk_attention_rows_eligible(const dpk_attn_params &p);
+bool dpk_attention_rows_fills(dp_ctx *ctx, const dpk_attn_params &p, int splits);
+int dpk_attention_rows_splits(dp_ctx *ctx, const dpk_attn_params &p);
+dp_status dpk_attention_rows(dp_ctx *ctx, const dpk_attn_params &p, float *scratch, int splits);
+
 // the most keys one query row sees
 static long row_keys(const dpk_attn_params &p) { return p.chunk > 0 && p.chunk < p.kv_len ? p.chunk : p.kv_len; }
 
@@ -353,6 +359,11 @@ size_t dpk_attention_scratch_bytes(dp_ctx *ctx, const dpk_attn_params &p, int *s
     const int s = dpk_attention_latent_splits(ctx, p);
     *splits_out = s;
     return s == 1 ? 0 : (size_t)p.batch * p.seq_len * p.num_heads * s * (p.v_dim + 2) * sizeof(float);
+  }
+  if (dpk_attention_rows_eligible(p)) {
+    const int s = dpk_attention_rows_splits(ctx, p);
+    *splits_out = s;
+    return s == 1 ? 0 : (size_t)p.batch * p.seq_len * p.num_heads * s * ((p.v_dim ? p.v_dim : p.head_dim) + 2) * sizeof(float);
   }
   const bool fast = fast_shape(p, &gt);
   const int G = p.num_heads / p.num_kv_heads;
@@ -410,6 +421,8 @@ static dp_status attention_impl(dp_ctx *ctx, const dpk_attn_params &p, float *sc
     DP_TRY(dpk_attention_latent(ctx, p, scratch, splits));
   } else if (use_tc(ctx, p, &gt)) {
     DP_TRY(dpk_attention_tc_split(ctx, p, scratch, splits));
+  } else if (dpk_attention_rows_eligible(p) && dpk_attention_rows_fills(ctx, p, splits)) {
+    DP_TRY(dpk_attention_rows(ctx, p, scratch, splits));
   } else if (fast_shape(p, &gt)) {
     if (p.head_dim == 128) {
       if (gt == 1) DP_TRY((launch_fast<16, 1, 8>(ctx, p, scratch, splits)));
@@ -448,8 +461,10 @@ dp_status dpk_attention(dp_ctx *ctx, const dpk_attn_params &p) {
   const size_t bytes = dpk_attention_scratch_bytes(ctx, p, &splits);
   float *scratch = nullptr;
   if (bytes) {
-    DP_TRY(dp_scratch(ctx, &ctx->attn_scratch, bytes, "attention_split_partials"));
-    scratch = (float *)ctx->attn_scratch->dptr;
+    const dp_status st = dp_scratch(ctx, &ctx->attn_scratch, bytes, "attention_split_partials");
+    if (st == DP_ERR_OOM && dpk_attention_rows_eligible(p)) splits = 1;  // (one part needs no room)
+    else if (st != DP_OK) return st;
+    else scratch = (float *)ctx->attn_scratch->dptr;
   }
   return dpk_attention_with_scratch(ctx, p, scratch, splits);
 }

@@ -576,7 +576,7 @@ dp_status run_rows(dp_model *m, int rows, bool decode, int seq, int start_pos) {
       if (s->f32) ap.out = (float *)s->a;
       else { ap.out_bf16 = (__nv_bfloat16 *)s->a; ap.out_stride = ks; }
       int splits = 1;
-      if (decode) dpk_attention_scratch_bytes(ctx, ap, &splits);
+      if (dpk_attention_scratch_bytes(ctx, ap, &splits) > m->attn_scratch->bytes) splits = 1;
       DP_TRY(dpk_attention_with_scratch(ctx, ap, (float *)m->attn_scratch->dptr, splits));
     } else if (L.latent()) {
       DP_TRY(latent_rows(m, l, rows, decode, seq, start_pos, ks, map));

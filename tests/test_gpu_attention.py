@@ -206,6 +206,59 @@ def test_heads_of_every_size(dev, D, G):
             assert_close(got[b], exp, f"D{D} G{G} B{B} T{T} sequence {b}")
 
 
+def _exact_rows(q, k, v, causal, start, window, cap, kv_start):
+    """64-bit rows [T, H, D] and, element by element, a bound of the f32 kernel's error.  A logit is off by at most 24 roundings
+    (chains of 8, 4, 4 and 2 products, the scale, the change of base; the cap's tanh and division) of the terms it sums, a
+    weight by twice that much and its exponential's 4, a sum of values by chains of 16 keys and of their count / 16."""
+    T, H, D = q.shape
+    G, kv, u = H // k.shape[1], k.shape[0], 2.0 ** -24
+    out, bound = np.zeros((T, H, D)), np.zeros((T, H, D))
+    i, j = np.arange(T)[:, None] + start, np.arange(kv)[None] + kv_start
+    seen = np.ones((T, kv), bool)
+    if causal:
+        seen &= j <= i
+    if window:
+        seen &= (j > i - window) | (i < window)
+    for h in range(H):
+        kh, vh = k[:, h // G], v[:, h // G]
+        z, size = q[:, h] @ kh.T / np.sqrt(D), np.abs(q[:, h]) @ np.abs(kh).T / np.sqrt(D)
+        if cap:
+            z, size = np.tanh(z / cap) * cap, size + 4 * cap
+        z = np.where(seen, z, -np.inf)
+        p = np.exp(z - z.max(1, keepdims=True))
+        p /= p.sum(1, keepdims=True)
+        out[:, h] = p @ vh
+        bound[:, h] = u * (2 * 24 * np.where(seen, size, 0).max(1)[:, None] + 4 + 2 * (16 + kv / 16 + 6)) * (p @ np.abs(vh)) + 1e-30
+    return out, bound
+
+
+@pytest.mark.parametrize("H,Hkv,D,T,kv,opt", [
+    (8, 4, 256, 150, 400, {}),                                          # groups of 2, tiles of 16 positions, splits
+    (24, 8, 132, 333, 333, dict(sliding_window=50)),                    # groups of 3 (a head a block), a size that fills no tile
+    (8, 1, 252, 130, 700, dict(attn_softcap=2.5)),                      # groups of 8
+    (2, 2, 160, 401, 401, dict(causal=False)),
+    (12, 1, 200, 90, 641, dict(kv_start=37)),                           # groups of 4, the cache begins behind the sequence's start
+    (32, 8, 256, 258, 258, {}),                                         # one part
+])
+def test_rows_in_f32(dev, H, Hkv, D, T, kv, opt):
+    s = synthetic.key(61, D * 100 + T)
+    start = kv - T + opt.get("kv_start", 0)
+    q, k, v = synthetic.normal_f32(s, T * H * D), synthetic.normal_f16(s + 1, kv * Hkv * D), synthetic.normal_f16(s + 2, kv * Hkv * D)
+    got = _attn(dev, q, k, v, H, D, seq_len=T, kv_len=kv, num_kv_heads=Hkv, start_pos=start, **opt).reshape(T, H, D)
+    exp, bound = _exact_rows(q.reshape(T, H, D).astype(np.float64), k.reshape(kv, Hkv, D).astype(np.float64), v.reshape(kv, Hkv, D).astype(np.float64),
+                             opt.get("causal", True), start, opt.get("sliding_window", 0), opt.get("attn_softcap", 0.0), opt.get("kv_start", 0))
+    assert np.all(np.abs(got - exp) <= bound), float((np.abs(got - exp) / bound).max())
+    if opt:
+        return
+    # a key that is NaN and values that are infinite change the rows that see them and no other
+    bad = kv - T // 2
+    k2, v2 = k.reshape(kv, -1).copy(), v.reshape(kv, -1).copy()
+    k2[bad + 1, ::3], v2[bad] = np.nan, np.inf
+    mixed = _attn(dev, q, k2.ravel(), v2.ravel(), H, D, seq_len=T, kv_len=kv, num_kv_heads=Hkv, start_pos=start).reshape(T, H, D)
+    first = bad - start
+    assert np.array_equal(mixed[:first], got[:first]) and not np.isfinite(mixed[first]).any() and (mixed[first + 1:] != got[first + 1:]).all()
+
+
 def test_attention_argument_errors(dev):
     q = dev.tensor_from(np.zeros(8 * 128, np.float32))
     kv = dev.tensor_from(np.zeros(16 * 2 * 128, np.float16))

@@ -286,6 +286,17 @@ def test_large_sizes_bf16(dev, name):
     m.destroy()
 
 
+def test_attention_rows_f32(dev):
+    """Prompts long enough for the query-tiled kernel over an f32 cache, values shorter than keys, in one portion and in two."""
+    cfg, n = config([attention(heads=12, kv_heads=2, dim=72, vdim=56, scale=0.2, chunk=170)], width=128), 333
+    w, t, logits, _ = oracle("attention rows f32", cfg, n)
+    m = build(dev, cfg, w, n)
+    check(m.extend(t, range(n)), logits, F32_TOL)
+    m.release(0)
+    check(np.concatenate([m.extend(t[:120], range(120)), m.extend(t[120:], range(n - 120))]), logits, F32_TOL)
+    m.destroy()
+
+
 @pytest.mark.parametrize("heads,kv_heads,dim", [(8, 2, 128), (6, 2, 64), (12, 1, 64)])
 def test_split_keys_bf16(dev, heads, kv_heads, dim):
     """A chunk so long that decoding splits its keys over several CTAs, before and after the chunk's edge."""
