@@ -175,6 +175,21 @@ def test_f16_weight_rows_kernel(dev, M, N, K):
         assert_close(goth[m].astype(np.float32), ref, f"f16-weight rows f16 act row {m}", rtol=2e-3)
 
 
+@pytest.mark.parametrize("M,N,K", [(2, 2, 64), (16, 8, 64), (17, 1187, 192), (64, 19000, 128), (65, 19011, 64), (64, 40001, 64), (129, 38000, 64), (7, 304, 4096)])
+def test_f16_weight_rows_tiles(dev, M, N, K):
+    """Tiles of every kind: a few rows, one MMA, two that share the activations, several rounds; ragged ends of rows and batch.
+    Bound: 22 bits of an activation, K / 16 sums of the accumulator and one of hi and lo, each cut to 24 bits."""
+    W = synthetic.normal_f16(synthetic.key(35, N), N * K, 0.02)
+    A = synthetic.normal_f32(synthetic.key(35, M), M * K).reshape(M, K)
+    w, a = W.reshape(N, K).astype(np.float64), A.astype(np.float64)
+    size = np.abs(a) @ np.abs(w).T
+    got = _matmul(dev, W, N, K, A, M, wdtype="f16").reshape(M, N)
+    assert np.all(np.abs(got - a @ w.T) <= size * (2.0 ** -22 + (K / 16 + 4) * 2.0 ** -23))
+    Ah = A.astype(np.float16)
+    got = _matmul(dev, W, N, K, Ah, M, wdtype="f16", a_dtype="f16").reshape(M, N)
+    assert np.all(np.abs(got - Ah.astype(np.float64) @ w.T) <= size * (2.0 ** -23 * (K / 16 + 4)) * (1 + 2.0 ** -10))
+
+
 def test_matmul_argument_errors(dev):
     N, K = 8, 256
     W = synthetic.q4k_matrix(synthetic.key(41, 0), N, K)
