@@ -13,8 +13,10 @@
 // a two-stage cp.async ring (rows padded by 16 bytes: conflict-free fragment reads).  Tensor-core math
 // with mma.sync m16n8k16 in the flash-attention arrangement: S = Q K^T with Q held in registers as an
 // f16 hi half and an f16 lo half (two products, so the f32 query loses nothing that matters), online
-// softmax in f32 per 16 x 32 score tile, O += P V with P likewise as f16 hi + lo halves and V fragments
-// from ldmatrix.trans.  f32 accumulators; the output is written once, normalised.
+// softmax in f32 per 16 x 32 score tile, O += P V with P likewise as f16 hi + lo halves; K and V fragments
+// by ldmatrix, four matrices at a time, masks and the rescaling of O only where a row needs them.  f32
+// accumulators; the output is written once, normalised.  Bound: the legacy tensor pipe, 34 G products in
+// 232 us at 2048 tokens of 32 heads (236 before loads of four matrices; keys of 192 values, 1500 tokens: 212 -> 196).
 #include "common.h"
 #include "pdl.cuh"
 
@@ -41,8 +43,11 @@ __device__ __forceinline__ void apf_mma(float (&c)[4], const uint32_t (&a)[4], u
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void apf_ldmatrix_x2_trans(uint32_t &r0, uint32_t &r1, uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n" : "=r"(r0), "=r"(r1) : "r"(addr) : "memory");
+__device__ __forceinline__ void apf_ldmatrix(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void apf_ldmatrix_trans(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
 __device__ __forceinline__ uint32_t apf_pack(float a, float b) {
   const __half2 h = __floats2half2_rn(a, b);
@@ -91,6 +96,7 @@ __global__ void __launch_bounds__(APF_THREADS, 1) attn_prefill_tc_kernel(dpk_att
   const int loA = p.chunk > 0 ? posA / p.chunk * p.chunk : 0, loB = p.chunk > 0 ? posB / p.chunk * p.chunk : 0;
   const int tile0 = p.chunk > 0 ? (start_pos + qtile * QT) / p.chunk * p.chunk / APF_KT : 0;
   const int warp_lo = p.chunk > 0 ? (start_pos + q0) / p.chunk * p.chunk : 0;
+  const int last_lo = p.chunk > 0 ? (start_pos + q0 + 15) / p.chunk * p.chunk : 0;
 
   const __half *kbase = p.k + (size_t)cb * p.kv_batch_stride + (size_t)kvh * k_pieces * 8;
   const __half *vbase = p.v + (size_t)cb * (p.v_batch_stride ? p.v_batch_stride : p.kv_batch_stride) + (size_t)kvh * v_pieces * 8;
@@ -170,8 +176,7 @@ __global__ void __launch_bounds__(APF_THREADS, 1) attn_prefill_tc_kernel(dpk_att
     __syncthreads();
     const int key0 = tile * APF_KT;
     if (key0 < warp_keys && key0 + APF_KT > warp_lo) {  // (warp-uniform) other tiles are masked for all of this warp's rows
-      const unsigned char *sK = apf_smem + (tile & 1) * L::STAGE;
-      const uint32_t sV = smem0 + (uint32_t)(tile & 1) * L::STAGE + L::VTILE;
+      const uint32_t sK = smem0 + (uint32_t)(tile & 1) * L::STAGE, sV = sK + L::VTILE;
       // ---- S = (scale * Q) K^T for 16 rows x 32 keys ----
       float sc[4][4];
 #pragma unroll
@@ -179,22 +184,27 @@ __global__ void __launch_bounds__(APF_THREADS, 1) attn_prefill_tc_kernel(dpk_att
 #pragma unroll
       for (int ks = 0; ks < KS; ks++) {
 #pragma unroll
-        for (int nt = 0; nt < 4; nt++) {
-          const unsigned char *kr = sK + (nt * 8 + g) * L::KROW + (16 * ks + 2 * t) * 2;
-          const uint32_t b0 = *reinterpret_cast<const uint32_t *>(kr), b1 = *reinterpret_cast<const uint32_t *>(kr + 16);
-          apf_mma(sc[nt], qh[ks], b0, b1);
-          apf_mma(sc[nt], ql[ks], b0, b1);
+        for (int nt = 0; nt < 4; nt += 2) {
+          uint32_t b[4];  // both halves of k of eight keys, then of the next eight
+          apf_ldmatrix(b, sK + (uint32_t)((nt * 8 + (lane & 7) + 8 * (lane >> 4)) * L::KROW + ks * 32 + ((lane >> 3) & 1) * 16));
+          apf_mma(sc[nt], qh[ks], b[0], b[1]);
+          apf_mma(sc[nt + 1], qh[ks], b[2], b[3]);
+          apf_mma(sc[nt], ql[ks], b[0], b[1]);
+          apf_mma(sc[nt + 1], ql[ks], b[2], b[3]);
         }
       }
       // ---- causal mask, online softmax ----
+      const bool whole = key0 + APF_KT - 1 <= start_pos + q0 && key0 + APF_KT <= kv_len && key0 >= last_lo;  // (warp-uniform) all rows see all keys
       float tmA = -INFINITY, tmB = -INFINITY;
 #pragma unroll
       for (int nt = 0; nt < 4; nt++) {
+        if (!whole) {
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const int key = key0 + nt * 8 + 2 * t + (e & 1);
-          const int pos = e < 2 ? posA : posB;
-          if (key > pos || key >= kv_len || key < (e < 2 ? loA : loB)) sc[nt][e] = -INFINITY;
+          for (int e = 0; e < 4; e++) {
+            const int key = key0 + nt * 8 + 2 * t + (e & 1);
+            const int pos = e < 2 ? posA : posB;
+            if (key > pos || key >= kv_len || key < (e < 2 ? loA : loB)) sc[nt][e] = -INFINITY;
+          }
         }
         tmA = fmaxf(tmA, fmaxf(sc[nt][0], sc[nt][1]));
         tmB = fmaxf(tmB, fmaxf(sc[nt][2], sc[nt][3]));
@@ -215,8 +225,10 @@ __global__ void __launch_bounds__(APF_THREADS, 1) attn_prefill_tc_kernel(dpk_att
       }
       lA = lA * cA + sA;
       lB = lB * cB + sB;
+      if (__any_sync(0xffffffffu, cA != 1.0f || cB != 1.0f)) {  // a new maximum in one of the rows
 #pragma unroll
-      for (int j = 0; j < NV; j++) { o[j][0] *= cA; o[j][1] *= cA; o[j][2] *= cB; o[j][3] *= cB; }
+        for (int j = 0; j < NV; j++) { o[j][0] *= cA; o[j][1] *= cA; o[j][2] *= cB; o[j][3] *= cB; }
+      }
       // ---- O += P V: P (16 x 32) as two A fragments, V fragments transposed out of shared memory ----
 #pragma unroll
       for (int kk = 0; kk < 2; kk++) {
@@ -229,13 +241,15 @@ __global__ void __launch_bounds__(APF_THREADS, 1) attn_prefill_tc_kernel(dpk_att
           pa[i] = *reinterpret_cast<const uint32_t *>(&hi);
           pl[i] = apf_pack(x0 - hf.x, x1 - hf.y);
         }
-        const uint32_t vrow = sV + (uint32_t)(16 * kk + (lane & 15)) * L::VROW;
+        const uint32_t vrow = sV + (uint32_t)(16 * kk + (lane & 15)) * L::VROW + (uint32_t)(lane >> 4) * 16u;
 #pragma unroll
-        for (int j = 0; j < NV; j++) {
-          uint32_t b0, b1;
-          apf_ldmatrix_x2_trans(b0, b1, vrow + (uint32_t)j * 16u);
-          apf_mma(o[j], pa, b0, b1);
-          apf_mma(o[j], pl, b0, b1);
+        for (int j = 0; j < NV; j += 2) {
+          uint32_t b[4];
+          apf_ldmatrix_trans(b, vrow + (uint32_t)j * 16u);
+          apf_mma(o[j], pa, b[0], b[1]);
+          apf_mma(o[j + 1], pa, b[2], b[3]);
+          apf_mma(o[j], pl, b[0], b[1]);
+          apf_mma(o[j + 1], pl, b[2], b[3]);
         }
       }
     }
