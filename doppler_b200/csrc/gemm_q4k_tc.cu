@@ -74,7 +74,7 @@ __global__ void __launch_bounds__((DQ_WARPS + 2) * 32, 1) gemm_q4k_tc_kernel(con
   const TcSmem L = tc_layout(BN, SA, SB, MT, NPROD);
   static_assert(MT * BN <= 512, "accumulators exceed tensor memory");
   constexpr uint32_t B_TILE = (uint32_t)BN * 128u;          // bytes of the f16 weight tile of a stage
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int n0 = blockIdx.x * BN, m0 = blockIdx.y * (128 * MT);
   // Split over K (grid.z parts, whole super-blocks each): a problem of few tiles (N = 4096 at M <= 256 is 32)
   // fills the GPU with several CTAs per tile.  Every part writes its own f32 tile; a second kernel adds the
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__((DQ_WARPS + 2) * 32, 1) gemm_q4k_tc_kernel(con
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   if (warp == 0) {
     // ---------------- activation tiles: TMA ----------------
@@ -137,33 +137,23 @@ __global__ void __launch_bounds__((DQ_WARPS + 2) * 32, 1) gemm_q4k_tc_kernel(con
       }
     }
   } else if (warp == 1) {
-    // ---------------- MMA issue ----------------
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc_f16(128, BN);
-      bool ok = true;
-      for (int kt = 0; kt < num_k && ok; kt++) {
-        const int sa = kt % SA, sb = kt % SB;
-        if (!mbar_wait_bounded(full_a(sa), (uint32_t)(kt / SA) & 1u, abort_flag)) { ok = false; break; }
-        if (!mbar_wait_bounded(full_b(sb), (uint32_t)(kt / SB) & 1u, abort_flag)) { ok = false; break; }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a_addr = smem_u32(smem + L.a + (uint32_t)sa * L.stage_a);
-        const uint32_t b_addr = smem_u32(smem + L.b + (uint32_t)sb * L.stage_b);
+    // ---------------- MMA issue (by the whole warp, see umma.cuh) ----------------
+    const uint32_t idesc = umma_idesc_f16(128, BN);
+    const uint64_t a_first = umma_desc_sw128(smem_u32(smem + L.a)), b_first = umma_desc_sw128(smem_u32(smem + L.b));
+    bool ok = true;
+    for (int kt = 0; kt < num_k; kt++) {
+      const int sa = kt % SA, sb = kt % SB;
+      if (!mbar_wait_warp(full_a(sa), (uint32_t)(kt / SA) & 1u, abort_flag) || !mbar_wait_warp(full_b(sb), (uint32_t)(kt / SB) & 1u, abort_flag)) { ok = false; break; }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint64_t adesc = a_first + (uint64_t)((uint32_t)sa * (L.stage_a >> 4)), bdesc = b_first + (uint64_t)((uint32_t)sb * (L.stage_b >> 4));
 #pragma unroll
-        for (int k16 = 0; k16 < BK / 16; k16++) {
-          const uint64_t bdesc = umma_desc_sw128(b_addr + (uint32_t)k16 * 32u);
-          const uint32_t acc = (kt > 0 || k16 > 0) ? 1u : 0u;
-#pragma unroll
-          for (int mt = 0; mt < MT; mt++) {
-            const uint64_t adesc = umma_desc_sw128(a_addr + (uint32_t)mt * 128u * 128u + (uint32_t)k16 * 32u);
-            umma_f16(tmem_base + (uint32_t)(mt * BN), adesc, bdesc, idesc, acc);
-            if constexpr (NPROD == 2) umma_f16(tmem_base + (uint32_t)(mt * BN), adesc, umma_desc_sw128(b_addr + B_TILE + (uint32_t)k16 * 32u), idesc, 1u);
-          }
-        }
-        // both stages are free once these MMAs have read them
-        umma_commit(done(kt % SD));
+      for (int mt = 0; mt < MT; mt++) {
+        if constexpr (NPROD == 2) umma_step_warp<false>(tmem_base + (uint32_t)(mt * BN), adesc + (uint64_t)(mt * (128 * 128 >> 4)), bdesc + (B_TILE >> 4), idesc, (uint32_t)kt);  // the small products first
+        umma_step_warp<false>(tmem_base + (uint32_t)(mt * BN), adesc + (uint64_t)(mt * (128 * 128 >> 4)), bdesc, idesc, NPROD == 2 ? 1u : (uint32_t)kt);
       }
-      if (ok) umma_commit(accum_bar);
+      umma_commit_warp<false>(done(kt % SD));  // both stages are free once these MMAs have read them
     }
+    if (ok) umma_commit_warp<false>(accum_bar);
   } else {
     // ---------------- weight tiles: dequantise into swizzled shared memory ----------------
     const int dw = warp - 2;            // 0..7
@@ -400,7 +390,7 @@ __global__ void __launch_bounds__((BNMAX / 16 + 2) * 32, 1) gemm_q4k_tc2_kernel(
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const TcSmem L = tc_layout(HBMAX, SA, SB, PS, NPROD);
   constexpr uint32_t B_TILE = (uint32_t)HBMAX * 128u;       // bytes of this CTA's half of the f16 weight tile of a stage
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const uint32_t rank = cluster_ctarank();
   const int n0 = cluster_x < wide_tiles ? cluster_x * bn_wide : wide_tiles * bn_wide + (cluster_x - wide_tiles) * bn_narrow;
   const int m0 = blockIdx.y * (256 * PS);
@@ -443,7 +433,7 @@ __global__ void __launch_bounds__((BNMAX / 16 + 2) * 32, 1) gemm_q4k_tc2_kernel(
   __syncthreads();
   cluster_sync_all();  // both CTAs' barriers exist and both allocations are done before anyone signals across
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   if (warp == 0) {
     // ---------------- activation tiles: this CTA's rows of both passes ----------------
@@ -471,30 +461,23 @@ __global__ void __launch_bounds__((BNMAX / 16 + 2) * 32, 1) gemm_q4k_tc2_kernel(
         mbar_arrive_remote(full_b0 + 8u * (uint32_t)sb);
       }
     }
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       const uint32_t idesc = umma_idesc_f16(256, bn);
+      const uint64_t a_first = umma_desc_sw128(smem_u32(smem + L.a)), b_first = umma_desc_sw128(smem_u32(smem + L.b));
       bool ok = true;
-      for (int kt = 0; kt < num_k && ok; kt++) {
+      for (int kt = 0; kt < num_k; kt++) {
         const int sa = kt % SA, sb = kt % SB;
-        if (!mbar_wait_bounded_cluster(full_a(sa), (uint32_t)(kt / SA) & 1u, abort_flag) ||
-            !mbar_wait_bounded_cluster(full_b(sb), (uint32_t)(kt / SB) & 1u, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp_cluster(full_a(sa), (uint32_t)(kt / SA) & 1u, abort_flag) || !mbar_wait_warp_cluster(full_b(sb), (uint32_t)(kt / SB) & 1u, abort_flag)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a_addr = smem_u32(smem + L.a + (uint32_t)sa * L.stage_a);
-        const uint32_t b_addr = smem_u32(smem + L.b + (uint32_t)sb * L.stage_b);
+        const uint64_t adesc = a_first + (uint64_t)((uint32_t)sa * (L.stage_a >> 4)), bdesc = b_first + (uint64_t)((uint32_t)sb * (L.stage_b >> 4));
 #pragma unroll
-        for (int k16 = 0; k16 < BK / 16; k16++) {
-          const uint64_t bdesc = umma_desc_sw128(b_addr + (uint32_t)k16 * 32u);
-          const uint32_t acc = (kt > 0 || k16 > 0) ? 1u : 0u;
-#pragma unroll
-          for (int ps = 0; ps < PS; ps++) {
-            const uint64_t adesc = umma_desc_sw128(a_addr + (uint32_t)ps * 128u * 128u + (uint32_t)k16 * 32u);
-            umma_f16_2sm(tmem_base + (uint32_t)(ps * BNMAX), adesc, bdesc, idesc, acc);
-            if constexpr (NPROD == 2) umma_f16_2sm(tmem_base + (uint32_t)(ps * BNMAX), adesc, umma_desc_sw128(b_addr + B_TILE + (uint32_t)k16 * 32u), idesc, 1u);
-          }
+        for (int ps = 0; ps < PS; ps++) {
+          if constexpr (NPROD == 2) umma_step_warp<true>(tmem_base + (uint32_t)(ps * BNMAX), adesc + (uint64_t)(ps * (128 * 128 >> 4)), bdesc + (B_TILE >> 4), idesc, (uint32_t)kt);  // the small products first
+          umma_step_warp<true>(tmem_base + (uint32_t)(ps * BNMAX), adesc + (uint64_t)(ps * (128 * 128 >> 4)), bdesc, idesc, NPROD == 2 ? 1u : (uint32_t)kt);
         }
-        umma_commit_2sm(done(kt % SD));  // arrives on both CTAs' barrier: their stages of this step are free
+        umma_commit_warp<true>(done(kt % SD));  // arrives on both CTAs' barrier: their stages of this step are free
       }
-      if (ok) umma_commit_2sm(accum_bar);
+      if (ok) umma_commit_warp<true>(accum_bar);
     }
   } else {
     // ---------------- this CTA's half of the weight tile ----------------
