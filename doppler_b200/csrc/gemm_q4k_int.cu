@@ -745,14 +745,20 @@ __device__ __forceinline__ float qi_row_scale(float mx, int e, int guard) {
   return guard && special ? __int_as_float(0x7fc00000) : qi_pow2(e);
 }
 
-__device__ __forceinline__ float qi_block_max(float v, float *sh) {  // eight warps
+template <int WARPS = 8>
+__device__ __forceinline__ float qi_block_max(float v, float *sh) {  // 8 or 32 warps
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
   __syncthreads();
-  float t = sh[0];
+  float t = sh[WARPS == 32 ? threadIdx.x & 31 : 0];
+  if constexpr (WARPS == 32) {
 #pragma unroll
-  for (int w = 1; w < 8; w++) t = fmaxf(t, sh[w]);
+    for (int o = 16; o > 0; o >>= 1) t = fmaxf(t, __shfl_xor_sync(0xffffffffu, t, o));
+  } else {
+#pragma unroll
+    for (int w = 1; w < WARPS; w++) t = fmaxf(t, sh[w]);
+  }
   return t;
 }
 
@@ -795,22 +801,23 @@ __global__ void __launch_bounds__(256) int_rows_kernel(const AT *__restrict__ in
 
 // The same for f32 rows with the row in registers (K % 32 == 0, K <= 1024 * NV, 16-byte aligned): one pass, 16-byte loads.
 // With norm_w the row is RMS-normalised first (rmsnorm.wgsl:119-187), element for element and reduction step for
-// reduction step as rmsnorm_vec_kernel (small_ops.cu) does it for rows of 1024..4096 values.
-template <int NV>
-__global__ void __launch_bounds__(256) int_rows_vec_kernel(const float *__restrict__ in, __half *__restrict__ hi, __half *__restrict__ lo, float *__restrict__ scale,
+// reduction step as rmsnorm_vec_kernel (small_ops.cu) does it for rows of 1024..4096 values, by 256 threads.  Few rows without
+// a norm take 1024 threads each (the same bits): a row's loads are one wait and not twelve deep; 64 x 12288 8.6 -> 5.7 us, 64 x 4096 4.6 -> 4.1.
+template <int NV, int T = 256>
+__global__ void __launch_bounds__(T) int_rows_vec_kernel(const float *__restrict__ in, __half *__restrict__ hi, __half *__restrict__ lo, float *__restrict__ scale,
                                                            __half *__restrict__ sums, int K, int kp, const IntPlan p, const float *__restrict__ norm_w, float eps, int guard) {
   pdl_launch();
   pdl_wait();
-  __shared__ float sh[8], shn[8];
+  __shared__ float sh[T / 32], shn[8];
   const int row = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n4 = K >> 2;
   const size_t base = (size_t)row * K, out = (size_t)row * kp;
   float4 v[NV];
 #pragma unroll
   for (int i = 0; i < NV; i++) {
-    const int idx = threadIdx.x + i * 256;
+    const int idx = threadIdx.x + i * T;
     v[i] = idx < n4 ? *reinterpret_cast<const float4 *>(in + base + 4 * idx) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   }
-  if (norm_w) {
+  if (T == 256 && norm_w) {
     float ss = 0.0f;
 #pragma unroll
     for (int i = 0; i < NV; i++) ss = fmaf(v[i].x, v[i].x, fmaf(v[i].y, v[i].y, fmaf(v[i].z, v[i].z, fmaf(v[i].w, v[i].w, ss))));
@@ -824,7 +831,7 @@ __global__ void __launch_bounds__(256) int_rows_vec_kernel(const float *__restri
     const float inv_rms = 1.0f / sqrtf(total / (float)K + eps);
 #pragma unroll
     for (int i = 0; i < NV; i++) {
-      const int idx = threadIdx.x + i * 256;
+      const int idx = threadIdx.x + i * T;
       if (idx < n4) {
         const float4 w = *reinterpret_cast<const float4 *>(norm_w + 4 * idx);
         v[i].x = v[i].x * inv_rms * w.x; v[i].y = v[i].y * inv_rms * w.y; v[i].z = v[i].z * inv_rms * w.z; v[i].w = v[i].w * inv_rms * w.w;
@@ -834,14 +841,14 @@ __global__ void __launch_bounds__(256) int_rows_vec_kernel(const float *__restri
   float mx = 0.0f;
 #pragma unroll
   for (int i = 0; i < NV; i++) mx = fmaxf(fmaxf(mx, fmaxf(fabsf(v[i].x), fabsf(v[i].y))), fmaxf(fabsf(v[i].z), fabsf(v[i].w)));
-  mx = qi_block_max(mx, sh);
+  mx = qi_block_max<T / 32>(mx, sh);
   const int e = qi_row_exponent(mx);
   const float down = qi_pow2(-e);
   if (threadIdx.x == 0) scale[row] = qi_row_scale(mx, e, guard);
   __half *sums_row = sums + (size_t)row * ((size_t)p.parts * p.npu * 256);
 #pragma unroll
   for (int i = 0; i < NV; i++) {
-    const int idx = threadIdx.x + i * 256;
+    const int idx = threadIdx.x + i * T;
     const float s0 = v[i].x * down, s1 = v[i].y * down, s2 = v[i].z * down, s3 = v[i].w * down;
     float t = (s0 + s1) + (s2 + s3);  // eight consecutive threads hold a sub-block
     t += __shfl_xor_sync(0xffffffffu, t, 1);
@@ -857,7 +864,7 @@ __global__ void __launch_bounds__(256) int_rows_vec_kernel(const float *__restri
   }
   if ((int)threadIdx.x < kp - K) hi[out + K + threadIdx.x] = lo[out + K + threadIdx.x] = __float2half_rn(0.0f);
   // (sub-blocks beyond a K that is no multiple of 256)
-  for (int s = (K >> 5) + (int)threadIdx.x; s < p.bpr * 8; s += 256) qi_put_sum(sums_row, p, s, 0.0f);
+  for (int s = (K >> 5) + (int)threadIdx.x; s < p.bpr * 8; s += T) qi_put_sum(sums_row, p, s, 0.0f);
 }
 
 // The same for f16 rows (K % 32 == 0, K <= 2048 * NV, 16-byte aligned): one pass, 16-byte accesses, where int_rows_kernel reads
@@ -906,15 +913,34 @@ __global__ void __launch_bounds__(256) int_rows_f16_kernel(const __half *__restr
 
 // C = sum of the parts of a K-split launch, in a fixed order (+ residual, which may be C itself)
 template <typename OutT>
-__global__ void __launch_bounds__(256) int_reduce_kernel(const float *__restrict__ parts, OutT *C, size_t n, int splits, const float *residual) {
+__global__ void __launch_bounds__(256) int_reduce_kernel(const float *__restrict__ parts, OutT *C, size_t n, int splits, const float *residual, int wide) {
   pdl_launch();
   pdl_wait();
+  auto put = [&](size_t i, float v) {
+    if constexpr (sizeof(OutT) == 4) C[i] = v;
+    else C[i] = __float2half_rn(v);
+  };
+  if (wide) {  // all parts' loads at once, 16 bytes each: one wait (64 x 4096, five parts: 3.6 us -> 2.6)
+    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n / 4; i += (size_t)gridDim.x * 256) {
+      float4 v[8];
+#pragma unroll
+      for (int z = 0; z < 8; z++)
+        if (z < splits) v[z] = *reinterpret_cast<const float4 *>(parts + (size_t)z * n + 4 * i);
+      const float4 r = residual ? *reinterpret_cast<const float4 *>(residual + 4 * i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+      for (int z = 1; z < 8; z++)
+        if (z < splits) { v[0].x += v[z].x; v[0].y += v[z].y; v[0].z += v[z].z; v[0].w += v[z].w; }
+      if (residual) { v[0].x += r.x; v[0].y += r.y; v[0].z += r.z; v[0].w += r.w; }
+      if constexpr (sizeof(OutT) == 4) *reinterpret_cast<float4 *>(C + 4 * i) = v[0];
+      else { put(4 * i, v[0].x); put(4 * i + 1, v[0].y); put(4 * i + 2, v[0].z); put(4 * i + 3, v[0].w); }
+    }
+    return;
+  }
   for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) {
     float acc = parts[i];
     for (int z = 1; z < splits; z++) acc += parts[(size_t)z * n + i];
     if (residual) acc += residual[i];
-    if constexpr (sizeof(OutT) == 4) C[i] = acc;
-    else C[i] = __float2half_rn(acc);
+    put(i, acc);
   }
 }
 
@@ -1022,8 +1048,10 @@ dp_status dpk_gemm_q4k_int(dp_ctx *ctx, const uint8_t *W, const void *A, dp_dtyp
   const float eps = fuse ? fuse->eps : 0.0f;
   if (vec) {
     const float *a = (const float *)A;
+    const bool few = M <= ctx->sm_count && !norm_w && K > 1024;
     auto rows = K <= 1024 ? int_rows_vec_kernel<1> : K <= 4096 ? int_rows_vec_kernel<4> : K <= 12288 ? int_rows_vec_kernel<12> : int_rows_vec_kernel<16>;
-    DP_LAUNCH(ctx, rows, (unsigned)M, 256, 0, a, hi, lo, scale, sums, K, kp, p, norm_w, eps, guard);
+    if (few) rows = K <= 4096 ? int_rows_vec_kernel<1, 1024> : K <= 12288 ? int_rows_vec_kernel<3, 1024> : int_rows_vec_kernel<4, 1024>;
+    DP_LAUNCH(ctx, rows, (unsigned)M, few ? 1024 : 256, 0, a, hi, lo, scale, sums, K, kp, p, norm_w, eps, guard);
   } else if (f32a) {
     DP_LAUNCH(ctx, int_rows_kernel<float>, (unsigned)M, 256, 0, (const float *)A, hi, lo, scale, sums, K, kp, p, guard);
   } else if (K % 32 == 0 && K <= 16384 && ((uintptr_t)A & 15) == 0) {
@@ -1072,11 +1100,12 @@ dp_status dpk_gemm_q4k_int(dp_ctx *ctx, const uint8_t *W, const void *A, dp_dtyp
   DP_TRY(st);
   if (p.parts > 1) {
     const size_t n = (size_t)M * N;
-    size_t grid = (n + 255) / 256;
+    const int wide = n % 4 == 0 && !(((uintptr_t)final_dst | (uintptr_t)residual) & 15);
+    size_t grid = ((wide ? n / 4 : n) + 255) / 256;
     if (grid > (size_t)ctx->sm_count * 8) grid = (size_t)ctx->sm_count * 8;
     const float *parts = (const float *)dst;
-    if (c_dtype == DP_F32) DP_LAUNCH(ctx, int_reduce_kernel<float>, (unsigned)grid, 256, 0, parts, (float *)final_dst, n, p.parts, residual);
-    else DP_LAUNCH(ctx, int_reduce_kernel<__half>, (unsigned)grid, 256, 0, parts, (__half *)final_dst, n, p.parts, residual);
+    if (c_dtype == DP_F32) DP_LAUNCH(ctx, int_reduce_kernel<float>, (unsigned)grid, 256, 0, parts, (float *)final_dst, n, p.parts, residual, wide);
+    else DP_LAUNCH(ctx, int_reduce_kernel<__half>, (unsigned)grid, 256, 0, parts, (__half *)final_dst, n, p.parts, residual, wide);
   }
   if (guard) {  // its launch prepared while the kernel before it runs: it has nothing to do as a rule
     const bool pdl = ctx->pdl;
