@@ -286,6 +286,17 @@ def test_large_sizes_bf16(dev, name):
     m.destroy()
 
 
+@pytest.mark.parametrize("width,groups,streams,taps,n", [(2048, 1, 3, 3, 1200), (1024, 2, 4, 4, 2500), (512, 1, 2, 1, 4800)])
+def test_boundaries_of_many_rows_f32(dev, width, groups, streams, taps, n):
+    """Portions whose rows stay in a block's registers between two sublayers, the second behind the first one's last rows."""
+    cfg = config([attention(heads=2, kv_heads=1, dim=16, vdim=16, chunk=20, mlp=None), mamba(heads=2, vdim=16, state=16, groups=1, norm_groups=1)],
+                 width=width, groups=groups, streams=streams, taps=taps)
+    w, t, logits, _ = oracle(f"boundaries {width}", cfg, n + 1100)
+    m = build(dev, cfg, w, n + 1100, max_rows=n)  # (one pass each)
+    check(np.concatenate([m.extend(t[:n], range(n)), m.extend(t[n:], range(1100))]), logits, F32_TOL)
+    m.destroy()
+
+
 def test_attention_rows_f32(dev):
     """Prompts long enough for the query-tiled kernel over an f32 cache, values shorter than keys, in one portion and in two."""
     cfg, n = config([attention(heads=12, kv_heads=2, dim=72, vdim=56, scale=0.2, chunk=170)], width=128), 333
