@@ -4,7 +4,8 @@
 // HBM-bound: the table (262 MB at 32000 x 4096) is streamed once for all rows, where the one-row kernel streams it once per
 // row.  32 rows at 32000 x 4096: 103 us; with that kernel 32 x 42 us and as many copies to the host between them.  A CTA of
 // eight warps owns 128 table rows; the weights are the A operand of mma.sync m16n8k16 straight from global memory (16-byte
-// loads, K permuted to fit them as in gemm_f16w_rows.cu).  The normed rows enter as three bf16 terms that add up to their
+// loads; K is permuted to fit them: a lane's eight values at 32 c + 8 t feed two MMAs, four as its k of the first, four of
+// the second, the B fragments likewise).  The normed rows enter as three bf16 terms that add up to their
 // 24 bits, so every product is the f32 one; the products of a 64-wide slice of K are summed in a fragment of their own and
 // added to the result with f32 additions, so that the tensor core's accumulation is never longer than twelve steps.
 #include "layers.h"
