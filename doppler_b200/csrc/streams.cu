@@ -208,14 +208,16 @@ __global__ void __launch_bounds__(SB_THREADS, 2) stream_boundary_kernel(const Bo
 // the next row's loads go out before this row's sum over the group, one barrier a row.  Bound: HBM (x read and written, y, the
 // sublayer's input: 318 MB at 2048 rows x 4 streams x 4096).  The kernel above holds a block of rows in shared memory, loads, waits and
 // convolves in turn and reads 3 rows more for every 15: 91 us there, 56 here.
+// A group's squares are summed in the order of the kernel above, lane l over the channels 4 l + 128 k, by every warp for itself
+// out of shared memory: a row is the same bits whichever of the two it goes through, however a prompt is cut.
 template <int SM, typename OutT>
 __global__ void __launch_bounds__(512) stream_rows_kernel(const BoundaryArgs a, OutT *__restrict__ dst) {
   pdl_launch();
   pdl_wait();
   constexpr int TAPS = 4;
-  __shared__ float red[2][16];
+  extern __shared__ float sb_h[];  // u of this row and the row before, [2][gs]
   const int S = a.streams, H = a.width, gs = H / a.next.groups, taps = a.next.taps, halo = taps > 1 ? taps - 1 : 0;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31;
   const int c = blockIdx.y * gs + threadIdx.x * 4, row0 = blockIdx.x * a.block_rows, end = min(row0 + a.block_rows, a.rows);
   const bool has_y = a.y != nullptr;
   float mix[SM][SM], out[SM], in[SM];
@@ -274,17 +276,19 @@ __global__ void __launch_bounds__(512) stream_rows_kernel(const BoundaryArgs a, 
         for (int i = 0; i < 4; i++) u.v[i] = fmaf(in[s], x[s].v[i], u.v[i]);
     }
     if (row + 1 < end) load(row + 1);
+    float *row_u = sb_h + turn * gs;
+    stv<4>(row_u + threadIdx.x * 4, u);
+    __syncthreads();  // (the other turn's row is read by all before anyone gets to the barrier that follows this one)
     float ss = 0.0f;
+#pragma unroll 4
+    for (int k = lane * 4; k < gs; k += 128) {
+      const FV<4> v = ldv<4>(row_u + k);
 #pragma unroll
-    for (int i = 0; i < 4; i++) ss = fmaf(u.v[i], u.v[i], ss);
+      for (int i = 0; i < 4; i++) ss = fmaf(v.v[i], v.v[i], ss);
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if (lane == 0) red[turn][warp] = ss;
-    __syncthreads();  // (the other turn's sums are read by all before anyone gets to the barrier that follows this one)
-    float total = lane < warps ? red[turn][lane] : 0.0f;
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-    const float inv = 1.0f / sqrtf(__shfl_sync(0xffffffffu, total, 0) / (float)gs + a.next.eps);
+    const float inv = 1.0f / sqrtf(ss / (float)gs + a.next.eps);
     FV<4> h, o;
 #pragma unroll
     for (int i = 0; i < 4; i++) h.v[i] = u.v[i] * inv * norm.v[i];
@@ -649,8 +653,8 @@ dp_status dpk_stream_boundary(dp_ctx *ctx, const float *x, float *x_out, const f
       a.x = x; a.y = y; a.x_out = x_out; a.end = end; a.next = next;
       a.streams = streams; a.width = width; a.rows = rows; a.dst_stride = dst_stride; a.block_rows = (int)R; a.map = map;
       const dim3 grid((unsigned)((rows + R - 1) / R), next.groups);
-      if (dst_bf16) DP_LAUNCH(ctx, (stream_rows_kernel<4, __nv_bfloat16>), grid, gs / 4, 0, a, (__nv_bfloat16 *)dst);
-      else DP_LAUNCH(ctx, (stream_rows_kernel<4, float>), grid, gs / 4, 0, a, (float *)dst);
+      if (dst_bf16) DP_LAUNCH(ctx, (stream_rows_kernel<4, __nv_bfloat16>), grid, gs / 4, (size_t)gs * 8, a, (__nv_bfloat16 *)dst);
+      else DP_LAUNCH(ctx, (stream_rows_kernel<4, float>), grid, gs / 4, (size_t)gs * 8, a, (float *)dst);
       return DP_OK;
     }
   }

@@ -297,6 +297,20 @@ def test_boundaries_of_many_rows_f32(dev, width, groups, streams, taps, n):
     m.destroy()
 
 
+@pytest.mark.parametrize("width,groups,streams,taps,n", [(2048, 1, 3, 3, 1200), (1024, 2, 4, 4, 2500), (512, 1, 2, 1, 4800)])
+def test_boundaries_do_not_depend_on_the_passes(dev, width, groups, streams, taps, n):
+    """One pass of many rows and passes of few go through two kernels between the sublayers, which sum a norm group's squares in the
+    same order: everything behind them is the same bits."""
+    layer = dict(heads=2, kv_heads=1, dim=128, vdim=128, chunk=10000, mlp=None)
+    cfg = config([attention(**layer), attention(**layer)], width=width, groups=groups, streams=streams, taps=taps)
+    w, t, got = weights(cfg), tokens(cfg, n), []
+    for max_rows in (n, 500):
+        m = build(dev, cfg, w, n, dtype="bfloat16", max_rows=max_rows)
+        got.append((m.extend(t, [n - 1]), m.read_hidden((n - 1) % max_rows + 1)[-100:]))
+        m.destroy()
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+
+
 def test_attention_rows_f32(dev):
     """Prompts long enough for the query-tiled kernel over an f32 cache, values shorter than keys, in one portion and in two."""
     cfg, n = config([attention(heads=12, kv_heads=2, dim=72, vdim=56, scale=0.2, chunk=170)], width=128), 333
