@@ -21,6 +21,7 @@
 #include "layers.h"
 #include "decay.cuh"
 #include "pdl.cuh"
+#include "tiles.h"
 #include "umma.cuh"
 
 #include <cstring>
@@ -227,28 +228,6 @@ GluArgs glu_args(const GluOut *g) {
   return a;
 }
 
-// Activation rows per tile, and whether two SMs share one: the least estimated time in cycles.  A K step takes its MMAs (two
-// cycles per activation row) or what it fetches from L2, at some 44 bytes a cycle and SM.
-struct TilePick {
-  int bn;
-  bool pair;
-};
-TilePick pick_tile(dp_ctx *ctx, int M, int N, int ksteps, bool may_pair) {
-  TilePick best = {16, false};
-  double best_cost = -1.0;
-  for (int pair = 0; pair <= (may_pair ? 1 : 0); pair++)
-    for (int bn = 16; bn <= 256; bn += 16) {
-      const long tiles = (long)((N + (pair ? 255 : 127)) / (pair ? 256 : 128)) * ((M + bn - 1) / bn), owners = pair ? ctx->sm_count / 2 : ctx->sm_count;
-      const long waves = (tiles + owners - 1) / owners;
-      const double fetch = (16384.0 + 128.0 * (pair ? bn / 2 : bn)) / 44.0, step = fetch > 2.0 * bn ? fetch : 2.0 * bn;
-      // (a pair's advantage counts by less than its bytes: it gains 8 % on the largest products, and loses 3 to 8 % on those of a few
-      // microseconds, 301 -> 311 us for 1500 tokens at width 1024)
-      const double cost = ((double)waves * (ksteps * step + 1500.0) + 12.0 * bn) * (pair ? 1.3 : 1.0);
-      if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = {bn, pair != 0}; }
-    }
-  return best;
-}
-
 // shape, strides and outputs are in `a`; the rest is chosen here
 dp_status launch_tc(dp_ctx *ctx, const void *W, int w_stride, const void *A, int a_stride, TcArgs a) {
   const int M = a.M, N = a.N, K = a.K;
@@ -256,7 +235,7 @@ dp_status launch_tc(dp_ctx *ctx, const void *W, int w_stride, const void *A, int
   EncodeTiledFn encode = get_encode();
   if (!encode) return dp_fail(ctx, DP_ERR_CUDA, "gemm (bf16): cuTensorMapEncodeTiled is not available");
   // (in a decode step's graph kernels launch their dependents early; those keep to launches without clusters)
-  const TilePick pick = pick_tile(ctx, M, N, (K + BK - 1) / BK, !ctx->pdl && ctx->sm_count >= 2);
+  const TilePick pick = pick_tile(ctx->sm_count, M, N, (K + BK - 1) / BK, !ctx->pdl && ctx->sm_count >= 2);
   a.bn = pick.bn;
   a.tiles_n = (N + (pick.pair ? 255 : 127)) / (pick.pair ? 256 : 128);
   a.tiles_m = (M + a.bn - 1) / a.bn;

@@ -1,0 +1,16 @@
+"""Sizes that the tensor-core kernels ask of an MMA, over the ranges their callers have."""
+import random
+
+from tiles_rule import pick
+
+
+def test_16_bit_products_ask_for_widths_that_exist():
+    """One CTA (128 features): 16 to 256 columns in steps of 16; two (256 features): 32 to 256 in steps of 32."""
+    rng, widths = random.Random(1), {True: set(), False: set()}
+    for _ in range(20000):
+        m, n, k = rng.randint(2, 4096), rng.randint(16, 32768), rng.choice([24, 64, 256, 768, 1024, 4096, 12288])
+        bn, pair = pick(m, n, k, sms=rng.choice([148, 132, 2]))
+        widths[pair].add(bn)
+        assert bn % (32 if pair else 16) == 0 and 16 <= bn <= 256, (m, n, k, bn, pair)
+        assert not pick(m, n, k, may_pair=False)[1]
+    assert {160, 192, 224, 256} <= widths[True]  # (the widths that tests of pairs have to reach)
