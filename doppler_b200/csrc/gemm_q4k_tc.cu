@@ -25,6 +25,7 @@
 #include "mbar.cuh"
 #include "pdl.cuh"
 #include "q4k.cuh"
+#include "tiles.h"
 #include "umma.cuh"
 
 #include <cuda.h>
@@ -370,9 +371,9 @@ __global__ void __launch_bounds__((DQ_WARPS + 2) * 32, 1) gemm_q4k_tc_kernel(con
 // read from shared memory once per pair.  Two passes (rows 0..255 and 256..511 of the tile) share each
 // B stage.  CTA 0 issues all MMAs; all "stage full" barriers live in CTA 0 (CTA 1's TMA and dequant
 // warps signal them across the cluster), "stage free" and "accumulators ready" are multicast to both.
-// The tile width is a run-time value (a multiple of 16 up to BNMAX): the first `wide_tiles` clusters of a
-// grid row take `bn_wide` columns, the others `bn_narrow`.  With 28 tiles of 176 and 46 of 160 columns the
-// 74 clusters of a B200 cover N = 12288 in one even wave, where uniform 256-wide tiles fill only 48.
+// The tile width is a run-time value (a multiple of 32 up to BNMAX): the first `wide_tiles` clusters of a
+// grid row take `bn_wide` columns, the others `bn_narrow`.  With 14 tiles of 192 and 60 of 160 columns the
+// 74 clusters of a B200 cover N = 12288 in one wave, where uniform 256-wide tiles fill only 48.
 // PS = passes: 256-row MMAs per pair tile (output tile 256*PS x bn).  One pass halves the activation bytes
 // per stage, which buys twice as many stages for the same shared memory.
 template <int BNMAX, typename OutT, int SA, int SB, int CH, int PS, int NPROD = 1>
@@ -835,8 +836,8 @@ dp_status dispatch_tc(dp_ctx *ctx, int bn, const CUtensorMap &tm, const uint8_t 
   // faster per SM.  It needs whole waves of 74 clusters to win (at M = 512, 48 uniform tiles of 256 columns
   // occupy 96 SMs), so the tiles are sized to the waves: with R = ceil(M / 512) rows of pair tiles, take the
   // fewest waves of 74 clusters that 256-wide tiles need, then as many column tiles per row as those waves
-  // hold, in two widths 16 apart.  N = 12288: M = 512 runs one wave of 28 x 176 + 46 x 160 columns; M = 2048
-  // three waves of 55 tiles (53 x 224 + 2 x 208).  Tiles narrower than 128 columns are left to the one-SM
+  // hold, in two widths 32 apart (tiles.h).  N = 12288: M = 512 runs one wave of 14 x 192 + 60 x 160 columns; M = 2048
+  // three waves of 55 tiles (54 x 224 + 1 x 192).  Tiles narrower than 128 columns are left to the one-SM
   // kernel (every SM re-reads its activation rows once per tile column, so narrow tiles are bound by L2).
   // Measurements of the alternatives that were tried and dropped: profiles/gemm_q4k_tc__config1.md.
   if (M > 256 && alpha.k_splits > 1 && N % 256 == 0) {  // few pair tiles: uniform 256-wide tiles, several clusters per tile along K
@@ -844,23 +845,16 @@ dp_status dispatch_tc(dp_ctx *ctx, int bn, const CUtensorMap &tm, const uint8_t 
     if constexpr (NPROD == 1) return launch_tc_2sm<OutT, 256, 3, 4, 2, 2, 1>(ctx, tm, W, C, M, N, K, alpha, cols, 0, 256, 256);
     else return launch_tc_2sm<OutT, 256, 3, 4, 2, 2, 2>(ctx, tm, W, C, M, N, K, alpha, cols, 0, 256, 256);
   }
-  if (M > 256 && N % 16 == 0) {
-    const int clusters = ctx->sm_count / 2, rows = (M + 511) / 512;
-    const int waves = (rows * ((N + 255) / 256) + clusters - 1) / clusters;
-    int cols = waves * clusters / rows;
-    if (cols > N / 96) cols = N / 96;
-    if (cols > 0) {
-      const int narrow = (N / 16 / cols) * 16;
-      const int n_wide = (N - cols * narrow) / 16;  // cols * narrow + 16 * n_wide == N, n_wide < cols
-      const int wide = narrow + 16, widest = n_wide ? wide : narrow;
-      if (narrow >= 128 && widest <= 192) {
-        if constexpr (NPROD == 1) return launch_tc_2sm<OutT, 192, 4, 8, 4, 2, 1>(ctx, tm, W, C, M, N, K, alpha, cols, n_wide, wide, narrow);
-        else return launch_tc_2sm<OutT, 192, 3, 4, 2, 2, 2>(ctx, tm, W, C, M, N, K, alpha, cols, n_wide, wide, narrow);
-      }
-      if (narrow >= 128 && widest <= 256) {
-        if constexpr (NPROD == 1) return launch_tc_2sm<OutT, 256, 3, 4, 2, 2, 1>(ctx, tm, W, C, M, N, K, alpha, cols, n_wide, wide, narrow);
-        else return launch_tc_2sm<OutT, 256, 3, 4, 2, 2, 2>(ctx, tm, W, C, M, N, K, alpha, cols, n_wide, wide, narrow);
-      }
+  if (M > 256) {
+    const PairColumns p = pair_columns(ctx->sm_count, M, N);
+    const int widest = p.wide_tiles ? p.wide : p.narrow;
+    if (p.cols && widest <= 192) {
+      if constexpr (NPROD == 1) return launch_tc_2sm<OutT, 192, 4, 8, 4, 2, 1>(ctx, tm, W, C, M, N, K, alpha, p.cols, p.wide_tiles, p.wide, p.narrow);
+      else return launch_tc_2sm<OutT, 192, 3, 4, 2, 2, 2>(ctx, tm, W, C, M, N, K, alpha, p.cols, p.wide_tiles, p.wide, p.narrow);
+    }
+    if (p.cols && widest <= 256) {
+      if constexpr (NPROD == 1) return launch_tc_2sm<OutT, 256, 3, 4, 2, 2, 1>(ctx, tm, W, C, M, N, K, alpha, p.cols, p.wide_tiles, p.wide, p.narrow);
+      else return launch_tc_2sm<OutT, 256, 3, 4, 2, 2, 2>(ctx, tm, W, C, M, N, K, alpha, p.cols, p.wide_tiles, p.wide, p.narrow);
     }
   }
   // one-SM kernel; up to 128 rows (batched decode steps) one 128-row accumulator per CTA, else two

@@ -28,3 +28,21 @@ inline TilePick pick_tile(int sm_count, int M, int N, int ksteps, bool may_pair)
   }
   return best;
 }
+
+// gemm_q4k_tc2_kernel (gemm_q4k_tc.cu): column tiles of a grid row of 512 activation rows, the first `wide_tiles` of them `wide`
+// columns, the others `narrow`: as many as fit the fewest waves of clusters that 256-wide tiles need.  Tiles of less than 128 columns
+// are not taken (cols == 0).
+struct PairColumns {
+  int cols, wide_tiles, wide, narrow;
+};
+inline PairColumns pair_columns(int sm_count, int M, int N) {
+  const int clusters = sm_count / 2, rows = (M + 511) / 512;
+  if (N % PAIR_STEP || clusters < 1) return {0, 0, 0, 0};
+  const int waves = (rows * ((N + 255) / 256) + clusters - 1) / clusters;
+  int cols = waves * clusters / rows;
+  if (cols > N / 96) cols = N / 96;
+  if (cols < 1) return {0, 0, 0, 0};
+  const int narrow = N / PAIR_STEP / cols * PAIR_STEP;
+  if (narrow < 128) return {0, 0, 0, 0};
+  return {cols, (N - cols * narrow) / PAIR_STEP, narrow + PAIR_STEP, narrow};  // cols * narrow + PAIR_STEP * wide_tiles == N, wide_tiles < cols
+}
