@@ -925,7 +925,9 @@ static dp_status gemm_q4k_tc_impl(dp_ctx *ctx, const uint8_t *W, const void *A, 
   //             180, 1024 x 6144 x 4096 115 -> 105, 2048 x 4096 x 4096 155 -> 135, 2048 x 24576 x 4096 763 -> 614, 2048 x 3072 x 1024 45 -> 46
   //   f16 rows  384 x 6144 x 4096 40 -> 40, 512 x 12288 x 4096 80 -> 70, 512 x 4096 x 12288 221 -> 156, 2048 x 24576 x 4096 502 -> 398
   // The two products stay for f16 rows where the pass over the rows and a unit's fixed cost weigh more: K up to 1024 with more than half a
-  // wave of the others' 512 x 256 pair tiles (2048 x 3072 x 1024 27 -> 37), and very small weights (32 x 256 x 1024 16 -> 18).
+  // wave of the others' 512 x 256 pair tiles (2048 x 3072 x 1024 27 -> 37), and, but for up to 64 rows with an f32 result, weights of less
+  // than 2^19 values.  Those few rows always had exact weights (a residue in f16 loses bits, 2e-6 against 4e-7, and a weight beyond f16's
+  // range is NaN there), and nothing rounds their result.
   // Shapes the others do not tile ran on CUDA cores (1000 x 1000 x 1000: f32 rows 105 -> 30, f16 rows 102 -> 27 us); they still do where
   // that is over within about 15 us, where the result is f32 and K below 640 (error of the f32 FMAs 4.1e-7 at K = 512, of the integer
   // tiles 4.8e-7; 5.7e-7 and 4.6e-7 at 1024), and with an alpha that a row's scale might carry out of f32's range.
@@ -934,7 +936,8 @@ static dp_status gemm_q4k_tc_impl(dp_ctx *ctx, const uint8_t *W, const void *A, 
     const bool few = M <= 256 || pair_tiles * 2 <= ctx->sm_count / 2;
     const float size = fabsf(alpha);
     const bool whole = (double)M * N * K >= (double)(1l << 27) && (K >= 640 || c_dtype == DP_F16) && (size == 0.0f || (size >= 0x1p-60f && size <= 0x1p60f));
-    const bool take = tiled ? a_dtype == DP_F32 || ((few || K > 1024) && (long)N * K >= (1l << 19)) : whole;
+    const bool small = (long)N * K < (1l << 19), rows64 = M <= 64 && c_dtype == DP_F32;
+    const bool take = tiled ? a_dtype == DP_F32 || rows64 || ((few || K > 1024) && !small) : whole;
     if (take) {
       DP_TRY(dpk_gemm_q4k_int(ctx, W, A, a_dtype, C, c_dtype, M, N, K, alpha, handled, fuse));
       if (*handled) return DP_OK;

@@ -68,9 +68,10 @@ def test_edges(dev, m, n, k, act, out):
 
 @pytest.mark.parametrize("act,out", [("f32", "f32"), ("f16", "f32")])
 @pytest.mark.parametrize("m,n,k", [(2, 2048, 256), (3, 384, 1536), (16, 1024, 768), (17, 512, 1280), (31, 4096, 1792), (32, 256, 2048), (33, 640, 2304), (48, 128, 4352), (64, 1024, 6400),
-                                   (64, 4096, 12288), (600, 2048, 1792), (2000, 1024, 2560)])
+                                   (64, 4096, 12288), (600, 2048, 1792), (2000, 1024, 2560), (2, 256, 256), (17, 128, 512), (32, 256, 1024), (64, 384, 1280)])
 def test_few_rows_and_sum_units(dev, m, n, k, act, out):
-    """From two rows on, every tile width; sum units of one to eight super-blocks, even and odd, in both orders of the products."""
+    """From two rows on, every tile width; sum units of one to eight super-blocks, even and odd, in both orders of the products; small
+    weights, whose f16 rows have exact weights too (some are beyond f16's range here)."""
     test_edges(dev, m, n, k, act, out)
 
 
