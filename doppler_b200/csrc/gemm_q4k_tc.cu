@@ -916,7 +916,9 @@ static dp_status gemm_q4k_tc_impl(dp_ctx *ctx, const uint8_t *W, const void *A, 
   if (fuse && fuse->norm_w && !(row_scaled && a_dtype == DP_F32 && c_dtype == DP_F32 && K % 4 == 0 && K >= 1024 && K <= 4096 &&
                                  ((uintptr_t)fuse->norm_w & 15) == 0 && ((uintptr_t)A & 15) == 0))
     return DP_OK;
-  if (M < 2 || (M < 32 && !tiled)) return DP_OK;  // one row, or few on a shape that is not tiled: the CUDA-core kernels
+  // one row, or few on a shape that is not tiled: the CUDA-core kernels; few f32 rows of mode 1 too: a batch's decode steps stay exact
+  // under the switch that rounds prompts
+  if (M < 2 || (M < 32 && (!tiled || mode == 1))) return DP_OK;
   // Exact weights: the integer-tile kernel (gemm_q4k_int.cu), whatever the size: one product less per K step than the tiles of
   // dequantised weights below, 4 to 20 times less error (f32 rows 3.7e-6 to 2.2e-5 -> 9e-7, f16 rows 4e-7), and weights beyond
   // f16's range.  A whole call, us, what ran before (two products for f16 rows, three for f32 rows; up to 64 f32 rows a kernel of their

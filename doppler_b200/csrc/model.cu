@@ -726,7 +726,8 @@ static dp_status q4k_linear(dp_model *m, const uint8_t *W, const float *x, float
   // product (the reference's rule for f32 activations, matmul.rules.json:15-22), with integer weight tiles and the rows
   // as two f16 halves (gemm_q4k_int.cu).  DP_PREFILL_TC=1: one pass, activations and weights rounded to f16 as in the
   // reference's tiled f16 prefill kernel (fused_matmul_q4_prefill_tiled_f16.wgsl), about 1e-3 of the output's rms away from the
-  // exact product; DP_PREFILL_TC=0 and few rows of shapes that are not tiled: the f32-exact CUDA-core kernel.
+  // exact product, from 32 rows on (fewer are steps of a batch and stay exact); DP_PREFILL_TC=0 and few rows of shapes that are not
+  // tiled: the f32-exact CUDA-core kernel.
   static int prefill_tc = -1;
   if (prefill_tc < 0) { const char *e = getenv("DP_PREFILL_TC"); prefill_tc = e ? atoi(e) : 3; }
   bool handled = false;
