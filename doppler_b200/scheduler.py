@@ -42,10 +42,10 @@ class Scheduler:
         if any(w < 0 or w >= len(tokens) for w in want):
             raise ValueError("a wanted place lies outside the tokens")
         if len(tokens) == 1 and s == 0 and len(self.slots) == 1:
-            if hasattr(self.model, "advance") and self.model.tp_size == 1:
-                self.model.advance(tokens[0])  # (the logits only where they are wanted)
+            if not want and hasattr(self.model, "advance") and self.model.tp_size == 1:
+                self.model.advance(tokens[0])  # (leaves the table's product out)
             else:
-                self.model.decode([tokens[0]], 1)
+                self.model.decode([tokens[0]], 1)  # (the table's product in the step's graph)
             rows = self.model.read_logits(self.model.cfg["vocab"]).reshape(1, -1) if want else np.empty((0, self.model.cfg["vocab"]), np.float32)
             return rows[want] if want else rows
         order = sorted(set(want))

@@ -1,0 +1,58 @@
+"""Which call of a runner a scheduler's step becomes."""
+import numpy as np
+import pytest
+
+from doppler_b200.scheduler import Scheduler
+
+
+class Runner:
+    max_batch, tp_size = 2, 1
+
+    def __init__(self):
+        self.cfg, self.calls = {"vocab": 5, "max_seq": 64}, []
+
+    def release(self, seq):
+        pass
+
+    def extend(self, tokens, want=(), seq=0):
+        self.calls.append(("extend", len(tokens), seq))
+        return np.zeros((len(want), 5), np.float32)
+
+    def decode(self, tokens, steps):
+        self.calls.append(("decode", tuple(tokens), steps))
+        return np.zeros((steps, 1), np.int32)
+
+    def advance(self, token):
+        self.calls.append(("advance", token))
+
+    def read_logits(self, n):
+        self.calls.append(("read_logits", n))
+        return np.arange(n, dtype=np.float32)
+
+
+class Sharded(Runner):
+    tp_size = 2
+
+
+class Plain(Runner):
+    advance = property()
+
+
+@pytest.mark.parametrize("runner", [Runner, Sharded, Plain])
+def test_one_token_of_the_only_sequence(runner):
+    """With its logits the whole step is one graph and the logits are read; without them, on one GPU, the table is left out."""
+    m = runner()
+    s = Scheduler(m)
+    assert np.array_equal(s.step("a", [3], [0, 0]), np.arange(5, dtype=np.float32) * np.ones((2, 1)))
+    assert m.calls == [("decode", (3,), 1), ("read_logits", 5)]
+    assert s.step("a", [4]).shape == (0, 5)
+    assert m.calls[2:] == [("advance", 4) if runner is Runner else ("decode", (4,), 1)]
+
+
+def test_everything_else_is_a_portion():
+    m = Runner()
+    s = Scheduler(m)
+    s.step("a", [1, 2], [1])
+    s.step("b", [3])
+    s.step("a", [4], [0])
+    assert m.calls == [("extend", 2, 0), ("extend", 1, 1), ("extend", 1, 0)]
