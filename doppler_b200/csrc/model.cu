@@ -565,7 +565,7 @@ extern "C" void dp_model_destroy(dp_model *m) {
   dp_stack_destroy(m);
   auto rel = [&](dp_buf b) { if (b) dp_buf_release(ctx, b); };
   for (LayerW &L : m->layers) { rel(L.qkv); rel(L.o); rel(L.gateup); rel(L.down); }
-  rel(m->norms); rel(m->embed); rel(m->lm_head); rel(m->rope); rel(m->act); rel(m->state); rel(m->logits_buf); rel(m->out_tokens); rel(m->attn_scratch); rel(m->actq);
+  rel(m->norms); rel(m->embed); rel(m->lm_head); rel(m->rope); rel(m->act); rel(m->state); rel(m->logits_buf); rel(m->out_tokens); rel(m->attn_scratch); rel(m->actq); rel(m->head_kept);
   for (dp_buf b : m->kc) rel(b);
   for (dp_buf b : m->vc) rel(b);
   if (m->pin_state) cudaFreeHost(m->pin_state);
@@ -647,6 +647,7 @@ extern "C" dp_status dp_model_load_final_norm(dp_model *m, const float *host, in
   if (!m || !host) return DP_ERR_INVALID;
   DP_CHECK(m->ctx, !m->stack, "loadFinalNorm: a decoder described layer by layer takes dp_model_load_tensor");
   DP_CHECK(m->ctx, n == m->cfg.hidden, "loadFinalNorm: expected %d values, got %d", m->cfg.hidden, n);
+  DP_TRY(dp_model_head(m));
   return dp_buf_upload(m->ctx, m->norms, host, (size_t)((char *)m->final_norm - (char *)m->norms->dptr), (size_t)n * 4);
 }
 
@@ -666,6 +667,7 @@ extern "C" dp_status dp_model_load_lm_head(dp_model *m, const void *host, int ro
   int hi = row0 + rows < m->vocab0 + m->vocab_l ? row0 + rows : m->vocab0 + m->vocab_l;
   if (hi <= lo) return DP_OK;
   const size_t rb = (size_t)m->cfg.hidden * 2;
+  DP_TRY(dp_model_head(m));
   return dp_buf_upload(m->ctx, m->lm_head, (const char *)host + (size_t)(lo - row0) * rb, (size_t)(lo - m->vocab0) * rb, (size_t)(hi - lo) * rb);
 }
 
@@ -1100,11 +1102,20 @@ static dp_status wanted_rows(dp_model *m, const char *op, const int32_t *want, i
   return DP_OK;
 }
 
-// Before a pass overwrites the hidden row of a step without logits: its logits, unless the pass has logits of its own
-static dp_status settle_head(dp_model *m, bool replaced) {
-  if (!m->head_pending) return DP_OK;
-  m->head_pending = false;
-  return replaced ? DP_OK : run_logits(m, m->h, 1);
+dp_status dp_model_head(dp_model *m) {
+  const float *row = m->head_row;
+  m->head_row = nullptr;
+  return row ? run_logits(m, row, 1) : DP_OK;
+}
+
+// Before a pass overwrites the hidden row of a step without logits: the row moves, unless the pass has logits of its own.  (Portions
+// without wanted places may follow; whoever reads logits behind them gets the last that there were.)
+static dp_status keep_head_row(dp_model *m, bool replaced) {
+  if (replaced) m->head_row = nullptr;
+  if (!m->head_row || m->head_row == (const float *)m->head_kept->dptr) return DP_OK;
+  DP_CUDA(m->ctx, cudaMemcpyAsync(m->head_kept->dptr, m->head_row, (size_t)m->cfg.hidden * 4, cudaMemcpyDeviceToDevice, m->ctx->stream));
+  m->head_row = (const float *)m->head_kept->dptr;
+  return DP_OK;
 }
 
 // One portion of a sequence: `n` tokens that follow what the sequence holds already, in blocks of at most m->T rows.
@@ -1121,7 +1132,7 @@ static dp_status run_portion(dp_model *m, const char *op, int seq, const int32_t
   for (int i = 0; i < n_want; i++)
     DP_CHECK(ctx, want[i] >= 0 && want[i] < n && (i == 0 || want[i] > want[i - 1]), "%s: wanted place %d is not an ascending place among the %d tokens", op, want[i], n);
   if (m->stack) DP_TRY(dp_stack_ready(m));
-  DP_TRY(settle_head(m, n_want > 0 || next_token));
+  DP_TRY(keep_head_row(m, n_want > 0 || next_token));
   dp_buf ids = nullptr;
   DP_TRY(dp_buf_acquire(ctx, (size_t)m->T * 4, "prefill_token_ids", &ids));
   dp_status st = DP_OK;
@@ -1200,7 +1211,7 @@ static dp_status run_packed(dp_model *m, const int32_t *seqs, const int32_t *con
   DP_TRY(dp_buf_acquire(ctx, host.size() * 4, "packed_rows", &buf));
   const int *dev = (const int *)buf->dptr;
   const PackedRows packed = {dev + rows, dev + 2 * rows, (const int4 *)(dev + spans_at), n, longest};
-  m->head_pending = false;  // its logits are replaced
+  m->head_row = nullptr;  // its logits are replaced
   auto run = [&]() -> dp_status {
     DP_TRY(dp_buf_upload(ctx, buf, host.data(), 0, host.size() * 4));
     DP_TRY(embed_rows(m, dev, rows, false));
@@ -1313,7 +1324,7 @@ extern "C" dp_status dp_model_decode(dp_model *m, int batch, const int32_t *firs
     DP_CHECK(ctx, m->seq_len[b] + steps <= c.max_seq, "decode: sequence %d would exceed max_seq %d", b, c.max_seq);
   }
   if (m->stack) DP_TRY(dp_stack_ready(m));
-  m->head_pending = false;  // its logits are replaced
+  m->head_row = nullptr;  // its logits are replaced
   if (m->out_tokens_cap < steps * batch) {
     if (m->out_tokens) { dp_buf_release(ctx, m->out_tokens); m->out_tokens = nullptr; }
     if (m->graph[0]) { dp_graph_destroy(m->graph[0]); m->graph[0] = nullptr; }
@@ -1376,6 +1387,7 @@ extern "C" dp_status dp_model_advance(dp_model *m, int32_t token) {
   st[0] = m->seq_len[0]; st[256] = m->seq_len[0] + 1; st[512] = token;
   DP_CUDA(ctx, cudaMemcpyAsync(m->state->dptr, st, 4096, cudaMemcpyHostToDevice, ctx->stream));
   if (!m->graph[1]) {
+    if (!m->head_kept) DP_TRY(dp_buf_acquire(ctx, (size_t)c.hidden * 4, "kept_hidden_row", &m->head_kept));
     dp_recorder *rec = nullptr;
     DP_TRY(dp_recorder_begin(ctx, "step_without_logits", 1, &rec));
     ctx->pdl = getenv("DP_PDL") ? atoi(getenv("DP_PDL")) != 0 : true;
@@ -1394,6 +1406,7 @@ extern "C" dp_status dp_model_advance(dp_model *m, int32_t token) {
   }
   DP_CUDA(ctx, cudaEventRecord(m->ev0, ctx->stream));
   DP_TRY(dp_graph_launch(m->graph[1]));
+  m->head_row = nullptr;  // overwritten; the new one counts once the step is known to be whole
   DP_CUDA(ctx, cudaEventRecord(m->ev1, ctx->stream));
   DP_CUDA(ctx, cudaMemcpyAsync(st + 1024, ctx->dev_status, 4, cudaMemcpyDeviceToHost, ctx->stream));
   DP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -1402,7 +1415,7 @@ extern "C" dp_status dp_model_advance(dp_model *m, int32_t token) {
   m->last_ms = ms;
   m->h_last = m->h;
   if (st[1024]) DP_TRY(dp_take_dev_status(ctx));
-  m->head_pending = true;
+  m->head_row = m->h;
   m->seq_len[0] += 1;
   return DP_OK;
 }
@@ -1410,7 +1423,7 @@ extern "C" dp_status dp_model_advance(dp_model *m, int32_t token) {
 extern "C" dp_status dp_model_read_logits(dp_model *m, float *host, int n) {
   if (!m || !host) return DP_ERR_INVALID;
   DP_CHECK(m->ctx, n > 0 && n <= m->cfg.max_batch * m->vocab_l, "readLogits: %d values requested, %d available", n, m->cfg.max_batch * m->vocab_l);
-  DP_TRY(settle_head(m, false));
+  DP_TRY(dp_model_head(m));
   DP_CUDA(m->ctx, cudaMemcpyAsync(host, m->logits, (size_t)n * 4, cudaMemcpyDeviceToHost, m->ctx->stream));
   DP_CUDA(m->ctx, cudaStreamSynchronize(m->ctx->stream));
   return DP_OK;
@@ -1430,7 +1443,7 @@ extern "C" dp_status dp_model_bench_gemv(dp_model *m, int reps, double *ms_total
   const dp_model_cfg &c = m->cfg;
   DP_CHECK(ctx, reps > 0, "bench_gemv: reps must be positive");
   DP_CHECK(ctx, !m->stack, "bench_gemv: the model holds no Q4_K matrices");
-  DP_TRY(settle_head(m, false));
+  DP_TRY(keep_head_row(m, false));
   const int H = c.hidden;
   struct Shape { int N, K; };
   const Shape sh[4] = {{m->qdim + 2 * m->kvdim, H}, {H, m->qdim}, {2 * m->inter, H}, {H, m->inter}};

@@ -58,12 +58,15 @@ struct dp_model {
   size_t weight_bytes = 0;
   int allreduce_mode = 0;
   dp_stack *stack = nullptr;  // a decoder described layer by layer (stack.cu): its weights, sequence state and activations
-  bool head_pending = false;  // the last pass was a step without logits: dp_model_read_logits computes them from m->h
+  const float *head_row = nullptr;  // the last logits to be had are a step's without them: dp_model_read_logits computes them from this hidden row
+  dp_buf head_kept = nullptr;       // ... where it is kept once a pass takes its place
   bool final_norm_done = false;  // set by run_layers when the exchange kernel already applied the final RMSNorm
 };
 
 // model.cu: device state of the decode loop, logits, argmax scratch and events (needs m->cfg, m->vocab_l, m->T)
 dp_status dp_model_alloc_runner(dp_model *m);
+
+dp_status dp_model_head(dp_model *m);  // the logits of head_row, if there is one (before weights change)
 
 // stack.cu
 void dp_stack_destroy(dp_model *m);

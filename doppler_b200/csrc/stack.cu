@@ -910,6 +910,7 @@ extern "C" dp_status dp_model_load_tensor(dp_model *m, int layer, dp_tensor_id i
   };
   const uint64_t bit = (uint64_t)1 << id;
   if (id == DP_T_EMBED || id == DP_T_FINAL_NORM) {
+    DP_TRY(dp_model_head(m));
     if (id == DP_T_EMBED) { DP_TRY(expect(s->cfg.vocab, H)); DP_TRY(mat_upload(ctx, s->embed, 0, host, rows, cols)); }
     else { DP_TRY(expect(1, H)); DP_TRY(upload_raw(ctx, s->final_norm, host, (size_t)H * 2)); }
     s->missing &= ~bit;

@@ -59,7 +59,7 @@ class Runner:
         return out
 
     def advance(self, token: int):
-        """One token of sequence 0 whose logits are not wanted (``read_logits`` still gives them if it is called next)."""
+        """One token of sequence 0 whose logits are not wanted (``read_logits`` still gives them until a pass with logits follows)."""
         self.device.check(self.device.lib.dp_model_advance(self.h, token))
 
     @property

@@ -362,7 +362,7 @@ dp_status dp_model_prefill_many(dp_model *m, int n, const int32_t *seqs, const i
 dp_status dp_model_decode(dp_model *m, int batch, const int32_t *first_tokens, int steps,
                           int32_t *out_tokens);
 /* One token of sequence 0 of a model on one GPU whose logits are not wanted: a decode step without the LM head and the greedy pick.
- * dp_model_read_logits computes them if it is called next. */
+ * dp_model_read_logits computes them if it is called before the next pass with logits. */
 dp_status dp_model_advance(dp_model *m, int32_t token);
 /* A portion of a sequence with logits: the n tokens continue what sequence `seq` holds, only they are run.
  * want: n_want ascending places in [0,n); logits (host) receives [n_want][vocab] in that order.  Nothing is

@@ -4,6 +4,7 @@ import pytest
 
 import fenorax_util as fu
 import virolorn_util as vu
+from doppler_b200 import _lib as L
 from doppler_b200 import synthetic
 from doppler_b200.model import DecoderModel
 from doppler_b200.scheduler import Scheduler
@@ -60,13 +61,14 @@ def test_steps_without_logits(dev, model):
             close(m.read_logits(), want[i])
             close(m.read_logits(), want[i])  # and again
     assert m.seq_len() == len(t)
-    # what overwrites the hidden row first computes the logits that were still to be had, or replaces them
+    # what overwrites the hidden row first puts it aside, or has logits of its own
     rows = []
     for step in (lambda x: m.decode([x], 1), m.advance):
         m.release(0)
         m.extend(t[:6])
         step(t[6])
-        m.extend(t[7:9])
+        m.extend(t[7:8])
+        m.extend(t[8:9])
         rows.append([m.read_logits()])
         step(t[9])
         rows[-1].append(m.extend(t[10:12], [1])[0])
@@ -85,6 +87,29 @@ def test_steps_without_logits(dev, model):
         if len(rows):
             close(rows[0], want[i])
     s.finish("a")
+    m.destroy()
+
+
+@pytest.mark.parametrize("model", [dense, fenorax])
+def test_new_weights_behind_a_step(dev, model):
+    """The logits of a step are those of the weights that it ran with."""
+    m = model(dev)
+    m.extend([1, 2, 3])
+    m.decode([4], 1)
+    want = m.read_logits()
+    for load in range(2):
+        m.release(0)
+        m.extend([1, 2, 3])
+        m.advance(4)
+        if model is dense:
+            rows = np.zeros((m.cfg["vocab"], m.cfg["hidden"]), np.float16)
+            m.load_final_norm(np.zeros(m.cfg["hidden"], np.float32)) if load else m.load_lm_head(rows)
+        else:
+            shape = (m.cfg["hidden"],) if load else (m.cfg["vocab"], m.cfg["hidden"])
+            m.load_tensor(-1, L.T_FINAL_NORM if load else L.T_EMBED, np.zeros(shape, np.uint16))
+        close(m.read_logits(), want)
+        m.destroy()
+        m = model(dev)
     m.destroy()
 
 

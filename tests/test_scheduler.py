@@ -1,7 +1,10 @@
 """Which call of a runner a scheduler's step becomes."""
+import os
+
 import numpy as np
 import pytest
 
+from doppler_b200 import scheduler
 from doppler_b200.scheduler import Scheduler
 
 
@@ -56,3 +59,15 @@ def test_everything_else_is_a_portion():
     s.step("b", [3])
     s.step("a", [4], [0])
     assert m.calls == [("extend", 2, 0), ("extend", 1, 1), ("extend", 1, 0)]
+
+
+def test_a_failed_step_leaves_no_hidden_row():
+    """dp_model_advance: the row that logits may still be computed from is given up when the step's graph is launched, and there again
+    only behind the last thing that can fail."""
+    with open(os.path.join(os.path.dirname(scheduler.__file__), "csrc", "model.cu")) as f:
+        text = f.read()
+    at = text.index('extern "C" dp_status dp_model_advance')
+    body = text[at:text.index("\n}\n", at)]
+    launch, gone, back = (body.index(x) for x in ("dp_graph_launch(", "m->head_row = nullptr;", "m->head_row = m->h;"))
+    assert launch < gone < back
+    assert not any(x in body[launch:gone].split(";", 1)[1] for x in ("DP_TRY", "DP_CUDA")) and not any(x in body[back:] for x in ("DP_TRY", "DP_CUDA"))
