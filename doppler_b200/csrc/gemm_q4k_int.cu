@@ -1033,14 +1033,25 @@ dp_status dpk_gemm_q4k_int(dp_ctx *ctx, const uint8_t *W, const void *A, dp_dtyp
   if (norm_w && (guard || !(vec && K >= 1024 && K <= 4096 && ((uintptr_t)norm_w & 15) == 0))) return DP_OK;
   const bool silu = !guard && fuse && fuse->silu_dst && c_dtype == DP_F32 && N % 16 == 0;
   const bool lo_first = f32a && (guard || M <= 64 || (fuse && fuse->exact_weights));
-  const IntPlan p = qi_plan(ctx, M, N, K, f32a, lo_first, !silu);
-
+  IntPlan p = qi_plan(ctx, M, N, K, f32a, lo_first, !silu);
   const int kp = (K + BK - 1) / BK * BK;
   const size_t a_bytes = ((size_t)M * kp * 2 + 255) / 256 * 256;
-  const size_t sum_cols = (size_t)p.parts * p.npu * 256, s_bytes = ((size_t)M * sum_cols * 2 + 255) / 256 * 256;
-  dp_status st = dp_scratch(ctx, &ctx->gemm_scratch, a_bytes * (f32a ? 2 : 1) + s_bytes + (size_t)M * 4, "matmul_a_f16");
-  if (st == DP_OK && p.parts > 1) st = dp_scratch(ctx, &ctx->gemm_split_scratch, (size_t)p.parts * M * N * 4, "matmul_k_split_parts");
-  if (st == DP_ERR_OOM && guard) return DP_OK;  // no memory for the pass over the rows: the CUDA cores need none
+  size_t sum_cols, s_bytes;
+  auto rows_scratch = [&]() -> dp_status {
+    sum_cols = (size_t)p.parts * p.npu * 256;
+    s_bytes = ((size_t)M * sum_cols * 2 + 255) / 256 * 256;
+    return dp_scratch(ctx, &ctx->gemm_scratch, a_bytes * (f32a ? 2 : 1) + s_bytes + (size_t)M * 4, "matmul_a_f16");
+  };
+  // Where memory is short: one part of K needs none for its sums, and the kernels behind this one need none for the rows.
+  dp_status st = rows_scratch();
+  if (st == DP_OK && p.parts > 1) {
+    st = dp_scratch(ctx, &ctx->gemm_split_scratch, (size_t)p.parts * M * N * 4, "matmul_k_split_parts");
+    if (st == DP_ERR_OOM) {
+      p = qi_plan(ctx, M, N, K, f32a, lo_first, false);
+      st = rows_scratch();
+    }
+  }
+  if (st == DP_ERR_OOM) return DP_OK;
   DP_TRY(st);
   char *base = (char *)ctx->gemm_scratch->dptr;
   __half *hi = (__half *)base, *lo = (__half *)(base + a_bytes), *sums = (__half *)(base + a_bytes * (f32a ? 2 : 1));

@@ -942,7 +942,7 @@ static dp_status gemm_q4k_tc_impl(dp_ctx *ctx, const uint8_t *W, const void *A, 
     const bool take = tiled ? a_dtype == DP_F32 || rows64 || ((few || K > 1024) && !small) : whole;
     if (take) {
       DP_TRY(dpk_gemm_q4k_int(ctx, W, A, a_dtype, C, c_dtype, M, N, K, alpha, handled, fuse));
-      if (*handled) return DP_OK;
+      if (*handled || few) return DP_OK;  // (no memory for its rows: few rows keep exact weights on the CUDA cores)
     }
   }
   if (!tiled) return DP_OK;

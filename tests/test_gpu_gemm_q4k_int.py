@@ -238,3 +238,34 @@ def test_epilogues_through_one_layer(dev, name, rows):
     # key or value off by 1e-6 is there for one entry in 500: 2^-11 / sqrt(500) = 2e-5 of the attention's share of a row
     err = np.sqrt(((got - x) ** 2).mean()) / x.std()
     assert err < 4e-5, err
+
+
+def test_little_memory_left():
+    """Where there is no room for the sums of the parts of K, or for the rows as f16 halves, a product runs without."""
+    import torch
+
+    rng, m, n, k = np.random.default_rng(5), 512, 2048, 12288
+    b = blocks(rng, n, k // 256)
+    b[:, :, :4] = (10.0 ** rng.uniform(-4, -2, (n, b.shape[1], 2))).astype(np.float16).view(np.uint8).reshape(n, -1, 4)
+    rows = [rng.standard_normal((m, k)).astype(t) for t in (np.float32, np.float16)]
+    results, used = [], []
+    for room in (0, 36 << 20, 12 << 20):  # (the rows take 32 and 16 MB, the parts 8 and 16)
+        d = ops.Device(0)
+        try:
+            w = d.weight_from(b.ravel(), "q4k", [n, k])
+            ts, outs = [d.tensor_from(a) for a in rows], [d.acquire_buffer(m * n * 4, "out") for _ in rows]
+            while room:
+                free = torch.cuda.mem_get_info(0)[0] - room
+                if free < 4 << 20:
+                    break
+                d.acquire_buffer(free >> 24 << 24 if free >= 64 << 20 else 4 << 20, "held")
+            before = d.pool_stats()["bytes_allocated"]
+            results.append([d.read_tensor(ops.run_matmul(t, w, m, n, k, output_buffer=o, output_dtype="f32")).reshape(m, n) for t, o in zip(ts, outs)])
+            used.append(d.pool_stats()["bytes_allocated"] - before)
+        finally:
+            d.close()
+    assert used[0] > used[1] > used[2] == 0, used
+    for i, a in enumerate(rows):
+        want = a.astype(np.float64) @ np.subtract(*parts(b)).T
+        for got in results:  # (f32 FMAs in order of K: 2e-6)
+            assert np.linalg.norm(got[i] - want) <= 4e-6 * np.linalg.norm(want)
