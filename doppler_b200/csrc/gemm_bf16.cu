@@ -170,6 +170,7 @@ __global__ void __launch_bounds__(BT_THREADS, 1) gemm_bf16_tc_kernel(const __gri
       for (int c0 = 0; c0 < a.bn; c0 += 16) {
         if (m0 + c0 >= a.M) break;  // (uniform) no such activation rows
         uint32_t r[16];
+        __syncwarp();  // (lanes store by themselves; tensor memory is read by the whole warp)
         tmem_ld16(taddr + (uint32_t)c0, r);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         if (a.glu.dst) {

@@ -145,17 +145,19 @@ __global__ void __launch_bounds__(FR_THREADS, 1) gemm_f16w_rows_kernel(const __g
         const int h = u / chunks, c0 = (u - h * chunks) * 16, f = tile * tile_rows + h * a.rows + row;
         const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)((b * a.halves + h) * cols + c0);
         uint32_t hi[16], lo[16];
+        __syncwarp();  // (lanes without a row skip the stores below; tensor memory is read by the whole warp)
         tmem_ld16(taddr, hi);
         if (a.planes == 2) tmem_ld16(taddr + (uint32_t)a.n, lo);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (row >= a.rows || f >= a.N) continue;
+        if (row < a.rows && f < a.N) {
 #pragma unroll
-        for (int i = 0; i < 16; i++) {
-          const int m = a.m_base + c0 + i;
-          if (m < a.M) {
-            const float v = (a.planes == 2 ? __uint_as_float(hi[i]) + __uint_as_float(lo[i]) : __uint_as_float(hi[i])) * a.alpha * (a.row_scale ? __ldg(a.row_scale + m) : 1.0f);
-            if constexpr (sizeof(OutT) == 4) reinterpret_cast<float *>(a.C)[(size_t)m * a.N + f] = v;
-            else reinterpret_cast<__half *>(a.C)[(size_t)m * a.N + f] = __float2half_rn(v);
+          for (int i = 0; i < 16; i++) {
+            const int m = a.m_base + c0 + i;
+            if (m < a.M) {
+              const float v = (a.planes == 2 ? __uint_as_float(hi[i]) + __uint_as_float(lo[i]) : __uint_as_float(hi[i])) * a.alpha * (a.row_scale ? __ldg(a.row_scale + m) : 1.0f);
+              if constexpr (sizeof(OutT) == 4) reinterpret_cast<float *>(a.C)[(size_t)m * a.N + f] = v;
+              else reinterpret_cast<__half *>(a.C)[(size_t)m * a.N + f] = __float2half_rn(v);
+            }
           }
         }
       }
