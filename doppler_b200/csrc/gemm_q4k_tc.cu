@@ -414,8 +414,7 @@ __global__ void __launch_bounds__((BNMAX / 16 + 2) * 32, 1) gemm_q4k_tc2_kernel(
   const uint32_t accum_bar = bars + 8u * (uint32_t)(SA + SB + SD);
   constexpr uint32_t TMEM_COLS = 512;
 
-  pdl_launch();
-  pdl_wait();
+  pdl_wait();  // (no early launch of dependents out of a launch of clusters, see gemm_q4k_int.cu)
   if (tid == 0) {
     for (int s = 0; s < SA; s++) mbar_init(full_a(s), 1);
     for (int s = 0; s < SD; s++) mbar_init(done(s), 1);

@@ -19,3 +19,10 @@ def body(file, kernel):
 def test_first_kernels_of_a_step_wait_before_they_launch(file, kernel):
     b = body(file, kernel)
     assert b.count("pdl_launch();") == 1 and 0 < b.index("pdl_wait();") < b.index("pdl_launch();")
+
+
+@pytest.mark.parametrize("file,kernel", [("gemm_q4k_int.cu", "gemm_q4k_int_kernel"), ("gemm_q4k_tc.cu", "gemm_q4k_tc2_kernel"), ("gemm_bf16.cu", "gemm_bf16_tc_kernel")])
+def test_launches_of_clusters_launch_no_dependents_early(file, kernel):
+    """Dependents of such a launch, which carries no programmatic attribute, were seen to read rows that it had not stored yet."""
+    b = body(file, kernel).replace("if constexpr (!PAIR) pdl_launch();", "")
+    assert "pdl_launch();" not in b and b.count("pdl_wait();") == 1
