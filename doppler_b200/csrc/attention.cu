@@ -325,6 +325,13 @@ bool dpk_attention_rows_eligible(const dpk_attn_params &p);
 bool dpk_attention_rows_fills(dp_ctx *ctx, const dpk_attn_params &p, int splits);
 int dpk_attention_rows_splits(dp_ctx *ctx, const dpk_attn_params &p);
 dp_status dpk_attention_rows(dp_ctx *ctx, const dpk_attn_params &p, float *scratch, int splits);
+// where the kernel behind it is the one that takes any shape; f16 heads of 64 and 128 in groups that the tensor-core kernels leave out (twelve
+// heads, say) stay with attn_split_kernel: 12 and 24 heads of 64, triples 220 000 15 -> 23 us, 450 000 22 -> 25, 1 000 000 35 -> 38, of 128 21 -> 33,
+// 31 -> 37, 54 -> 59; faster only from 2 500 000 on (68 -> 62), and with up to 6 % more error
+static bool uses_rows(const dpk_attn_params &p) {
+  int gt;
+  return !fast_shape(p, &gt) && dpk_attention_rows_eligible(p);
+}
 
 // the most keys one query row sees
 static long row_keys(const dpk_attn_params &p) { return p.chunk > 0 && p.chunk < p.kv_len ? p.chunk : p.kv_len; }
@@ -360,7 +367,7 @@ size_t dpk_attention_scratch_bytes(dp_ctx *ctx, const dpk_attn_params &p, int *s
     *splits_out = s;
     return s == 1 ? 0 : (size_t)p.batch * p.seq_len * p.num_heads * s * (p.v_dim + 2) * sizeof(float);
   }
-  if (dpk_attention_rows_eligible(p)) {
+  if (uses_rows(p)) {
     const int s = dpk_attention_rows_splits(ctx, p);
     *splits_out = s;
     return s == 1 ? 0 : (size_t)p.batch * p.seq_len * p.num_heads * s * ((p.v_dim ? p.v_dim : p.head_dim) + 2) * sizeof(float);
@@ -421,7 +428,7 @@ static dp_status attention_impl(dp_ctx *ctx, const dpk_attn_params &p, float *sc
     DP_TRY(dpk_attention_latent(ctx, p, scratch, splits));
   } else if (use_tc(ctx, p, &gt)) {
     DP_TRY(dpk_attention_tc_split(ctx, p, scratch, splits));
-  } else if (dpk_attention_rows_eligible(p) && dpk_attention_rows_fills(ctx, p, splits)) {
+  } else if (uses_rows(p) && dpk_attention_rows_fills(ctx, p, splits)) {
     DP_TRY(dpk_attention_rows(ctx, p, scratch, splits));
   } else if (fast_shape(p, &gt)) {
     if (p.head_dim == 128) {
@@ -462,7 +469,7 @@ dp_status dpk_attention(dp_ctx *ctx, const dpk_attn_params &p) {
   float *scratch = nullptr;
   if (bytes) {
     const dp_status st = dp_scratch(ctx, &ctx->attn_scratch, bytes, "attention_split_partials");
-    if (st == DP_ERR_OOM && dpk_attention_rows_eligible(p)) splits = 1;  // (one part needs no room)
+    if (st == DP_ERR_OOM && uses_rows(p)) splits = 1;  // (one part needs no room)
     else if (st != DP_OK) return st;
     else scratch = (float *)ctx->attn_scratch->dptr;
   }

@@ -1,6 +1,6 @@
 // Attention of several query rows in f32 arithmetic, query-tiled: f16 or f32 caches, key and value sizes up to 256 in steps of
-// four, any GQA ratio, every mask of attn_range.  For what the tensor-core portions (attention_prefill.cu) do not take: f32
-// caches, heads of 64 or 256, sliding windows, soft caps, rows without a causal mask.
+// four, any GQA ratio, every mask of attn_range.  For f32 caches and for f16 heads that are not 64 or 128 values (those have kernels of
+// their own: attention_prefill.cu, attention_tc.cu, attn_split_kernel) or whose values are not as long as their keys.
 //
 // A block holds 32 (position, head) rows of one KV head and walks the keys in tiles of 64, so a key is read once for 32 rows
 // and not once for each (or for the four heads of a position).  S = Q K^T and O += P V are register tiles of 4 rows x 4 keys and
@@ -321,6 +321,7 @@ int dpk_attention_rows_splits(dp_ctx *ctx, const dpk_attn_params &p) {
 // has been through its first tiles (cold code, a load behind every barrier).  us, the kernel that goes row by row -> this one:
 //   f16 heads of 256, triples: 61 000 47 -> 58, 120 000 46 -> 54, 160 000 56 -> 60, 245 000 146 -> 63, 256 000 96 -> 62,
 //     410 000 82 -> 56, 2 000 000 397 -> 167, 67 000 000 10 940 -> 2 940
+//   f16 heads of 32 and 48, 220 000: 25 to 48 -> 15 to 27; of 96: 29 to 49 -> 25 to 37 (one KV head of 96 without a mask 25 -> 27)
 //   f32 heads of 128: 58 000 16 -> 31, 116 000 25 -> 28, 230 000 38 -> 32, 500 000 72 -> 43, 3 900 000 430 -> 142
 bool dpk_attention_rows_eligible(const dpk_attn_params &p) {
   if (!rows_shape(p)) return false;

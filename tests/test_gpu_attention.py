@@ -239,6 +239,16 @@ def _exact_rows(q, k, v, causal, start, window, cap, kv_start):
     (2, 2, 160, 401, 401, dict(causal=False)),
     (12, 1, 200, 90, 641, dict(kv_start=37)),                           # groups of 4, the cache begins behind the sequence's start
     (32, 8, 256, 258, 258, {}),                                         # one part
+    # 64 and 128 values a row in shared memory
+    (8, 8, 48, 260, 260, {}),
+    (16, 4, 32, 300, 300, dict(sliding_window=60)),
+    (6, 2, 40, 200, 220, dict(causal=False)),                           # groups of 3
+    (12, 1, 60, 200, 200, {}),                                          # groups of 12, four heads a block
+    (24, 2, 56, 200, 201, dict(attn_softcap=2.5)),
+    (8, 2, 96, 300, 300, dict(sliding_window=100)),
+    (4, 4, 72, 330, 330, dict(attn_softcap=2.5)),
+    (12, 1, 124, 120, 140, dict(causal=False)),
+    (24, 2, 120, 200, 200, dict(sliding_window=70, attn_softcap=5.0)),
 ])
 def test_rows_in_f32(dev, H, Hkv, D, T, kv, opt):
     s = synthetic.key(61, D * 100 + T)
@@ -250,13 +260,50 @@ def test_rows_in_f32(dev, H, Hkv, D, T, kv, opt):
     assert np.all(np.abs(got - exp) <= bound), float((np.abs(got - exp) / bound).max())
     if opt:
         return
-    # a key that is NaN and values that are infinite change the rows that see them and no other
+    # a key that is NaN and values that are infinite change the rows that see them and no other; those are what they are by themselves
+    # (one row runs on another kernel): infinite or NaN behind the values, and zeros, as every kernel here has it, behind the key
     bad = kv - T // 2
     k2, v2 = k.reshape(kv, -1).copy(), v.reshape(kv, -1).copy()
     k2[bad + 1, ::3], v2[bad] = np.nan, np.inf
     mixed = _attn(dev, q, k2.ravel(), v2.ravel(), H, D, seq_len=T, kv_len=kv, num_kv_heads=Hkv, start_pos=start).reshape(T, H, D)
     first = bad - start
-    assert np.array_equal(mixed[:first], got[:first]) and not np.isfinite(mixed[first]).any() and (mixed[first + 1:] != got[first + 1:]).all()
+    assert np.array_equal(mixed[:first], got[:first]) and not np.isfinite(mixed[first]).any()
+    for r in (first, first + 1, T - 1):
+        alone = _attn(dev, q.reshape(T, -1)[r], k2.ravel(), v2.ravel(), H, D, seq_len=1, kv_len=kv, num_kv_heads=Hkv, start_pos=start + r).reshape(H, D)
+        assert np.array_equal(np.isfinite(mixed[r]), np.isfinite(alone)) and np.array_equal(mixed[r] == 0, alone == 0)
+
+
+@pytest.mark.parametrize("H,Hkv,D,causal", [(12, 2, 96, True), (8, 8, 256, True), (12, 1, 40, False)])
+def test_rows_in_f32_of_several_sequences(dev, H, Hkv, D, causal):
+    """Sequences that hold fewer keys than the call allows for, one of them none."""
+    B, T, kv, lens = 4, 100, 160, [160, 37, 0, 101]
+    s = synthetic.key(62, D)
+    q, k, v = synthetic.normal_f32(s, B * T * H * D), synthetic.normal_f16(s + 1, B * kv * Hkv * D), synthetic.normal_f16(s + 2, B * kv * Hkv * D)
+    lens_buffer = dev.tensor_from(np.asarray(lens, np.int32)).buffer
+    got = _attn(dev, q, k, v, H, D, seq_len=T, kv_len=kv, num_kv_heads=Hkv, start_pos=kv - T, causal=causal, batch=B, kv_batch_stride=kv * Hkv * D,
+                kv_len_buffer=lens_buffer).reshape(B, T, H, D)
+    dev.release_buffer(lens_buffer)
+    for b, n in enumerate(lens):
+        if n == 0:
+            assert not got[b].any()
+            continue
+        kb, vb = (x.reshape(B, kv, Hkv, D)[b, :n].astype(np.float64) for x in (k, v))
+        exp, bound = _exact_rows(q.reshape(B, T, H, D)[b].astype(np.float64), kb, vb, causal, kv - T, 0, 0.0, 0)
+        assert np.all(np.abs(got[b] - exp) <= bound), (b, float((np.abs(got[b] - exp) / bound).max()))
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Hkv", [1, 2])
+def test_groups_of_twelve_go_row_by_row(dev, Hkv, D):
+    """f16 heads of 64 and 128 that no tensor-core kernel takes: however many rows a call has, a row is the same bits."""
+    T, H, s = 1600 // Hkv, 12 * Hkv, synthetic.key(63, D)
+    q, k, v = synthetic.normal_f32(s, T * H * D).reshape(T, -1), synthetic.normal_f16(s + 1, T * Hkv * D), synthetic.normal_f16(s + 2, T * Hkv * D)
+
+    def rows(i, n):
+        return _attn(dev, q[i:i + n].ravel(), k, v, H, D, seq_len=n, kv_len=T, num_kv_heads=Hkv, start_pos=i, sliding_window=20).reshape(n, -1)
+
+    part = T // 4  # (enough rows for one part of the keys)
+    assert np.array_equal(rows(0, T), np.concatenate([rows(i, part) for i in range(0, T, part)]))
 
 
 def test_attention_argument_errors(dev):
