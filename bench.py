@@ -255,7 +255,7 @@ def gemv_case(dev, ops, synthetic, N, K, copies, reps, peak):
 def gemm_case(dev, ops, synthetic, M, N, K, copies, reps, peak, variant="default", adtype="f16"):
     copies = copies or 4
     ws = [dev.weight_from(synthetic.q4k_matrix(synthetic.key(5, i), N, K), "q4k", [N, K]) for i in range(copies)]
-    if adtype == "f32":  # the runner's case: f32 activations and output, f32-exact product (three tensor-core products)
+    if adtype == "f32":  # the runner's case: f32 activations and output, f32-exact product (integer weight tiles, two tensor-core products)
         a = dev.tensor_from(synthetic.normal_f32(synthetic.key(5, 100), M * K).reshape(M, K))
     else:
         a = dev.tensor_from(synthetic.normal_f16(synthetic.key(5, 100), M * K).reshape(M, K))
@@ -317,7 +317,7 @@ def kernels_record(dev, peak):
     return {
         "config0_gemv_3072x1024": keep(g0, ("us_per_call", "GBps", "frac_of_measured_hbm", "note")),
         "config1_gemm_512x12288x4096": dict(keep(g1, ("us_per_call", "TFLOPs", "frac_of_measured_burst", "frac_of_measured_sustained")),
-                                            note="default: exact product (dequantised weights kept to f32 accuracy), gate 1e-3"),
+                                            note="default: exact product (integer weight tiles), gate 1e-3"),
         "config1_gemm_f16_weights": dict(keep(g1f, ("us_per_call", "TFLOPs", "frac_of_measured_burst", "frac_of_measured_sustained")),
                                          note="opt-in: weights rounded to f16 as in the reference's tiled f16 prefill kernel"),
         "config2_attention_b32_ctx8192": keep(a2, ("us_per_call", "GBps", "frac_of_measured_hbm")),
@@ -810,7 +810,7 @@ def main():
                     times_p.append((time.perf_counter() - t0) * 1e3)
                 pms = statistics.median(times_p)
                 line["prefill"] = {"prompt_tokens": context, "ms": pms, "tokens_per_s": context / (pms / 1e3),
-                                   "note": "f32 activations, f32-exact product (three tensor-core products per K step)"}
+                                   "note": "f32 activations, f32-exact product (integer weight tiles, two tensor-core products per K step)"}
             except Exception as e:
                 line["prefill"] = {"failed": str(e)}
         model.destroy()

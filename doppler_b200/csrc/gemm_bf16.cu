@@ -11,7 +11,8 @@
 // cluster of two CTAs owns 256 features (cta_group::2) and each brings its 128 weight rows and half of the activation rows,
 // 32 KB.  The products of a prompt of 2048 tokens (the ten of four 4096-wide Fenorax layers): 1777 us with the MMAs out of a
 // branch of one lane, 1575 from a converged warp (umma.cuh), 1452 in pairs; of 1500 tokens (22 of four Virolorn layers) 1753, 1483, 1436;
-// of 40 tokens at width 1024 129 -> 97.
+// of 40 tokens at width 1024 129 -> 97.  (Pairs then had widths in steps of 16, 240 and 176 here; with steps of 32, 256 and 192, whole
+// prompts take the same.)
 //
 // dpk_gemm_f16_tc: the same kernel with f16 operands and an f16 result.
 //

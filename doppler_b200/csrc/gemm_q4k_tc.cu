@@ -15,8 +15,8 @@
 //     header per row and step), dequantise in registers, w = fma(d*sc, q, -dmin*m) rounded to
 //     f16, and store the BN x 64 tile into shared memory in the same 128-byte-swizzled K-major
 //     layout the tensor core expects (each weight is dequantised once per CTA);
-//   - warp 1 (one lane) issues tcgen05.mma (kind::f16, M=128, N=BN, K=16) for both accumulators
-//     and commits to an mbarrier that frees the stage.
+//   - warp 1 (all of it runs the loop, one elected lane issues, see umma.cuh) issues tcgen05.mma (kind::f16,
+//     M=128, N=BN, K=16) for both accumulators and commits to an mbarrier that frees the stage.
 // After the last step warps 2..9 read the accumulators back with tcgen05.ld (each warp its own
 // 32-lane quarter of tensor memory) and write C as f32 or f16.
 // Every mbarrier wait is bounded; on give-up the CTA raises a status word and still frees its
@@ -927,8 +927,10 @@ static dp_status gemm_q4k_tc_impl(dp_ctx *ctx, const uint8_t *W, const void *A, 
   //   f16 rows  384 x 6144 x 4096 40 -> 40, 512 x 12288 x 4096 80 -> 70, 512 x 4096 x 12288 221 -> 156, 2048 x 24576 x 4096 502 -> 398
   // The two products stay for f16 rows where the pass over the rows and a unit's fixed cost weigh more: K up to 1024 with more than half a
   // wave of the others' 512 x 256 pair tiles (2048 x 3072 x 1024 27 -> 37), and, but for up to 64 rows with an f32 result, weights of less
-  // than 2^19 values.  Those few rows always had exact weights (a residue in f16 loses bits, 2e-6 against 4e-7, and a weight beyond f16's
-  // range is NaN there), and nothing rounds their result.
+  // than 2^19 values.  Those few rows always had exact weights (a residue in f16 loses bits: 6e-7, 1.2e-6 and 1.8e-6 at K = 256, 512 and 768
+  // against 3.1e-7; and a weight beyond f16's range is NaN there), and nothing rounds their result.  They cost a cluster's launch and a
+  // pass over the rows, us a call, two products -> integer tiles: 32 x 256 x 256 8.5 -> 14.5, 32 x 512 x 768 12.4 -> 16.5, 32 x 256 x 1024 16.1 -> 16.5,
+  // 32 x 384 x 1280 23.2 -> 18.6.
   // Shapes the others do not tile ran on CUDA cores (1000 x 1000 x 1000: f32 rows 105 -> 30, f16 rows 102 -> 27 us); they still do where
   // that is over within about 15 us, where the result is f32 and K below 640 (error of the f32 FMAs 4.1e-7 at K = 512, of the integer
   // tiles 4.8e-7; 5.7e-7 and 4.6e-7 at 1024), and with an alpha that a row's scale might carry out of f32's range.

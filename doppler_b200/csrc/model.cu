@@ -1341,9 +1341,8 @@ extern "C" dp_status dp_model_decode(dp_model *m, int batch, const int32_t *firs
   memset(st, 0, 4096);
   for (int b = 0; b < batch; b++) { st[b] = m->seq_len[b]; st[256 + b] = m->seq_len[b] + 1; st[512 + b] = first_tokens[b]; }
   DP_CUDA(ctx, cudaMemcpyAsync(m->state->dptr, st, 4096, cudaMemcpyHostToDevice, ctx->stream));
-  const int slot = 0;
-  if (!m->graph[slot] || m->graph_batch[slot] != batch) {
-    if (m->graph[slot]) { dp_graph_destroy(m->graph[slot]); m->graph[slot] = nullptr; }
+  if (!m->graph[0] || m->graph_batch != batch) {
+    if (m->graph[0]) { dp_graph_destroy(m->graph[0]); m->graph[0] = nullptr; }
     dp_recorder *rec = nullptr;
     DP_TRY(dp_recorder_begin(ctx, "decode_step", 1, &rec));
     ctx->pdl = getenv("DP_PDL") ? atoi(getenv("DP_PDL")) != 0 : true;  // kernels of the step overlap their launch with the predecessor's tail
@@ -1352,11 +1351,11 @@ extern "C" dp_status dp_model_decode(dp_model *m, int batch, const int32_t *firs
     m->recording_decode = false;
     ctx->pdl = false;
     if (s != DP_OK) { std::string keep = ctx->err; dp_recorder_abort(rec); ctx->err = keep; return s; }
-    DP_TRY(dp_recorder_finish_graph(rec, &m->graph[slot]));
-    m->graph_batch[slot] = batch;
+    DP_TRY(dp_recorder_finish_graph(rec, &m->graph[0]));
+    m->graph_batch = batch;
   }
   DP_CUDA(ctx, cudaEventRecord(m->ev0, ctx->stream));
-  for (int s = 0; s < steps; s++) DP_TRY(dp_graph_launch(m->graph[slot]));
+  for (int s = 0; s < steps; s++) DP_TRY(dp_graph_launch(m->graph[0]));
   DP_CUDA(ctx, cudaEventRecord(m->ev1, ctx->stream));
   // tokens and the device status word come back together, one synchronisation per call
   DP_CUDA(ctx, cudaMemcpyAsync(m->pin_out, m->out_tokens->dptr, (size_t)steps * batch * 4, cudaMemcpyDeviceToHost, ctx->stream));

@@ -52,7 +52,7 @@ struct dp_model {
   std::vector<int> seq_len;
   const PackedRows *packed = nullptr;  // set while run_layers runs such a pass
   dp_graph *graph[2] = {nullptr, nullptr};  // a decode step; a step of one sequence without logits
-  int graph_batch[2] = {0, 0};
+  int graph_batch = 0;                      // sequences of the decode step
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   double last_ms = 0;
   size_t weight_bytes = 0;

@@ -110,8 +110,8 @@ extern "C" dp_status dp_matmul(dp_ctx *ctx, dp_recorder *rec, const dp_tensor *A
       // fused_matmul_q4_prefill_tiled_f16.wgsl:201: weights rounded to f16 first), one tensor-core product.
       if (!o.exact_weights && M > 1 && A->dtype == DP_F16)
         st = dpk_gemm_q4k_tc(ctx, (const uint8_t *)bptr, aptr, A->dtype, cptr, o.out_dtype, M, N, K, o.alpha, o.f16_weights != 0, &handled);
-      // f32 activations select the f32-exact product (matmul.rules.json:15-22): from 32 rows on the tensor
-      // cores compute it in three passes (f16 halves and rounding residues of activations and weights)
+      // f32 activations select the f32-exact product (matmul.rules.json:15-22): from two rows on the tensor cores compute it out of
+      // integer weight tiles and the rows' two f16 halves
       else if (!o.exact_weights && M >= 2 && A->dtype == DP_F32 && o.out_dtype == DP_F32)
         st = dpk_gemm_q4k_tc_rowscaled(ctx, (const uint8_t *)bptr, (const float *)aptr, (float *)cptr, M, N, K, o.alpha, 3, &handled);
       if (st == DP_OK && !handled)

@@ -207,9 +207,10 @@ __global__ void __launch_bounds__(SB_THREADS, 2) stream_boundary_kernel(const Bo
 // thread: a block walks down its rows with a group's channels in its threads.  The last taps - 1 rows of h stay in registers,
 // the next row's loads go out before this row's sum over the group, one barrier a row.  Bound: HBM (x read and written, y, the
 // sublayer's input: 318 MB at 2048 rows x 4 streams x 4096).  The kernel above holds a block of rows in shared memory, loads, waits and
-// convolves in turn and reads 3 rows more for every 15: 91 us there, 56 here.
+// convolves in turn and reads 3 rows more for every 15: 91 us there, 56 here when a thread's squares went straight into the sum.
 // A group's squares are summed in the order of the kernel above, lane l over the channels 4 l + 128 k, by every warp for itself
-// out of shared memory: a row is the same bits whichever of the two it goes through, however a prompt is cut.
+// out of shared memory: a row is the same bits whichever of the two it goes through, however a prompt is cut.  (A whole prompt of
+// 2048 tokens takes the same with either order, 3.27 ms.)
 template <int SM, typename OutT>
 __global__ void __launch_bounds__(512) stream_rows_kernel(const BoundaryArgs a, OutT *__restrict__ dst) {
   pdl_launch();

@@ -266,8 +266,7 @@ def test_f32_activation_gemm_runs_on_the_tensor_cores(dev):
 
 @pytest.mark.parametrize("M,N,K", [(64, 4096, 12288), (64, 6144, 4096), (40, 1536, 2048), (2, 256, 256), (17, 128, 512), (33, 384, 1024)])
 def test_small_batch_gemm_weights_on_the_m_side(dev, M, N, K):
-    """2..64 activation rows (batched decode steps): the kernel with the 128 weight rows of a tile on the MMA's M
-    side, units of (tile, super-block column) dealt evenly to one CTA per SM, split tiles added in CTA order.
+    """2..64 activation rows (batched decode steps): integer weight tiles on the MMA's M side, parts of K added in order.
     f32 activations spanning ten decades against the exact product per row (gate 2e-5 up to K = 2048, growing
     with sqrt(K) beyond); two runs give the same
     bits; f16 activations with both weight numerics."""
@@ -294,9 +293,9 @@ def test_small_batch_gemm_weights_on_the_m_side(dev, M, N, K):
 
 
 def test_two_sm_gemm_split_over_k(dev):
-    """More than 256 rows on few 512 x 256 pair tiles (here two): the two-SM kernel runs several clusters per tile
-    along K, every part writes its own partial tile and the parts are added in a fixed order.  f32 activations
-    (three products per K step) against the exact product per row, a ragged row count, and the same bits twice."""
+    """More than 256 rows on few tiles: several clusters per tile along K, every part writes its own partial tile and the
+    parts are added in a fixed order.  f32 activations (integer weight tiles, two products per K step) against the exact
+    product per row, a ragged row count, and the same bits twice."""
     M, N, K = 300, 512, 4096
     W = synthetic.q4k_matrix(synthetic.key(97, 0), N, K)
     A = synthetic.normal_f32(synthetic.key(97, 1), M * K).reshape(M, K)
@@ -318,7 +317,7 @@ def test_few_tiles_long_k_is_deterministic(dev):
     """A problem of few output tiles and a long K (here two tiles, K = 4096) is split over K: several CTAs per
     tile take whole super-blocks each, write their own partial tile, and a second kernel adds the parts in a
     fixed order (no atomics), so two runs give the same bits; f16 activations against the exact product,
-    f32 activations (three products per K step in one f32 accumulator) against it per row."""
+    f32 activations (two products per K step) against it per row."""
     M, N, K = 96, 256, 4096
     W = synthetic.q4k_matrix(synthetic.key(94, 0), N, K)
     A = synthetic.normal_f16(synthetic.key(94, 1), M * K)

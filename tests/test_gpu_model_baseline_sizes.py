@@ -58,8 +58,8 @@ def test_config4_shape_batch1_64_tokens(dev, nine_b_two_layers):
 
 @pytest.mark.parametrize("B", [64, 12])
 def test_config4_shape_batch64(dev, nine_b_two_layers, B):
-    """Batch 64 and batch 12: up to 32 rows the runner folds RMSNorm, silu(gate)*up and the
-    residual adds into the small-batch projections, beyond it launches them as kernels of their own."""
+    """Batch 64 and batch 12: the runner folds RMSNorm, silu(gate)*up and the residual adds into the
+    projections on integer weight tiles."""
     cfg, w = nine_b_two_layers
     steps, max_seq = 12, 32
     lens = [2 + (i * 5) % 8 for i in range(B)]
