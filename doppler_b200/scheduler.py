@@ -42,10 +42,11 @@ class Scheduler:
         if any(w < 0 or w >= len(tokens) for w in want):
             raise ValueError("a wanted place lies outside the tokens")
         if len(tokens) == 1 and s == 0 and len(self.slots) == 1:
-            if not want and hasattr(self.model, "advance") and self.model.tp_size == 1:
-                self.model.advance(tokens[0])  # (leaves the table's product out)
+            if hasattr(self.model, "advance") and self.model.tp_size == 1:
+                # (the logits only where they are wanted; where all are, as fast as the decode step's graph: 220 us for 226, 427 for 431)
+                self.model.advance(tokens[0])
             else:
-                self.model.decode([tokens[0]], 1)  # (the table's product in the step's graph)
+                self.model.decode([tokens[0]], 1)
             rows = self.model.read_logits(self.model.cfg["vocab"]).reshape(1, -1) if want else np.empty((0, self.model.cfg["vocab"]), np.float32)
             return rows[want] if want else rows
         order = sorted(set(want))
